@@ -365,11 +365,7 @@ int32_t fvc_context_destroy(fvc_context *c) {
   for (int i = 0; i < fvc::Scratch::kVec; ++i) cudaFree(c->S.v[i]);
   for (int i = 0; i < 10; ++i) cudaFree(c->S.f[i]);
   cudaFree(c->S.g);
-  cudaFree(c->S.partials);
   cudaFree(c->S.sync);
-  cudaFree(c->S.err);
-  cudaFree(c->S.result);
-  cudaFree(c->S.iresult);
   cudaFree(c->S.trace);
   cudaFree(c->S.history);
   cudaFree(c->d_b);

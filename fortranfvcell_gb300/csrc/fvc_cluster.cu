@@ -366,9 +366,7 @@ int32_t enqueue_pcg_cluster(const DeviceMatrix &A, Scratch &S, const double *b, 
     return FVC_ERR_UNSUPPORTED;
   }
   if (!launch) return FVC_OK;
-  cudaMemsetAsync(S.err, 0, 64, stream);  // the whole error block (wait and check words)
-  cudaMemsetAsync(S.iresult, 0, 16 * sizeof(int), stream);
-  cudaMemsetAsync(S.result, 0, 16 * sizeof(double), stream);
+  reset_sync(S, stream, 0);
   ClArgs a{};
   a.A = SellView<double>{A.n, A.nslices, A.sptr, A.col, A.val, A.diag, A.diag_mode};
   a.minv = A.jinv;

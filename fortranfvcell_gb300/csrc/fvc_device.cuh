@@ -13,6 +13,7 @@
 // products and sums are rounded separately, as the Fortran loops do).
 #pragma once
 #include <cooperative_groups.h>
+#include <climits>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -67,17 +68,25 @@ enum CheckCode : int {
   } while (0)
 #endif
 
+// One block's partial of one reduced quantity with the episode that wrote
+// it, moved by single 16-byte accesses: a reader that finds the episode has
+// the value, with no ordering between the slot and any other word.
+struct __align__(16) RedSlot {
+  unsigned long long v, ep;
+};
+
 // Grid synchronisation state of one persistent launch.  `count` is a
 // monotonically increasing arrival counter (episode e completes when it
-// reaches e * nblocks, so it never needs resetting inside the launch);
-// `flag` holds the last released episode.  Partials and totals rotate over
-// four slots so a block running ahead never overwrites data still read.
+// reaches e * nblocks, so it never needs resetting inside the launch).  The
+// slots rotate over four sets so a block running ahead never overwrites
+// data still read; they are zeroed with the counter before the launch, so
+// that no slot carries an episode of an earlier one.
 struct GridSync {
-  unsigned int *count;
-  unsigned int *flag;
+  unsigned int *count;     // [0] arrivals of the sums and barriers; [8] (its
+                           // own 32-byte sector) publications (exchange_totals)
+  unsigned long long *xw;  // words of the exact sums (exact_sum), whole grids only
   int *err;                // sticky error (FVC_ERR_TIMEOUT on a stuck wait)
-  double *partials;        // 4 slots x kMaxNV x nblocks
-  double *totals;          // 4 slots x kMaxNV
+  RedSlot *slots;          // 4 sets x kMaxNV x nblocks
   unsigned int nblocks;    // blocks that synchronise through this state
   unsigned int base;       // blockIdx.x of the first of them (0 for a whole grid)
   // nonzero: the nblocks blocks are one thread-block cluster; the waits
@@ -86,13 +95,19 @@ struct GridSync {
   int cluster = 0;
 };
 
+// How often this launch has synchronised: reductions and barriers (the
+// episodes of the counter and the slots), published, and summed exactly.
+struct Episode {
+  unsigned int n = 0, pub = 0, x = 0;
+};
+
 constexpr int kMaxNV = 4;
 
 // The cluster form of a reduction.  Lane 0 of warp 0 of every CTA has
-// stored its block's NV partials in its own slot (mine); every thread of
-// every CTA then meets at the cluster barrier (arrive.release /
-// wait.acquire at cluster scope: the slots, and every global-memory write
-// made before it, are visible to the whole cluster after it); warp 0 reads
+// stored its block's NV partials in its own slot; every thread of every CTA
+// has then met at the cluster barrier (arrive.release / wait.acquire at
+// cluster scope: the slots, and every global-memory write made before it,
+// are visible to the whole cluster after it).  Here warp 0 reads
 // the CTAs' slots in rank order through distributed shared memory and sums
 // them in a fixed shuffle tree, so every CTA holds identical totals (in lane
 // 0 of warp 0).  There is no spin-wait: the barrier is the hardware's, and
@@ -103,18 +118,18 @@ constexpr int kMaxNV = 4;
 // no CTA's shared memory goes away while another reads it.
 template <int NV>
 __device__ __forceinline__ void cluster_exchange(double (*slots)[kMaxNV], unsigned int ep,
-                                                 double (&t)[NV > 0 ? NV : 1]) {
+                                                 double (&t)[NV]) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
-  cl.sync();
-  if (NV > 0 && threadIdx.x < 32) {
+  if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     const int nb = (int)cl.num_blocks();
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
       double u = (lane < nb) ? *cl.map_shared_rank(&slots[ep & 1u][q], lane) : 0.0;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) u = __dadd_rn(u, __shfl_down_sync(0xffffffffu, u, o));
+      for (int o = 8; o > 0; o >>= 1)  // at most 16 CTAs
+        u = __dadd_rn(u, __shfl_down_sync(0xffffffffu, u, o));
       t[q] = u;
     }
   }
@@ -131,27 +146,72 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 
-__device__ __forceinline__ unsigned int atom_add_acq_rel(unsigned int *p, unsigned int v) {
-  unsigned int old;
-  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-  return old;
-}
 __device__ __forceinline__ void red_add_release(unsigned int *p, unsigned int v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ void st_release(unsigned int *p, unsigned int v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void red_add_relaxed(unsigned int *p, unsigned int v) {
+  asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
   unsigned int v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ unsigned int ld_relaxed(const unsigned int *p) {
+  unsigned int v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_slot(RedSlot *p, double v, unsigned int ep) {
+  asm volatile(
+      "{\n .reg .b128 r;\n mov.b128 r, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], r;\n}" ::"l"(p),
+      "l"(__double_as_longlong(v)), "l"((unsigned long long)ep)
+      : "memory");
+}
+__device__ __forceinline__ RedSlot ld_slot(const RedSlot *p) {
+  RedSlot s;
+  asm volatile(
+      "{\n .reg .b128 r;\n ld.relaxed.gpu.global.b128 r, [%2];\n mov.b128 {%0, %1}, r;\n}"
+      : "=l"(s.v), "=l"(s.ep)
+      : "l"(p)
+      : "memory");
+  return s;
+}
 
 // Every wait is bounded: after kBarrierTimeoutNs the block records
 // FVC_ERR_TIMEOUT and leaves; the other waiters see the flag and leave too,
 // so a broken launch returns an error instead of spinning.
 constexpr uint64_t kBarrierTimeoutNs = 4000000000ull;  // 4 s
+
+// Waits until count reaches target; called by a whole warp.  kAcquire: what
+// the other blocks wrote before their release arrivals is visible afterwards.
+// All lanes poll, with a vote per turn: after a spin loop that a part of a
+// warp ran, the warp went on in pieces -- __syncwarp or not -- and a chain of
+// shuffles and FP64 additions took 2830 instead of 670 clocks.  The error word
+// and the clock are looked at every 64th poll only: in every poll they cost
+// another trip to L2 and delayed the hit by half of it.  False, with err set,
+// when the wait exceeded its bound.
+template <bool kAcquire>
+__device__ __forceinline__ bool wait_count(const unsigned int *count, int *err,
+                                           unsigned int target) {
+  unsigned int spins = 0;
+  uint64_t t0 = 0;
+  bool ok = true;
+  while (__any_sync(0xffffffffu,
+                    (kAcquire ? ld_acquire(count) : ld_relaxed(count)) < target)) {
+    if ((++spins & 63u) == 0) {
+      const uint64_t now = global_ns();
+      if (t0 == 0) t0 = now;
+      const bool late = now - t0 > kBarrierTimeoutNs;
+      if (__any_sync(0xffffffffu, late || *(volatile int *)err != 0)) {
+        if (late) atomicExch(err, 7 /* FVC_ERR_TIMEOUT */);
+        ok = false;
+        break;
+      }
+    }
+  }
+  return ok;
+}
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -181,212 +241,688 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *red) {
   __syncthreads();
 }
 
-// Grid-wide barrier (NV == 0) or deterministic all-reduce of NV doubles
-// per thread.  One arrival atomic per block; the last block to arrive sums
-// the per-block partials in block order (the same order whichever block is
-// last) and releases the others, which then read the NV totals.  Returns
-// false, with gs.err set, when a wait exceeded its bound.
-template <int NV>
-__device__ __forceinline__ bool grid_allreduce(const GridSync &gs, unsigned int &episode,
-                                               double (&v)[NV > 0 ? NV : 1], double *red) {
-  __shared__ int s_last, s_ok;
-  if (NV > 0) {
-    block_sum<(NV > 0 ? NV : 1)>(v, red);
-  } else {
-    __syncthreads();
+// The partials of one quantity summed in block order (lane l takes blocks
+// l, l + 32, ...): the same total in every block, valid in lane 0.  The
+// slots must hold their values (an acquire wait on count).
+__device__ __forceinline__ double sum_slots(const RedSlot *p, unsigned int nb) {
+  const unsigned int lane = threadIdx.x & 31;
+  double t = 0.0;
+#pragma unroll 1
+  for (unsigned int b = lane; b < nb; b += 32)
+    t = __dadd_rn(t, __longlong_as_double((long long)ld_slot(p + b).v));
+  return warp_sum(t);
+}
+
+// Grid-wide barrier that publishes every block's writes: one release
+// arrival per block, one acquire poll of the counter.  Returns false, with
+// gs.err set, when the wait exceeded its bound.
+__device__ __forceinline__ bool grid_barrier(const GridSync &gs, Episode &episode) {
+  __shared__ int s_ok;
+  __syncthreads();
+  const unsigned int ep = ++episode.n;
+  if (gs.cluster) {
+    cooperative_groups::this_cluster().sync();
+    return true;
   }
+  if (gs.nblocks == 1) return true;
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) red_add_release(gs.count, 1u);
+    const bool ok = wait_count<true>(gs.count, gs.err, ep * gs.nblocks);
+    if (threadIdx.x == 0) s_ok = ok ? 1 : 0;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// Deterministic all-reduce of NV doubles per thread, publishing the blocks'
+// writes like grid_barrier: every block sums the partials itself in block
+// order.  The totals are in every thread's v.
+template <int NV>
+__device__ __forceinline__ bool grid_allreduce(const GridSync &gs, Episode &episode,
+                                               double (&v)[NV], double *red) {
+  __shared__ int s_ok;
+  block_sum<NV>(v, red);
+  const unsigned int ep = ++episode.n;
   if (gs.cluster) {
     __shared__ double s_slot[2][kMaxNV];
-    const unsigned int ep = ++episode;
-    if (NV > 0 && threadIdx.x == 0)
+    if (threadIdx.x == 0)
 #pragma unroll
       for (int q = 0; q < NV; ++q) s_slot[ep & 1u][q] = v[q];
-    double t[NV > 0 ? NV : 1];
+    double t[NV];
+    cooperative_groups::this_cluster().sync();
     cluster_exchange<NV>(s_slot, ep, t);
-    if (NV > 0) {
-      if (threadIdx.x == 0)
+    if (threadIdx.x == 0)
 #pragma unroll
-        for (int q = 0; q < NV; ++q) red[q] = t[q];
-      __syncthreads();
+      for (int q = 0; q < NV; ++q) red[q] = t[q];
+  } else if (gs.nblocks == 1) {  // one block: its sum is the total (same value)
+    if (threadIdx.x == 0)
 #pragma unroll
-      for (int q = 0; q < NV; ++q) v[q] = red[q];
-      __syncthreads();
-    }
-    return true;
-  }
-  if (gs.nblocks == 1) {  // one block: its sum is the total (same value)
-    ++episode;
-    if (NV > 0) {
-      if (threadIdx.x == 0)
+      for (int q = 0; q < NV; ++q) red[q] = v[q];
+  } else {
+    const unsigned int nb = gs.nblocks;
+    RedSlot *part = gs.slots + (size_t)(ep & 3u) * kMaxNV * nb;
+    if (threadIdx.x < 32) {
+      if (threadIdx.x == 0) {
 #pragma unroll
-        for (int q = 0; q < NV; ++q) red[q] = v[q];
-      __syncthreads();
-#pragma unroll
-      for (int q = 0; q < NV; ++q) v[q] = red[q];
-      __syncthreads();
-    }
-    return true;
-  }
-  const unsigned int ep = ++episode;
-  const unsigned int nb = gs.nblocks;
-  double *part = gs.partials + (size_t)(ep & 3u) * kMaxNV * nb;
-  double *tot = gs.totals + (ep & 3u) * kMaxNV;
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) part[(size_t)q * nb + (blockIdx.x - gs.base)] = v[q];
-    const unsigned int old = atom_add_acq_rel(gs.count, 1u);
-    s_last = (old == ep * nb - 1u);
-    s_ok = 1;
-  }
-  __syncthreads();
-  if (s_last) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (NV > 0 && warp < NV) {
-      const double *p = part + (size_t)warp * nb;
-      double t = 0.0;
-      for (unsigned int b = lane; b < nb; b += 32) t = __dadd_rn(t, __ldcg(p + b));
-      t = warp_sum(t);
-      if (lane == 0) __stcg(tot + warp, t);
+        for (int q = 0; q < NV; ++q)
+          st_slot(part + (size_t)q * nb + (blockIdx.x - gs.base), v[q], ep);
+        red_add_release(gs.count, 1u);
+      }
+      const bool ok = wait_count<true>(gs.count, gs.err, ep * nb);
+      if (threadIdx.x == 0) s_ok = ok ? 1 : 0;
     }
     __syncthreads();
-    if (threadIdx.x == 0) st_release(gs.flag, ep);
-  } else if (threadIdx.x == 0) {
-    const uint64_t t0 = global_ns();
-    unsigned int spins = 0;
-    while (ld_acquire(gs.flag) < ep) {
-      if (*(volatile int *)gs.err != 0) {
-        s_ok = 0;
-        break;
-      }
-      if ((++spins & 255u) == 0 && global_ns() - t0 > kBarrierTimeoutNs) {
-        atomicExch(gs.err, 7 /* FVC_ERR_TIMEOUT */);
-        s_ok = 0;
-        break;
-      }
-      __nanosleep(20);
+    if (!s_ok) return false;
+    const int warp = threadIdx.x >> 5;
+    if (warp < NV) {
+      const double t = sum_slots(part + (size_t)warp * nb, nb);
+      if ((threadIdx.x & 31) == 0) red[warp] = t;
     }
   }
   __syncthreads();
-  if (!s_ok) return false;
 #pragma unroll
-  for (int q = 0; q < NV; ++q) v[q] = __ldcg(tot + q);
+  for (int q = 0; q < NV; ++q) v[q] = red[q];
+  __syncthreads();
   return true;
 }
 
-// Grid-wide deterministic sum of NV FP64 values per thread, for the FP64
-// solvers.  GB300 issues FP64 at ~2 lanes per clock per SM, so the block
-// sum avoids a butterfly in every warp (5 x 32 lanes x 32 warps adds):
-// the values go to shared memory (buf: NV x blockDim doubles), four warps
-// (one per SM sub-partition) add 8 values per lane each, warp 0 adds those
-// and finishes with a shuffle tree -- a fixed order, about 2.5x fewer FP64
-// instructions (blockDim.x must be a multiple of 128).  The block's
-// partial is published with a release add on the grid counter; every block waits for all arrivals and sums all
-// partials in block order itself.  Lane 0 of warp 0 then calls f(totals)
-// -- the place for the iteration's scalar FP64 work (one thread instead of
-// 1024) -- and one __syncthreads hands its results (through shared memory)
-// to the block.  Returns false when a wait exceeded its bound (gs.err set).
-template <int NV, typename F>
-__device__ __forceinline__ bool grid_allreduce_d(const GridSync &gs, unsigned int &episode,
-                                                 const double (&v)[NV], double *buf, F &&f) {
-  __shared__ int s_ok;
-  __shared__ double s_part[NV][128];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int bd = blockDim.x, per = bd >> 7;  // values per lane of the first level
+// The exchange of the grid-wide sums of the solvers (grid_sum_d and
+// grid_allreduce_ff).  Thread 0 puts its block's partial of each quantity
+// into its slots and counts itself in; every block then waits for all and
+// sums all partials itself in a fixed order, so that every block holds
+// identical totals.
+//
+// The arrival is relaxed, so that it does not wait for the block's stores to
+// be performed, and each partial carries its episode, so the slots need no
+// ordering against the counter (a slot read too early is read again); 152
+// blocks: 2.12 instead of 2.97 us for one double with 128 threads, 2.74
+// instead of 3.62 us with 1024, against a release arrival and an acquire
+// wait.  Polling the slots alone, without the counter, took 3.8 us: 152
+// blocks reading 2.4 KB over and over keep the writers off the same lines.
+template <int NV>
+__device__ __forceinline__ void grid_arrive(const GridSync &gs, unsigned int ep,
+                                            const double (&bsum)[NV]) {
+  const unsigned int nb = gs.nblocks;
+  RedSlot *part = gs.slots + (size_t)(ep & 3u) * kMaxNV * nb + (blockIdx.x - gs.base);
 #pragma unroll
-  for (int q = 0; q < NV; ++q) buf[q * bd + threadIdx.x] = v[q];
-  if (threadIdx.x == 0) s_ok = 1;
-  __syncthreads();
-  if (warp < 4) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      const double *b = buf + q * bd + warp * (bd >> 2) + lane;
-      double u = b[0];
-      for (int k = 1; k < per; ++k) u = __dadd_rn(u, b[32 * k]);
-      s_part[q][warp * 32 + lane] = u;
+  for (int q = 0; q < NV; ++q) st_slot(part + (size_t)q * nb, bsum[q], ep);
+  red_add_relaxed(gs.count, 1u);
+}
+
+// The partials of cnt blocks from slot i0 on into out (shared memory): the
+// whole block, one slot per thread.  (A lane's five slots held together cost the
+// solvers' loops spills, and the staged kernels, whose shared memory leaves no
+// L1, a third of their speed.)
+__device__ __forceinline__ void read_slots(const GridSync &gs, unsigned int ep, unsigned int i0,
+                                           unsigned int cnt, double *out) {
+  const RedSlot *p = gs.slots + (size_t)(ep & 3u) * kMaxNV * gs.nblocks + i0;
+  const unsigned int lane = threadIdx.x & 31u;
+#pragma unroll 1
+  for (unsigned int w = threadIdx.x - lane; w < cnt; w += blockDim.x) {
+    const unsigned int i = min(w + lane, cnt - 1);
+    RedSlot s = ld_slot(p + i);
+    unsigned int tries = 0;
+    // (the counter passed a slot's store: read again)
+    while (__any_sync(0xffffffffu, s.ep != ep)) {
+      if (++tries == (1u << 24)) {  // (seconds; a store takes none)
+        atomicExch(gs.err, 7 /* FVC_ERR_TIMEOUT */);
+        break;
+      }
+      s = ld_slot(p + i);
     }
+    if (w + lane < cnt) out[i] = __longlong_as_double((long long)s.v);
   }
-  __syncthreads();
-  const unsigned int ep = ++episode;
+}
+
+// The cluster barrier with mid() run by thread 0 between its arrival and its
+// wait (what it costs hides in the barrier's latency).
+template <typename M>
+__device__ __forceinline__ void cluster_sync_mid(M &&mid) {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  if (threadIdx.x == 0) mid();
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// The last step of both sums: thread 0 holds its block's partials.
+// kPublish: the blocks' vector writes before it are visible to the other
+// blocks after it, for a next phase that gathers them.  A second counter
+// carries that (release arrival and acquire wait of warp 2), beside the
+// partials and not before them: its wait for the block's stores hides in the
+// sum's two trips to L2.  tot: shared memory for cap partials of each quantity.
+template <int NV, bool kPublish, typename S, typename M, typename F>
+__device__ __forceinline__ bool exchange_totals(const GridSync &gs, Episode &episode,
+                                                const double (&bsum)[NV], double *tot,
+                                                unsigned int cap, S &&side, M &&mid, F &&f) {
+  __shared__ int s_ok[2];
+  __shared__ double s_t[NV];
+  if (kPublish) ++episode.pub;
+  const unsigned int ep = ++episode.n;
   if (gs.cluster) {
     __shared__ double s_slot[2][kMaxNV];
-    if (warp == 0) {
+    if (threadIdx.x == 0) {
 #pragma unroll
-      for (int q = 0; q < NV; ++q) {
-        double u = s_part[q][lane];
-#pragma unroll
-        for (int k = 1; k < 4; ++k) u = __dadd_rn(u, s_part[q][32 * k + lane]);
-        u = warp_sum(u);
-        if (lane == 0) s_slot[ep & 1u][q] = u;
-      }
+      for (int q = 0; q < NV; ++q) s_slot[ep & 1u][q] = bsum[q];
     }
+    if (threadIdx.x == 32) side();
+    __syncwarp();
+    cluster_sync_mid(mid);
     double t[NV];
     cluster_exchange<NV>(s_slot, ep, t);
     if (threadIdx.x == 0) f(t);
     __syncthreads();
     return true;
   }
-  if (warp == 0) {
-    const unsigned int nb = gs.nblocks;
-    double *part = gs.partials + (size_t)(ep & 3u) * kMaxNV * nb;
-    double bsum[NV];
+  if (gs.nblocks == 1) {  // one block: its sum is the total (same value)
+    if (threadIdx.x == 0) {
+      mid();
+      f(bsum);
+    } else if (threadIdx.x == 32) {
+      side();
+    }
+    __syncthreads();
+    return true;
+  }
+  const unsigned int nb = gs.nblocks;
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) {
+      grid_arrive<NV>(gs, ep, bsum);
+      mid();
+    }
+    const bool ok = wait_count<false>(gs.count, gs.err, ep * nb);
+    if (threadIdx.x == 0) s_ok[0] = ok ? 1 : 0;
+  } else if (threadIdx.x < 64) {
+    if (threadIdx.x == 32) side();
+  } else if (kPublish && threadIdx.x < 96) {
+    if (threadIdx.x == 64) red_add_release(gs.count + 8, 1u);
+    const bool ok = wait_count<true>(gs.count + 8, gs.err, episode.pub * nb);
+    if (threadIdx.x == 64) s_ok[1] = ok ? 1 : 0;
+  }
+  __syncthreads();
+  if (!s_ok[0] || (kPublish && !s_ok[1])) return false;
+  // the partials of quantity q in block order: lane l of warp q takes blocks
+  // l, l + 32, ... (from shared memory, cap at a time)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double u = 0.0;
+#pragma unroll 1
+  for (unsigned int b0 = 0; b0 < nb; b0 += cap) {
+    const unsigned int cnt = min(nb - b0, cap);
+#pragma unroll
+    for (int q = 0; q < NV; ++q) read_slots(gs, ep, q * nb + b0, cnt, tot + q * cap);
+    __syncthreads();
+    if (warp < NV) {
+      const double *p = tot + warp * cap;
+#pragma unroll 1
+      for (unsigned int b = lane; b < cnt; b += 128) {
+        double v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = (b + 32 * k < cnt) ? p[b + 32 * k] : 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (b + 32 * k < cnt) u = (b0 == 0 && b < 32 && k == 0) ? v[0] : __dadd_rn(u, v[k]);
+      }
+    }
+    if (b0 + cap < nb) __syncthreads();  // before tot is filled again
+  }
+  if (warp < NV) {
+    u = warp_sum(u);
+    if (lane == 0) s_t[warp] = u;
+  }
+  if (NV > 1) __syncthreads();
+  if (threadIdx.x == 0) f(s_t);
+  __syncthreads();
+  return true;
+}
+
+// Grid-wide deterministic sum of NV FP64 values per thread, for the FP64
+// solvers.  GB300 issues one FP64 warp instruction per 76 clocks and SM
+// sub-partition, whatever the active lanes, with 64 clocks of latency, so
+// the chain of dependent additions is what a sum costs.  The values go to
+// shared memory (buf: NV x blockDim doubles); four warps (one per
+// sub-partition) add blockDim / 128 values per lane in two chains and
+// finish with a shuffle tree; lane 0 of warp 0 adds the four (a fixed
+// order; blockDim.x must be a multiple of 128; 10 dependent additions for
+// 1024 threads).  The blocks' partials travel through grid_arrive /
+// grid_collect (or the cluster).  Lane 0 of warp 0 then calls f(totals) --
+// the place for the iteration's scalar FP64 work (one thread instead of
+// 1024) -- and one __syncthreads hands its results (through shared memory)
+// to the block.  Scalar work that needs nothing of this sum (a division is
+// 570 clocks) hides in the wait: thread 0 calls mid() between its arrival
+// and its wait, for values f uses; thread 32 calls side(), for values of
+// later phases.  Returns false when a wait exceeded its bound (gs.err set).
+template <int NV, bool kPublish, typename S, typename M, typename F>
+__device__ __forceinline__ bool grid_sum_d(const GridSync &gs, Episode &episode,
+                                           const double (&v)[NV], double *buf, S &&side, M &&mid,
+                                           F &&f) {
+  __shared__ double s_part[NV][4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int bd = blockDim.x, per = bd >> 7;  // values per lane of the first level
+#pragma unroll
+  for (int q = 0; q < NV; ++q) buf[q * bd + threadIdx.x] = v[q];
+  __syncthreads();
+  if (warp < 4) {
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
-      double u = s_part[q][lane];
-#pragma unroll
-      for (int k = 1; k < 4; ++k) u = __dadd_rn(u, s_part[q][32 * k + lane]);
-      bsum[q] = warp_sum(u);
-    }
-    bool ok = true;
-    double t[NV];
-    if (nb == 1) {  // one block: its sum is the total (same value)
-#pragma unroll
-      for (int q = 0; q < NV; ++q) t[q] = bsum[q];
-    } else {
-      if (lane == 0) {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) part[(size_t)q * nb + (blockIdx.x - gs.base)] = bsum[q];
-        red_add_release(gs.count, 1u);
-        const unsigned int target = ep * nb;
-        const uint64_t t0 = global_ns();
-        unsigned int spins = 0;
-        while (ld_acquire(gs.count) < target) {
-          if (*(volatile int *)gs.err != 0) {
-            ok = false;
-            break;
-          }
-          if ((++spins & 255u) == 0 && global_ns() - t0 > kBarrierTimeoutNs) {
-            atomicExch(gs.err, 7 /* FVC_ERR_TIMEOUT */);
-            ok = false;
-            break;
-          }
-          __nanosleep(20);
+      const double *b = buf + q * bd + warp * (bd >> 2) + lane;
+      double u = b[0];
+      if (per > 1) {
+        double u2 = b[32];
+#pragma unroll 1
+        for (int k = 2; k < per; k += 2) {
+          u = __dadd_rn(u, b[32 * k]);
+          if (k + 1 < per) u2 = __dadd_rn(u2, b[32 * k + 32]);
         }
+        u = __dadd_rn(u, u2);
       }
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-#pragma unroll
-      for (int q = 0; q < NV; ++q) {
-        double u = 0.0;
-        if (ok) {
-          const double *pp = part + (size_t)q * nb;
-          for (unsigned int b = lane; b < nb; b += 32) u = __dadd_rn(u, __ldcg(pp + b));
-        }
-        t[q] = warp_sum(u);
-      }
-    }
-    if (lane == 0) {
-      if (ok)
-        f(t);
-      else
-        s_ok = 0;
+      u = warp_sum(u);
+      if (lane == 0) s_part[q][warp] = u;
     }
   }
   __syncthreads();
-  return s_ok != 0;
+  double bsum[NV];
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+      bsum[q] = __dadd_rn(__dadd_rn(s_part[q][0], s_part[q][1]),
+                          __dadd_rn(s_part[q][2], s_part[q][3]));
+  return exchange_totals<NV, kPublish>(gs, episode, bsum, buf, bd, side, mid, f);
 }
 
-__device__ __forceinline__ bool grid_barrier(const GridSync &gs, unsigned int &episode) {
-  double none[1];
-  return grid_allreduce<0>(gs, episode, none, nullptr);
+// ---- scalar work of the recurrences ---------------------------------------
+// One thread does it between two phases, so its dependent FP64 instructions
+// (64 clocks each; a division 570, a square root 570) are the whole grid's
+// wait.
+
+// (Functions: their callers are one thread's code between two phases.)
+static __device__ __noinline__ double divide(double t, double d) { return t / d; }
+static __device__ __noinline__ double root(double v) { return sqrt(v); }
+
+// A divisor whose reciprocal was taken ahead of the dividend.
+struct Divisor {
+  double d, r;  // r = 1/d, or 0 when d is too far from 1 for quotient()
+  __device__ __forceinline__ void set(double v) {
+    d = v;
+    const int e = (__double2hiint(v) >> 20) & 0x7ff;
+    r = (e > 1023 - 500 && e < 1023 + 500) ? divide(1.0, v) : 0.0;
+  }
+};
+
+// t / d by Markstein's correction of t * (1/d) (IBM J. Res. Dev. 34, 1990):
+// three dependent FMAs after t instead of a division; within half an ulp and
+// a few parts in 2^53 of it.  Divisors out of range, and quotients that are
+// not finite, take the division.
+__device__ __forceinline__ double quotient(double t, const Divisor &v) {
+  const double q = t * v.r;
+  const double z = fma(fma(-q, v.d, t), v.r, q);
+  if (__double_as_longlong(v.r) == 0 || (__double2hiint(z) & 0x7ff00000) == 0x7ff00000)
+    return divide(t, v.d);
+  return z;
+}
+
+// The stopping test sqrt(s) < conv, without the square root while s is
+// clearly above conv^2 (bound from sqrt_bound; s >= 0 or NaN: the bits of
+// nonnegative doubles order like the numbers, a NaN above all of them).
+__device__ __forceinline__ long long sqrt_bound(double conv) {
+  const double c2 = conv * conv;
+  // conv^2 not a normal number: always take the square root
+  if (!(c2 > 1.0e-290 && c2 < 1.0e290)) return 0x7ff0000000000000ll;
+  return __double_as_longlong(c2 * (1.0 + 1.0e-14));
+}
+__device__ __forceinline__ bool sqrt_below(double s, double conv, long long bound) {
+  if (__double_as_longlong(s) > bound) return false;
+  return root(s) < conv;
+}
+__device__ __forceinline__ bool is_nan_bits(double v) {
+  return (__double_as_longlong(v) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ bool not_finite_bits(double v) {
+  return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000;
+}
+
+// No scalar work beside a sum.
+struct NoScalars {
+  __device__ void operator()() const {}
+};
+
+// ---- exact sums --------------------------------------------------------------
+// The sums above cost a chain of some 25 dependent FP64 additions (64 clocks
+// each) and the reading of every block's partial; at 66k rows the two sums of
+// a CG iteration were two thirds of it.  The sums below add integers instead.
+// Every thread splits its FP64 partial into kLimbs signed limbs of kLimbBits
+// bits of one fixed-point window that all blocks know (its top lies
+// kWindowHead bits above the total of the same sum one iteration ago); a
+// warp adds a limb with one redux, a block its warps' with another, and the
+// blocks add theirs into one 64-bit word per limb with relaxed atomics.
+// Integer addition is associative, so the total does not depend on the
+// order: deterministic, and exact but for the bits below the window (less
+// than 2^-53.7 of the total, see sum_bad) and the limbs' addition in FP64.  The word's upper bits count the
+// blocks that have added, so that one poll of the words is the whole
+// exchange: no slots, no counter, no order between them.  The words only
+// grow; a total is the difference to their value one use earlier (snap).
+//
+// A sum whose window does not hold it -- a partial at or above its top (or
+// NaN, Inf), or a total that has dropped by more than 2^22, the same verdict
+// in every block -- is taken again in a window set by the largest partial of
+// all blocks (window_by_partials), as is the first of a kind.
+//
+constexpr int kLimbs = 6, kLimbBits = 21, kWindowBits = kLimbs * kLimbBits, kWindowHead = 32;
+// Words of one set (two sets alternate): limb k of quantity q at 8 q + k, so
+// that the atomics of a block, and each poll of it, are one request.  With a
+// line of 128 bytes per word the polls of 152 blocks queued at the L2 slices
+// that held two of the words: sums of 4 thousand clocks became 9, depending on
+// the buffer's address.
+constexpr int kXWords = 32;
+constexpr int kNoWindow = INT_MIN;
+constexpr int kXBlocks = 2047;            // most blocks a word's count serves
+
+// A block's state of the exact sums (shared memory).
+struct ExactState {
+  unsigned long long snap[2][kXWords];
+  int ovf[32];
+  double tot[kMaxNV];
+  int top[kMaxNV];  // the window of the running sum
+  int flag, pub_ok;
+  int sure;  // that window follows from the partials
+  int nan;   // and some partial was NaN or Inf: so is the total
+};
+// The window of one kind of sum: its top, an exponent of two, per quantity.
+template <int NV>
+struct SumWindow {
+  int top[NV];
+};
+
+__device__ __forceinline__ int window_top(double total) {
+  const int e = (__double2hiint(total) >> 20) & 0x7ff;
+  // zero, subnormal, NaN or Inf, or near the ends of the exponents: none
+  return (e < 200 || e > 1800) ? kNoWindow : e - 1022 + kWindowHead;
+}
+template <int NV>
+__device__ __forceinline__ void window_set(SumWindow<NV> &w, const double *t) {
+#pragma unroll
+  for (int q = 0; q < NV; ++q) w.top[q] = window_top(t[q]);
+}
+
+// A warp's values +-m 2^e (m < 2^53; up to two per lane) as limbs of the window
+// with the given top, added over the warp and left in part[32 k + warp] for
+// limb k.  True in the lanes whose value does not fit.
+__device__ __forceinline__ bool add_limbs(int (&l)[kLimbs], unsigned long long m, int e, int neg,
+                                          int top) {
+  const int s = e - (top - kWindowBits);  // bit of the window m starts at
+  unsigned long long hi = 0, lo;
+  if (s >= 64) {
+    lo = 0;
+    hi = m << (s & 63);
+  } else if (s > 0) {
+    lo = m << s;
+    hi = m >> (64 - s);
+  } else {
+    lo = (s > -64) ? m >> -s : 0;
+  }
+  constexpr int M = (1 << kLimbBits) - 1;
+  const int x[kLimbs] = {(int)lo & M,
+                         (int)(lo >> 21) & M,
+                         (int)(lo >> 42) & M,
+                         (int)((lo >> 63) | (hi << 1)) & M,
+                         (int)(hi >> 20) & M,
+                         (int)(hi >> 41) & M};
+#pragma unroll
+  for (int k = 0; k < kLimbs; ++k) l[k] += (x[k] ^ -neg) + neg;
+  return s > kWindowBits - 53 - 1;
+}
+__device__ __forceinline__ void warp_limbs(const int (&l)[kLimbs], int *part) {
+  const int lane = threadIdx.x & 31;
+  int mine = 0;
+#pragma unroll
+  for (int k = 0; k < kLimbs; ++k) {
+    const int r = __reduce_add_sync(0xffffffffu, l[k]);
+    if (lane == k) mine = r;
+  }
+  if (lane < kLimbs) part[32 * lane + (threadIdx.x >> 5)] = mine;
+}
+__device__ __forceinline__ bool put_limbs(double v, int top, int *part) {
+  int l[kLimbs] = {0, 0, 0, 0, 0, 0};
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const int ex = (int)(b >> 52) & 0x7ff;
+  const unsigned long long m = (b & 0xfffffffffffffull) | ((unsigned long long)(ex != 0) << 52);
+  const bool ovf = add_limbs(l, m, (ex ? ex : 1) - 1075, (int)(b >> 63), top);
+  warp_limbs(l, part);
+  return ovf;
+}
+// The value of an FP32 pair, its parts renormalised so that they do not overlap
+__device__ __forceinline__ bool put_limbs(float s, float c, int top, int *part) {
+  int l[kLimbs] = {0, 0, 0, 0, 0, 0};
+  const float hi = __fadd_rn(s, c);
+  const float lo = __fsub_rn(c, __fsub_rn(hi, s));
+  bool ovf = false;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const unsigned int b = __float_as_uint(k ? lo : hi);
+    const int ex = (int)(b >> 23) & 0xff;
+    const unsigned int m = (b & 0x7fffffu) | ((unsigned int)(ex != 0) << 23);
+    // NaN and Inf: an exponent no window holds
+    const int e = ex == 0xff ? 4096 : (ex ? ex : 1) - 150;
+    ovf = add_limbs(l, (unsigned long long)m, e, (int)(b >> 31), top) || ovf;
+  }
+  warp_limbs(l, part);
+  return ovf;
+}
+
+// Limb k of a total in FP64: L 2^(21 k) units of the window, exact (|L| <
+// 2^41) unless it leaves FP64's exponents (then 0 or Inf).
+__device__ __forceinline__ double limb_value(long long L, int k, int top) {
+  const double v = (double)L;
+  const int hi = __double2hiint(v), sh = top - kWindowBits + kLimbBits * k;
+  const int e = ((hi >> 20) & 0x7ff) + sh;
+  if (L == 0 || e <= 0) return 0.0;
+  if (e >= 0x7ff) return __hiloint2double((hi & 0x80000000) | 0x7ff00000, 0);
+  return __hiloint2double(hi + (sh << 20), __double2loint(v));
+}
+// Whether a total lies so low in its window that what the threads dropped
+// below it (up to 2^18.3 threads, less than one unit each) could matter:
+// below 2^72 units.
+__device__ __forceinline__ bool sum_bad(double t, int top) {
+  const int e = ((__double2hiint(t) >> 20) & 0x7ff) - 1023;
+  return e < top - kWindowBits + 72;
+}
+
+__device__ __forceinline__ void exact_init(ExactState &xs) {  // a __syncthreads must follow
+#pragma unroll 1
+  for (int i = threadIdx.x; i < 2 * kXWords; i += blockDim.x) (&xs.snap[0][0])[i] = 0;
+}
+
+// The window of a sum from its partials: its top above the largest exponent
+// (ex, biased) of all threads of all blocks, by a maximum exchanged through
+// the reduction slots and a barrier.  Cold: the first sum of a kind, and one
+// that its window did not hold.  False when a wait exceeded its bound.
+static __device__ __noinline__ bool window_by_partials(const GridSync &gs, Episode &episode,
+                                                       ExactState &xs, int *top, int nv,
+                                                       const int *ex, int *part) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const unsigned int ep = ++episode.n;
+  __shared__ int s_ok;
+  RedSlot *slots = gs.slots + (size_t)(ep & 3u) * kMaxNV * gs.nblocks;
+  __syncthreads();  // part is free
+  for (int q = 0; q < nv; ++q) {
+    const int m = __reduce_max_sync(0xffffffffu, ex[q]);
+    if (lane == 0) part[q * 32 + warp] = m;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 0; q < nv; ++q) {
+      int m = 0;
+      for (int w = 0; w < nw; ++w) m = max(m, part[q * 32 + w]);
+      st_slot(slots + (size_t)q * gs.nblocks + blockIdx.x, (double)m, ep);
+    }
+    // (one block counts no arrivals, see grid_barrier)
+    if (gs.nblocks > 1) red_add_release(gs.count, 1u);
+  }
+  if (warp == 0) {
+    const bool ok = gs.nblocks == 1 || wait_count<true>(gs.count, gs.err, ep * gs.nblocks);
+    if (lane == 0) s_ok = ok ? 1 : 0;
+  }
+  __syncthreads();
+  if (!s_ok) return false;
+  if (warp == 0) {
+    bool nan = false;
+    for (int q = 0; q < nv; ++q) {
+      int m = 0;
+      for (unsigned int b = lane; b < gs.nblocks; b += 32)
+        m = max(m, (int)__longlong_as_double((long long)ld_slot(slots + (size_t)q * gs.nblocks + b).v));
+      m = __reduce_max_sync(0xffffffffu, m);
+      nan = nan || m == 0x7ff;
+      // |partial| < 2^(m - 1022)
+      if (lane == 0) top[q] = max(min(m, 0x7fe), 1) - 1022 + 1;
+    }
+    if (lane == 0) xs.nan = nan ? 1 : 0;
+  }
+  __syncthreads();
+  return true;
+}
+
+// Warp 0's part of an exact sum of nv quantities: the block's limbs from its
+// warps' (part), their exchange through the words, the totals into xs.tot and
+// the verdict into xs.flag (0 a wait exceeded its bound, 1 good, 2 the window
+// did not hold it).
+__device__ __forceinline__ void exact_words(unsigned long long *xw, int *err, unsigned int nb,
+                                                unsigned int set, int nv, const int *part,
+                                                ExactState &xs) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  // lane 8 q + k holds limb k of quantity q
+  const int lq = lane >> 3, lk = lane & 7;
+  const bool mine = lq < nv && lk < kLimbs;
+  long long w = 0;
+#pragma unroll 1
+  for (int q = 0; q < nv; ++q)
+#pragma unroll
+    for (int k = 0; k < kLimbs; ++k) {
+      const int r =
+          __reduce_add_sync(0xffffffffu, lane < nw ? part[(q * kLimbs + k) * 32 + lane] : 0);
+      if (lane == 8 * q + k) w = r;
+    }
+  const bool o = __any_sync(0xffffffffu, lane < nw && xs.ovf[lane] != 0);
+  long long L = 0;
+  bool ok = true, bad = false;
+  // (the other lanes poll along on the first word, see wait_count)
+  unsigned long long *word = xw + set * kXWords + (mine ? lane : 0);
+  const int top = xs.top[mine ? lq : 0];
+  if (mine)  // bits 0-41 the limb, 42-52 blocks that overflowed, 53-63 blocks
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(word),
+                 "l"(w + ((long long)(o ? 1 : 0) << 42) + (1ll << 53))
+                 : "memory");
+  const unsigned long long prev = xs.snap[set][mine ? lane : 0];
+  __syncwarp();
+  unsigned long long now;
+  unsigned int spins = 0;
+  uint64_t t0 = 0;
+  for (;;) {
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(word) : "memory");
+    const long long d = (long long)(now - prev);
+    L = (long long)((unsigned long long)d << 22) >> 22;
+    const long long c = (d - L) >> 42;
+    bad = (c & 2047) != 0;
+    if (__all_sync(0xffffffffu, (unsigned int)(c >> 11) == nb)) break;
+    if ((++spins & 63u) == 0) {
+      const uint64_t ns = global_ns();
+      if (t0 == 0) t0 = ns;
+      const bool late = ns - t0 > kBarrierTimeoutNs;
+      if (__any_sync(0xffffffffu, late || *(volatile int *)err != 0)) {
+        if (late) atomicExch(err, 7 /* FVC_ERR_TIMEOUT */);
+        ok = false;
+        break;
+      }
+    }
+  }
+  if (mine) xs.snap[set][lane] = now;
+  __syncwarp();
+  // the limbs of a quantity added in FP64
+  double tq = mine ? limb_value(L, lk, top) : 0.0;
+#pragma unroll
+  for (int k = 1; k < 8; k <<= 1) tq = __dadd_rn(tq, __shfl_xor_sync(0xffffffffu, tq, k));
+  if (xs.sure) {
+    bad = false;  // only NaN and Inf overflow a window that follows from the partials
+    if (xs.nan) tq = __longlong_as_double(0x7ff8000000000000ll);
+  } else {
+    bad = bad || (mine && sum_bad(tq, top));
+  }
+  bad = __any_sync(0xffffffffu, bad);
+  ok = __all_sync(0xffffffffu, ok);
+  if (lk == 0 && lq < nv) xs.tot[lq] = tq;
+  if (lane == 0) xs.flag = !ok ? 0 : bad ? 2 : 1;
+  __syncwarp();
+}
+
+// Warps 0 and 1 of the block meet (the values of side() for f()).
+__device__ __forceinline__ void join_warps01() {
+  __syncwarp();
+  asm volatile("barrier.sync 1, 64;" ::: "memory");
+}
+
+// Grid-wide deterministic sum of NV values per thread: put(q, top, part) leaves
+// the limbs of the warp's values of quantity q (put_limbs), expo(q) gives the
+// value's biased FP64 exponent.  part: shared memory for NV * kLimbs * 32
+// ints.  win: the window of this kind of sum.  Thread 0 calls f(totals) as in
+// grid_sum_d; thread 32 calls side() while warp 0 exchanges (kJoin: for values
+// f uses).  kPublish: as in exchange_totals.  Returns false when a wait
+// exceeded its bound (gs.err set).
+template <int NV, bool kPublish, bool kJoin, typename C, typename X, typename S, typename F>
+__device__ __forceinline__ bool exact_sum(const GridSync &gs, Episode &episode, ExactState &xs,
+                                          SumWindow<NV> &win, int *part, C &&put, X &&expo,
+                                          S &&side, F &&f) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (kPublish) ++episode.pub;
+  bool first = true, have = true;
+#pragma unroll
+  for (int q = 0; q < NV; ++q) have = have && win.top[q] != kNoWindow;
+#pragma unroll 1
+  for (;;) {
+    if (!have) {
+      int ex[NV];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) ex[q] = expo(q);
+      if (!window_by_partials(gs, episode, xs, win.top, NV, ex, part)) return false;
+    }
+    const unsigned int set = (episode.x++) & 1u;
+    bool ovf = false;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) ovf = put(q, win.top[q], part + q * kLimbs * 32) || ovf;
+    ovf = __any_sync(0xffffffffu, ovf);
+    if (lane == 0) xs.ovf[warp] = ovf ? 1 : 0;
+    if (threadIdx.x < NV) xs.top[threadIdx.x] = win.top[threadIdx.x];
+    if (threadIdx.x == 0) xs.sure = have ? 0 : 1;
+    __syncthreads();
+    if (warp == 0) {
+      exact_words(gs.xw, gs.err, gs.nblocks, set, NV, part, xs);
+      if (kJoin && first) join_warps01();
+      if (lane == 0 && xs.flag == 1) {
+        window_set<NV>(win, xs.tot);
+        f(xs.tot);
+      }
+    } else if (warp == 1) {
+      if (lane == 0 && first) side();
+      if (kJoin && first) join_warps01();
+    } else if (kPublish && warp == 2 && first) {
+      if (lane == 0) red_add_release(gs.count + 8, 1u);
+      const bool ok = wait_count<true>(gs.count + 8, gs.err, episode.pub * gs.nblocks);
+      if (lane == 0) xs.pub_ok = ok ? 1 : 0;
+    }
+    __syncthreads();
+    if (kPublish && !xs.pub_ok) return false;
+    const int r = xs.flag;
+    if (r != 2) return r == 1;
+    first = false;
+    have = false;
+  }
+}
+
+// exact_sum of FP64 partials; buf: NV x blockDim doubles of shared memory.
+template <int NV, bool kPublish, bool kJoin, typename S, typename F>
+__device__ __forceinline__ bool grid_sum_x(const GridSync &gs, Episode &episode, ExactState &xs,
+                                           SumWindow<NV> &win, const double (&v)[NV], double *buf,
+                                           S &&side, F &&f) {
+  return exact_sum<NV, kPublish, kJoin>(
+      gs, episode, xs, win, reinterpret_cast<int *>(buf),
+      [&](int q, int top, int *part) { return put_limbs(v[q], top, part); },
+      [&](int q) { return (__double2hiint(v[q]) >> 20) & 0x7ff; }, side, f);
 }
 
 // Streaming loads of read-only matrix data (never written by the kernel
@@ -487,9 +1023,11 @@ __device__ __forceinline__ double sell_row_f64(const SellView<double> &A, int s,
   };
   if (A.diag_mode == DIAG_LAST) {
     t = __dmul_rn(ld_stream(vp), xf(colk(0)));
+#pragma unroll 1
     for (int k = 1; k < w; ++k) t = __dadd_rn(t, __dmul_rn(ld_stream(vp + 32 * k), xf(colk(k))));
     return __dadd_rn(t, xd);
   }
+#pragma unroll 1
   for (int k = 0; k < w; ++k) t = __dadd_rn(t, __dmul_rn(ld_stream(vp + 32 * k), xf(colk(k))));
   return t;
 }
@@ -522,6 +1060,7 @@ __device__ __forceinline__ double sell_row_fma(const SellView<double> &A, int s,
     for (int k = 0; k < 4; ++k)
       if (k < w) t = fma(a[k], xf(c[k]), t);
   } else {
+#pragma unroll 1
     for (int k = 0; k < w; ++k) {
       int c = ld_stream(cp + 32 * k);
       FVC_CHK((unsigned)c < (unsigned)A.n, A.chk, kChkColumn, c = row);
@@ -592,6 +1131,7 @@ __device__ __forceinline__ double sell_row_fma_t(const SellView<double> &A, int 
     for (int k = 0; k < 4; ++k)
       if (k < w) t = fma(A.val[m[k]], xf(c[k]), t);
   } else {
+#pragma unroll 1
     for (int k = 0; k < w; ++k) {
       int c = ld_stream(cp + 32 * k), m = ld_stream(mp + 32 * k);
       FVC_CHK((unsigned)c < (unsigned)A.n, A.chk, kChkColumn, c = row);
@@ -611,20 +1151,33 @@ __device__ __forceinline__ double row_fma(const SellView<double> &A, int s, int 
 }
 
 // Host side: scratch for the grid synchronisation of a persistent launch.
+// One buffer: counter (64 bytes) | error block (64) | result (16 doubles) |
+// iresult (16 ints) | padding | the words of the exact sums | the reduction
+// slots; one memset clears it.
+constexpr size_t kXBytes = 2 * (size_t)kXWords * sizeof(unsigned long long);
+constexpr size_t kSyncHead = 512 + kXBytes;
+static_assert(64 + 64 + 16 * sizeof(double) + 16 * sizeof(int) <= 512, "sync header");
+constexpr size_t kSyncBlocks = 1280;  // blocks the first allocation serves
+
+inline size_t slot_bytes(size_t nblocks) { return 4 * kMaxNV * nblocks * sizeof(RedSlot); }
+
 inline int32_t ensure_sync(Scratch &S, size_t nblocks) {
-  const size_t need = 4 * kMaxNV * nblocks + 4 * kMaxNV;
-  if (S.npart < need) {
-    if (S.partials) cudaFree(S.partials);
-    S.partials = nullptr;
-    if (cudaMalloc(&S.partials, sizeof(double) * need) != cudaSuccess) return FVC_ERR_CUDA;
-    S.npart = need;
-  }
-  if (!S.sync) {
-    if (cudaMalloc(&S.sync, 64) != cudaSuccess) return FVC_ERR_CUDA;
-    if (cudaMalloc(&S.err, 64) != cudaSuccess || cudaMemset(S.err, 0, 64) != cudaSuccess)
+  if (S.nslot < nblocks) {
+    const size_t cap = std::max(nblocks, kSyncBlocks);
+    if (S.sync) cudaFree(S.sync);
+    S.sync = nullptr;
+    S.nslot = 0;
+    char *buf = nullptr;
+    if (cudaMalloc(&buf, kSyncHead + slot_bytes(cap)) != cudaSuccess ||
+        cudaMemset(buf, 0, kSyncHead) != cudaSuccess)
       return FVC_ERR_CUDA;
-    if (cudaMalloc(&S.result, 16 * sizeof(double)) != cudaSuccess) return FVC_ERR_CUDA;
-    if (cudaMalloc(&S.iresult, 16 * sizeof(int)) != cudaSuccess) return FVC_ERR_CUDA;
+    S.sync = reinterpret_cast<unsigned int *>(buf);
+    S.err = reinterpret_cast<int *>(buf + 64);
+    S.result = reinterpret_cast<double *>(buf + 128);
+    S.iresult = reinterpret_cast<int *>(buf + 128 + 16 * sizeof(double));
+    S.nslot = cap;
+  }
+  if (!S.trace) {
     if (cudaMalloc(&S.trace, 2 * kTraceMax * sizeof(double)) != cudaSuccess) return FVC_ERR_CUDA;
     if (cudaMalloc(&S.history, kHistoryMax * sizeof(float)) != cudaSuccess) return FVC_ERR_CUDA;
   }
@@ -634,10 +1187,9 @@ inline int32_t ensure_sync(Scratch &S, size_t nblocks) {
 inline GridSync make_sync(const Scratch &S, int nblocks) {
   GridSync g;
   g.count = S.sync;
-  g.flag = S.sync + 8;  // separate 32-byte sector from the counter
   g.err = S.err;
-  g.partials = S.partials;
-  g.totals = S.partials + 4 * kMaxNV * (size_t)nblocks;
+  g.xw = reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(S.sync) + 512);
+  g.slots = reinterpret_cast<RedSlot *>(reinterpret_cast<char *>(S.sync) + kSyncHead);
   g.nblocks = (unsigned int)nblocks;
   g.base = 0;
   return g;
@@ -652,11 +1204,10 @@ inline GridSync make_sync(const Scratch &S, int nblocks) {
 inline int *check_word(const Scratch &S) { return S.err ? S.err + 8 : nullptr; }
 int32_t check_word_status(const Scratch &S, cudaStream_t stream);
 
-inline void reset_sync(Scratch &S, cudaStream_t stream) {
-  cudaMemsetAsync(S.sync, 0, 64, stream);
-  cudaMemsetAsync(S.err, 0, 64, stream);
-  cudaMemsetAsync(S.iresult, 0, 16 * sizeof(int), stream);
-  cudaMemsetAsync(S.result, 0, 16 * sizeof(double), stream);
+// The counter, error block, results and the slots of nblocks blocks start
+// at zero (nblocks 0: a launch that reduces through its cluster).
+inline void reset_sync(Scratch &S, cudaStream_t stream, size_t nblocks) {
+  cudaMemsetAsync(S.sync, 0, kSyncHead + slot_bytes(nblocks), stream);
 }
 
 }  // namespace fvc

@@ -58,11 +58,10 @@ struct Scratch {
   double *v[kVec] = {nullptr};  // Krylov vectors
   float *f[10] = {nullptr};     // FP32 vectors (mixed precision)
   double *g = nullptr;          // GMRES basis (k+1) x n
-  double *partials = nullptr;   // reduction partials
-  size_t npart = 0;
-  unsigned int *sync = nullptr; // barrier counter + generation
-  int *err = nullptr;
-  double *result = nullptr;     // solver scalars written by block 0
+  unsigned int *sync = nullptr; // one buffer: arrival counter, error block,
+  size_t nslot = 0;             // results and the reduction slots of nslot blocks
+  int *err = nullptr;           // ... its error block
+  double *result = nullptr;     // ... solver scalars written by block 0
   int *iresult = nullptr;
   double *trace = nullptr;      // per residual replacement: (iteration, ||r||/||b||)
   float *history = nullptr;     // per iteration: recursive ||r||/||b|| (first kHistoryMax)

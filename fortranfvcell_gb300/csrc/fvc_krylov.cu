@@ -28,6 +28,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "fvc_device.cuh"
@@ -80,15 +81,13 @@ struct Part {
   }
 };
 
+// (Not unrolled: a solver's loop runs each phase once per iteration over a
+// few rows per thread; unrolled by the compiler the PCG kernel had 103 KB of
+// code, and the BiCGSTAB of 262k rows took 2 % longer.)
 #define FOR_ROWS(P)                                          \
+  _Pragma("unroll 1")                                        \
   for (int s_ = (P).sb + (P).warp; s_ < (P).se; s_ += (P).nwarps) \
     for (int row = s_ * 32 + (P).lane, once_ = 1; once_ && row < (P).n; once_ = 0)
-
-template <int NV>
-__device__ __forceinline__ bool reduce(const KArgs &a, unsigned int &ep, double (&v)[NV],
-                                       double *red) {
-  return grid_allreduce<NV>(a.gs, ep, v, red);
-}
 
 __device__ __forceinline__ void finish_to(double *result, int *iresult, bool lead, int iters,
                                           int status, double conv, double crit, int inner) {
@@ -106,13 +105,26 @@ __device__ __forceinline__ void finish(const KArgs &a, int iters, int status,
   finish_to(a.result, a.iresult, blockIdx.x == 0, iters, status, conv, crit, inner);
 }
 
+// The sums of the solver bodies: exact ones over a whole grid (kX), those of
+// grid_sum_d for the groups and clusters of a batch and the cluster kernels.
+// side: scalars of later phases, mid: scalars f uses (thread 0 or 32).
+template <bool kX, int NV, bool kPublish, typename S, typename M, typename F>
+__device__ __forceinline__ bool sum_rows(const GridSync &gs, Episode &ep, ExactState &xs,
+                                         SumWindow<NV> &win, const double (&v)[NV], double *buf,
+                                         S &&side, M &&mid, F &&f) {
+  constexpr bool kMid = !std::is_same<std::decay_t<M>, NoScalars>::value;
+  if (!kX) return grid_sum_d<NV, kPublish>(gs, ep, v, buf, side, mid, f);
+  if (kMid) return grid_sum_x<NV, kPublish, true>(gs, ep, xs, win, v, buf, mid, f);
+  return grid_sum_x<NV, kPublish, false>(gs, ep, xs, win, v, buf, side, f);
+}
+
 // Energy norm x.Ax and the FP64 residual ||b-Ax||^2, ||b||^2 in one pass
 // over the rows of P (x must be complete at every row: called right after
-// a synchronisation of gs); the lead block writes result[0, 3, 4].
-template <bool kT = false>
-__device__ __forceinline__ bool epilogue_to(const KArgs &a, const Part &P, const GridSync &gs,
-                                            double *result, bool lead, unsigned int &ep,
-                                            double *red, bool energy_xb) {
+// a synchronisation of gs); sum adds the three over the blocks and thread 0
+// of the lead block writes result[0, 3, 4].
+template <bool kT = false, typename Sum>
+__device__ __forceinline__ void epilogue_to(const KArgs &a, const Part &P, double *result,
+                                            bool lead, bool energy_xb, Sum &&sum) {
   double acc[3] = {0.0, 0.0, 0.0};
   const double *x = a.x;
   FOR_ROWS(P) {
@@ -123,19 +135,13 @@ __device__ __forceinline__ bool epilogue_to(const KArgs &a, const Part &P, const
     acc[1] = fma(rr, rr, acc[1]);
     acc[2] = fma(bi, bi, acc[2]);
   }
-  if (!grid_allreduce<3>(gs, ep, acc, red)) return false;
-  if (lead && threadIdx.x == 0) {
-    result[0] = acc[0];
-    result[3] = acc[1];
-    result[4] = acc[2];
-  }
-  return true;
-}
-
-__device__ __forceinline__ bool epilogue(const KArgs &a, unsigned int &ep, double *red,
-                                         bool energy_xb) {
-  return epilogue_to(a, Part(a.A.nslices, a.A.n), a.gs, a.result, blockIdx.x == 0, ep, red,
-                     energy_xb);
+  sum(acc, [&](const double *t) {
+    if (lead) {
+      result[0] = t[0];
+      result[3] = t[1];
+      result[4] = t[2];
+    }
+  });
 }
 
 // ---------------------------------------------------------------------
@@ -152,21 +158,30 @@ __device__ __forceinline__ bool epilogue(const KArgs &a, unsigned int &ep, doubl
 // and z, which saves the barrier.  Both give the same bits.
 // kMaxT: the most threads per block the kernel is launched with (the
 // reductions' staging buffer holds that many values per reduced quantity).
-template <bool kStoreP, int kMaxT = 1024>
+template <bool kStoreP, int kMaxT = 1024, bool kX = true>
 __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const GridSync &gs,
                                         double *result, int *iresult, bool lead) {
-  __shared__ double red[kMaxNV * 32];
-  __shared__ double buf[2 * kMaxT];
+  __shared__ double buf[3 * kMaxT];
   // scalars of the recurrence, updated by lane 0 of warp 0 inside the
   // all-reduces and read by every thread after them
   __shared__ struct {
-    double d, alpha, beta, conv, crit;
-    int stop;  // 0 go on, 1 converged, 2 NaN/Inf
+    double d, alpha, beta, conv, rr;
+    Divisor dv;       // d, its reciprocal taken while the p.q sum travels
+    long long bound;  // of the stopping test (sqrt_bound)
+    int stop;         // 0 go on, 1 converged, 2 NaN/Inf
   } sh;
+  __shared__ ExactState xs;
+  __shared__ SumWindow<1> wpq;
+  __shared__ SumWindow<1> wrz;
+  __shared__ SumWindow<2> wrr;
+  exact_init(xs);
+  if (threadIdx.x == 0) wpq.top[0] = wrz.top[0] = wrr.top[0] = kNoWindow;
+  __syncthreads();
   double *r = a.v0, *z = a.v1, *q = a.v4, *x = a.x;
+  const NoScalars none;
   const double *minv = a.minv, *b = a.b;
   const bool rule0 = a.stop_rule == 0;
-  unsigned int ep = 0;
+  Episode ep;
 
   // r = b - A x ; z = r/m ; p = z ; d = r.z  (x = 0 when init)
   double acc[2] = {0.0, 0.0};
@@ -181,20 +196,25 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
     const double ri = b[row] - ax;
     const double zi = ri * minv[row];
     r[row] = ri;
+    z[row] = zi;
     a.v2[row] = zi;
     acc[0] = fma(ri, zi, acc[0]);
     acc[1] = fma(b[row], b[row], acc[1]);
   }
-  if (!grid_allreduce_d<2>(gs, ep, acc, buf, [&](const double *t) {
+  if (!sum_rows<kX, 2, true>(gs, ep, xs, wrr, acc, buf, none, none, [&](const double *t) {
         sh.d = t[0];
-        sh.conv = rule0 ? a.tol * sqrt(fabs(t[0])) : a.tol * sqrt(t[1]);
+        sh.conv = a.tol * root(rule0 ? fabs(t[0]) : t[1]);
+        sh.bound = sqrt_bound(sh.conv);
         sh.beta = 0.0;
-        sh.crit = 0.0;
+        sh.rr = 0.0;
         sh.stop = 0;
+        wrz.top[0] = window_top(t[0]);
+        wrr.top[1] = kNoWindow;
       }))
     return;
 
-  double *pprev = a.v2, *pcur = a.v2;
+  // the first p = z + 0 p_prev (p_prev = z): no case of its own in the loop
+  double *pprev = a.v2, *pcur = kStoreP ? a.v2 : a.v3;
   double beta = 0.0;
   int j, status = FVC_OK;
   for (j = 1; j <= a.maxit; ++j) {
@@ -204,7 +224,7 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
       FOR_ROWS(P) pcur[row] = fma(beta, pcur[row], z[row]);
       if (!grid_barrier(gs, ep)) return;
     }
-    if (j == 1 || kStoreP) {
+    if (kStoreP) {
       FOR_ROWS(P) {
         const double *pc = pcur;
         const double qi = sell_row_fma(a.A, s_, P.lane, row, [&](int k) { return pc[k]; });
@@ -222,8 +242,10 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
         pq[0] = fma(pi, qi, pq[0]);
       }
     }
-    if (!grid_allreduce_d<1>(gs, ep, pq, buf,
-                             [&](const double *t) { sh.alpha = sh.d / t[0]; }))
+    // what follows touches own rows only: nothing to publish
+    if (!sum_rows<kX, 1, false>(
+            gs, ep, xs, wpq, pq, buf, [&] { sh.dv.set(sh.d); }, none,
+            [&](const double *t) { sh.alpha = divide(sh.d, t[0]); }))
       return;
     const double alpha = sh.alpha;
     // x += alpha p ; r -= alpha q ; z = r/m ; r.z (and r.r for stop_rule 1)
@@ -241,15 +263,20 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
         rr2[1] = fma(ri, ri, rr2[1]);
       }
     }
-    // beta = r.z / d ; d = beta d ; the reference's stopping test
+    // beta = r.z / d ; d = beta d ; the reference's stopping test.  The sum
+    // publishes z where the next SpMV gathers it (with a stored p the
+    // barrier before that SpMV publishes p)
     auto step = [&](const double *t) {
-      sh.beta = t[0] / sh.d;
+      sh.beta = quotient(t[0], sh.dv);
       sh.d = sh.beta * sh.d;
-      sh.crit = rule0 ? sqrt(fabs(sh.d)) : sqrt(t[1]);
-      sh.stop = (!(sh.crit == sh.crit) || isinf(sh.d)) ? 2 : (sh.crit < sh.conv ? 1 : 0);
+      const double crit2 = rule0 ? fabs(sh.d) : t[rule0 ? 0 : 1];
+      sh.rr = crit2;
+      sh.stop = (is_nan_bits(crit2) || not_finite_bits(sh.d)) ? 2
+                : sqrt_below(crit2, sh.conv, sh.bound)        ? 1
+                                                              : 0;
     };
-    const bool ok = rule0 ? grid_allreduce_d<1>(gs, ep, rz, buf, step)
-                          : grid_allreduce_d<2>(gs, ep, rr2, buf, step);
+    const bool ok = rule0 ? sum_rows<kX, 1, !kStoreP>(gs, ep, xs, wrz, rz, buf, none, none, step)
+                          : sum_rows<kX, 2, !kStoreP>(gs, ep, xs, wrr, rr2, buf, none, none, step);
     if (!ok) return;
     if (sh.stop == 2) {
       status = FVC_ERR_NAN;
@@ -266,8 +293,14 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
     j = a.maxit;
     status = FVC_ERR_NOCONV;
   }
-  finish_to(result, iresult, lead, j, status, sh.conv, sh.crit, 0);
-  epilogue_to(a, P, gs, result, lead, ep, red, false);
+  finish_to(result, iresult, lead, j, status, sh.conv, root(sh.rr), 0);
+  if (!grid_barrier(gs, ep)) return;  // x of every row before the epilogue's SpMV
+  __shared__ SumWindow<3> we;
+  if (threadIdx.x == 0) we.top[0] = kNoWindow;
+  __syncthreads();
+  epilogue_to(a, P, result, lead, false, [&](const double(&v)[3], auto f) {
+    sum_rows<kX, 3, false>(gs, ep, xs, we, v, buf, none, none, f);
+  });
 }
 
 constexpr int kStorePRows = 262144;
@@ -302,13 +335,14 @@ __global__ void __launch_bounds__(1024, 1) pcg_f64(KArgs a) {
 // them -- five synchronisations per iteration instead of three, about half
 // the FP64 instructions (a gathered neighbour costs one FMA instead of
 // three or two), the same bits.
-template <int kMaxT = 1024, bool kT = false, bool kStoreZ = false>
+template <int kMaxT = 1024, bool kT = false, bool kStoreZ = false, bool kX = true>
 __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, const GridSync &gs,
                                              double *result, int *iresult, bool lead) {
-  __shared__ double red[kMaxNV * 32];
   __shared__ double buf[3 * kMaxT];
   __shared__ struct {
-    double d, conv, rr0, alpha, w, beta, crit;
+    double d, conv, rr0, alpha, w, aw, beta, crit2;
+    Divisor dv, rv;   // d, and this iteration's s.r
+    long long bound;  // of the stopping test (sqrt_bound)
     int stop;     // 0 go on, 1 converged, 2 NaN/Inf, 3 breakdown
     int restart;  // a breakdown: the next iteration restarts from s
     int fresh;    // this iteration started from r0 = s (the start or a restart)
@@ -316,9 +350,16 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
   } sh;
   double *r = a.v0, *t = a.v7, *x = a.x;
   double *scur = a.v1, *snxt = a.v2, *pold = a.v3, *pnew = a.v4, *vold = a.v5, *vnew = a.v6;
+  __shared__ ExactState xs;
+  __shared__ SumWindow<2> w1, w2;
+  __shared__ SumWindow<3> w3;
+  exact_init(xs);
+  if (threadIdx.x == 0) w1.top[0] = w2.top[0] = w3.top[0] = kNoWindow;
+  __syncthreads();
   const double *minv = a.minv, *b = a.b;
   const bool rule0 = a.stop_rule == 0;
-  unsigned int ep = 0;
+  Episode ep;
+  const NoScalars none;
 
   // r = b - A x ; p = s = r ; d = r.(r/m)   (x = 0 when init)
   double acc[2] = {0.0, 0.0}, acc3[3];
@@ -332,15 +373,19 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
     }
     const double ri = b[row] - ax;
     r[row] = ri;
-    pnew[row] = ri;
     scur[row] = ri;
+    pold[row] = 0.0;  // the first p = s + 0 (0 - 0 v): no case of its own
+    vold[row] = 0.0;
     acc[0] = fma(ri, ri * minv[row], acc[0]);
     acc[1] = fma(b[row], b[row], acc[1]);
   }
-  if (!grid_allreduce_d<2>(gs, ep, acc, buf, [&](const double *q) {
+  if (!sum_rows<kX, 2, true>(gs, ep, xs, w1, acc, buf, none, none, [&](const double *q) {
         sh.d = q[0];
-        sh.conv = rule0 ? a.tol * sqrt(fabs(q[0])) : a.tol * sqrt(q[1]);
-        sh.crit = 0.0;
+        sh.dv.set(q[0]);
+        sh.conv = a.tol * root(rule0 ? fabs(q[0]) : q[1]);
+        sh.bound = sqrt_bound(sh.conv);
+        sh.crit2 = 0.0;
+        w1.top[0] = kNoWindow;
         sh.stop = 0;
         sh.restart = 0;
         sh.fresh = 1;
@@ -357,24 +402,13 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
       double *zp = a.v8;
       FOR_ROWS(P) {
         if (restart) r[row] = scur[row];
-        const double pi =
-            (j == 1) ? pnew[row] : fma(beta, fma(-w, vold[row], pold[row]), scur[row]);
+        const double pi = fma(beta, fma(-w, vold[row], pold[row]), scur[row]);
         pnew[row] = pi;
         zp[row] = pi * minv[row];
       }
       if (!grid_barrier(gs, ep)) return;
       FOR_ROWS(P) {
         const double vi = row_fma<kT>(a.A, s_, P.lane, row, [&](int k) { return zp[k]; });
-        vnew[row] = vi;
-        const double ri = r[row];
-        acc[0] = fma(scur[row], ri, acc[0]);
-        acc[1] = fma(vi, ri, acc[1]);
-      }
-    } else if (j == 1) {
-      FOR_ROWS(P) {
-        const double *pc = pnew;
-        const double vi =
-            row_fma<kT>(a.A, s_, P.lane, row, [&](int k) { return pc[k] * minv[k]; });
         vnew[row] = vi;
         const double ri = r[row];
         acc[0] = fma(scur[row], ri, acc[0]);
@@ -398,11 +432,12 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
     }
     // r.v = 0 (the reference's alpha = r.s/0) or r.s = 0 (alpha = 0, no
     // progress): alpha = 0, the iteration takes only its w step, and the
-    // next one restarts
-    if (!grid_allreduce_d<2>(gs, ep, acc, buf, [&](const double *q) {
+    // next one restarts.  Phase 2 gathers v unless z' is stored (whose
+    // barrier then publishes what it gathers)
+    if (!sum_rows<kX, 2, !kStoreZ>(gs, ep, xs, w1, acc, buf, none, none, [&](const double *q) {
           sh.rr0 = q[0];
           sh.brk = (q[0] == 0.0 || q[1] == 0.0) ? 1 : 0;
-          sh.alpha = sh.brk ? 0.0 : q[0] / q[1];
+          sh.alpha = sh.brk ? 0.0 : divide(q[0], q[1]);
         }))
       return;
     alpha = sh.alpha;
@@ -437,8 +472,10 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
     }
     // t = 0 exactly: s' = 0, the alpha step solved the system (the
     // reference's 0/0 there gives NaN); w = 0 keeps x and s' as they are
-    if (!grid_allreduce_d<2>(gs, ep, acc, buf,
-                             [&](const double *q) { sh.w = (q[1] != 0.0) ? q[0] / q[1] : 0.0; }))
+    // (phase 3 touches own rows only: nothing to publish)
+    if (!sum_rows<kX, 2, false>(
+            gs, ep, xs, w2, acc, buf, [&] { sh.rv.set(sh.rr0); }, none,
+            [&](const double *q) { sh.w = (q[1] != 0.0) ? divide(q[0], q[1]) : 0.0; }))
       return;
     w = sh.w;
     // phase 3: x += alpha z ; x += w z' ; s'' = s' - w t ; s''.z' ; r.s'' ; s''.s''
@@ -457,11 +494,14 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
       acc3[1] = fma(r[row], si, acc3[1]);
       acc3[2] = fma(si, si, acc3[2]);
     }
-    if (!grid_allreduce_d<3>(gs, ep, acc3, buf, [&](const double *q) {
-          const double b0 = q[0] / sh.d;
-          sh.crit = rule0 ? sqrt(fabs(b0)) : sqrt(q[2]);
-          sh.stop = (!(sh.crit == sh.crit) || !(sh.w == sh.w)) ? 2 : (sh.crit < sh.conv ? 1 : 0);
-          sh.beta = (q[1] / sh.rr0) * (sh.alpha / sh.w);
+    auto before3 = [&] { sh.aw = divide(sh.alpha, sh.w); };
+    if (!sum_rows<kX, 3, !kStoreZ>(gs, ep, xs, w3, acc3, buf, none, before3, [&](const double *q) {
+          const double crit2 = rule0 ? fabs(quotient(q[0], sh.dv)) : q[2];
+          sh.crit2 = crit2;
+          sh.stop = (is_nan_bits(crit2) || is_nan_bits(sh.w))   ? 2
+                    : sqrt_below(crit2, sh.conv, sh.bound) ? 1
+                                                           : 0;
+          sh.beta = quotient(q[1], sh.rv) * sh.aw;
           // breakdown guard (where the reference's recurrence divides by
           // zero and goes on with Inf/NaN): w = 0, r.s'' = 0 or a beta that
           // is not finite restart the iteration from the current residual
@@ -469,7 +509,7 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
           // itself started from its residual ends the solve (FVC_ERR_BREAKDOWN).
           // Iterations without a breakdown are unchanged.
           const bool broke = sh.stop == 0 &&
-                             (sh.brk || sh.w == 0.0 || q[1] == 0.0 || !isfinite(sh.beta));
+                             (sh.brk || sh.w == 0.0 || q[1] == 0.0 || not_finite_bits(sh.beta));
           sh.restart = 0;
           if (broke && sh.fresh) {
             sh.stop = 3;
@@ -501,8 +541,13 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
     j = a.maxit;
     status = FVC_ERR_NOCONV;
   }
-  finish_to(result, iresult, lead, j, status, sh.conv, sh.crit, 0);
-  epilogue_to<kT>(a, P, gs, result, lead, ep, red, false);
+  finish_to(result, iresult, lead, j, status, sh.conv, root(sh.crit2), 0);
+  if (!grid_barrier(gs, ep)) return;  // x of every row before the epilogue's SpMV
+  if (threadIdx.x == 0) w3.top[0] = kNoWindow;
+  __syncthreads();
+  epilogue_to<kT>(a, P, result, lead, false, [&](const double(&v)[3], auto f) {
+    sum_rows<kX, 3, false>(gs, ep, xs, w3, v, buf, none, none, f);
+  });
 }
 
 __global__ void __launch_bounds__(1024, 1) bicgstab_f64(KArgs a) {
@@ -512,8 +557,8 @@ __global__ void __launch_bounds__(1024, 1) bicgstab_f64(KArgs a) {
 // A small system's BiCGSTAB on one thread-block cluster: the same body, its
 // reductions and barriers through the cluster (GridSync.cluster), its
 // vectors in global memory (L2-resident at these sizes)
-__global__ void __launch_bounds__(256) bicgstab_cl(KArgs a) {
-  bicgstab_run<256>(a, Part(a.A.nslices, a.A.n), a.gs, a.result, a.iresult, blockIdx.x == 0);
+__global__ void __launch_bounds__(256, 1) bicgstab_cl(KArgs a) {
+  bicgstab_run<256, false, false, false>(a, Part(a.A.nslices, a.A.n), a.gs, a.result, a.iresult, blockIdx.x == 0);
   cluster_close(a.gs);
 }
 
@@ -550,9 +595,9 @@ __global__ void __launch_bounds__(kMaxT, 1024 / kMaxT) krylov_batched(KArgs a, c
   ak.tol = d.tol;
   ak.init = d.init;
   if (d.code == 2)
-    bicgstab_run<kMaxT, false, true>(ak, P, d.gs, d.result, d.iresult, rank == 0);
+    bicgstab_run<kMaxT, false, true, false>(ak, P, d.gs, d.result, d.iresult, rank == 0);
   else
-    pcg_run<true, kMaxT>(ak, P, d.gs, d.result, d.iresult, rank == 0);
+    pcg_run<true, kMaxT, false>(ak, P, d.gs, d.result, d.iresult, rank == 0);
   cluster_close(d.gs);
 }
 
@@ -574,7 +619,7 @@ __global__ void __launch_bounds__(1024, 1) gmres_f64(KArgs a) {
   const double *minv = a.minv, *b = a.b;
   auto G = [&](int i) { return a.g + (size_t)(i - 1) * n; };  // 1-based column
   auto H = [&](int i, int jj) -> double & { return h[(i - 1) + (jj - 1) * (k + 1)]; };
-  unsigned int ep = 0;
+  Episode ep;
   double acc[1];
 
   // x = 0 ; econv = tol*||b||
@@ -583,7 +628,7 @@ __global__ void __launch_bounds__(1024, 1) gmres_f64(KArgs a) {
     x[row] = 0.0;
     acc[0] = fma(b[row], b[row], acc[0]);
   }
-  if (!reduce<1>(a, ep, acc, red)) return;
+  if (!grid_allreduce<1>(a.gs, ep, acc, red)) return;
   const double econv = a.tol * sqrt(acc[0]);
   int l, nit = 0, ni = 0, status = FVC_OK;
   double crit = 0.0;
@@ -597,7 +642,7 @@ __global__ void __launch_bounds__(1024, 1) gmres_f64(KArgs a) {
       g1[row] = gi;
       acc[0] = fma(gi, gi, acc[0]);
     }
-    if (!reduce<1>(a, ep, acc, red)) return;
+    if (!grid_allreduce<1>(a.gs, ep, acc, red)) return;
     if (threadIdx.x == 0) e[0] = sqrt(acc[0]);
     __syncthreads();
     const double e1inv = 1.0 / e[0];
@@ -617,7 +662,7 @@ __global__ void __launch_bounds__(1024, 1) gmres_f64(KArgs a) {
         gn[row] = vi;
         acc[0] = fma(vi, g1c[row], acc[0]);
       }
-      if (!reduce<1>(a, ep, acc, red)) return;
+      if (!grid_allreduce<1>(a.gs, ep, acc, red)) return;
       double beta = acc[0];
       if (threadIdx.x == 0) H(1, i) = beta;
       // modified Gram-Schmidt: subtract, then dot with the next vector
@@ -630,7 +675,7 @@ __global__ void __launch_bounds__(1024, 1) gmres_f64(KArgs a) {
           gn[row] = vi;
           acc[0] = fma(vi, (jj < i) ? gnext[row] : vi, acc[0]);
         }
-        if (!reduce<1>(a, ep, acc, red)) return;
+        if (!grid_allreduce<1>(a.gs, ep, acc, red)) return;
         beta = acc[0];
         if (jj < i && threadIdx.x == 0) H(jj + 1, i) = beta;
       }
@@ -685,7 +730,9 @@ __global__ void __launch_bounds__(1024, 1) gmres_f64(KArgs a) {
     if (status == FVC_OK) status = FVC_ERR_NOCONV;
   }
   finish(a, l, status, econv, crit, nit);
-  epilogue(a, ep, red, true);
+  epilogue_to(a, P, a.result, blockIdx.x == 0, true, [&](double(&v)[3], auto f) {
+    if (grid_allreduce<3>(a.gs, ep, v, red) && threadIdx.x == 0) f(v);
+  });
 }
 
 // ---------------------------------------------------------------------
@@ -808,7 +855,7 @@ Launch persistent_launch(K kernel, const DeviceMatrix &A, const fvc_opts &o) {
   if (o.blocks_per_sm > 0 && o.blocks_per_sm < occ) occ = o.blocks_per_sm;
   const int warps = L.threads / 32;
   const int need = (A.nslices + warps - 1) / warps;
-  L.blocks = std::max(1, std::min(occ * sm_count(), need));
+  L.blocks = std::max(1, std::min({occ * sm_count(), need, kXBlocks}));
   if (o.max_blocks > 0) L.blocks = std::min(L.blocks, o.max_blocks);
   return L;
 }
@@ -844,7 +891,7 @@ int32_t enqueue_persistent(K kernel, const DeviceMatrix &A, Scratch &S, const do
   Launch L = persistent_launch(kernel, A, o);
   int32_t rc = ensure_vectors(S, (size_t)A.n, nvec, (size_t)L.blocks, gmres);
   if (rc != FVC_OK || !launch) return rc;
-  reset_sync(S, stream);
+  reset_sync(S, stream, (size_t)L.blocks);
   KArgs a{};
   a.A = view64(A);
   a.A.chk = check_word(S);
@@ -1037,10 +1084,7 @@ int32_t enqueue_bicgstab_cluster(const DeviceMatrix &A, Scratch &S, const double
   }
   int32_t rc = ensure_vectors(S, (size_t)A.n, 8, 1, false);
   if (rc != FVC_OK || !launch) return rc;
-  // the error block (wait and check words) and the result slots start at zero
-  cudaMemsetAsync(S.err, 0, 64, stream);
-  cudaMemsetAsync(S.iresult, 0, 16 * sizeof(int), stream);
-  cudaMemsetAsync(S.result, 0, 16 * sizeof(double), stream);
+  reset_sync(S, stream, 0);
   KArgs a{};
   a.A = view64(A);
   a.A.chk = check_word(S);
@@ -1057,6 +1101,7 @@ int32_t enqueue_bicgstab_cluster(const DeviceMatrix &A, Scratch &S, const double
   a.v6 = S.v[6];
   a.v7 = S.v[7];
   a.gs = make_sync(S, 1);
+  a.gs.xw = nullptr;
   a.gs.nblocks = (unsigned int)csize;
   a.gs.cluster = csize > 1 ? 1 : 0;
   a.tol = tol;
@@ -1374,25 +1419,24 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
     --nb[k];
     --total;
   }
-  // one device buffer: per system a 64-byte counter sector, partials and
-  // totals, results; then the error word, descriptors and block map
-  size_t part_doubles = 0;
-  for (int s = 0; s < nsys; ++s) part_doubles += (size_t)4 * kMaxNV * (nb[s] + 1);
-  const size_t ctr_bytes = (size_t)nsys * 64 + 64;
+  // one device buffer: per system a 64-byte counter sector, the error word,
+  // the reduction slots (groups: clusters have none); then results,
+  // descriptors and the block map.  ctr_bytes: what every launch zeroes of it
+  const size_t part_off = (size_t)nsys * 64 + 64;
+  const size_t ctr_bytes = part_off + (csize > 0 ? 0 : slot_bytes((size_t)total));
   const size_t res_bytes = (size_t)nsys * 16 * sizeof(double);
   const size_t ires_bytes = (size_t)nsys * 16 * sizeof(int);
   const size_t sys_bytes = (size_t)nsys * sizeof(BatchSys);
   const size_t sob_bytes = (size_t)total * sizeof(int);
-  const size_t bytes =
-      ctr_bytes + part_doubles * sizeof(double) + res_bytes + ires_bytes + sys_bytes + sob_bytes;
+  const size_t bytes = ctr_bytes + res_bytes + ires_bytes + sys_bytes + sob_bytes;
   char *buf = nullptr;
   if (persistent ? cudaMalloc((void **)&buf, bytes) != cudaSuccess
                  : cudaMallocAsync((void **)&buf, bytes, stream) != cudaSuccess)
     return FVC_ERR_CUDA;
   unsigned int *ctr = reinterpret_cast<unsigned int *>(buf);
   int *err = reinterpret_cast<int *>(buf + (size_t)nsys * 64);
-  double *part = reinterpret_cast<double *>(buf + ctr_bytes);
-  double *res = part + part_doubles;
+  RedSlot *part = reinterpret_cast<RedSlot *>(buf + part_off);
+  double *res = reinterpret_cast<double *>(buf + ctr_bytes);
   int *ires = reinterpret_cast<int *>(res + (size_t)nsys * 16);
   BatchSys *dsys = reinterpret_cast<BatchSys *>(reinterpret_cast<char *>(ires) + ires_bytes);
   int *dsob = reinterpret_cast<int *>(reinterpret_cast<char *>(dsys) + sys_bytes);
@@ -1413,10 +1457,9 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
     // defect-correction sweep (BiCGSTAB), as in a single solve
     d.inner_tol = (o.inner_tol > 0) ? o.inner_tol : kInnerTolDefault;
     d.gs.count = ctr + (size_t)s * 16;
-    d.gs.flag = ctr + (size_t)s * 16 + 8;
     d.gs.err = err;
-    d.gs.partials = part + poff;
-    d.gs.totals = part + poff + (size_t)4 * kMaxNV * nb[s];
+    d.gs.slots = csize > 0 ? nullptr : part + poff;
+    d.gs.xw = nullptr;
     d.gs.nblocks = (unsigned int)nb[s];
     // a cluster launch numbers its blocks from 0: the base within the segment
     d.gs.base = (unsigned int)(csize > 0 ? b0 - seg_off[seg] : b0);
@@ -1425,7 +1468,7 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
     d.result = res + (size_t)s * 16;
     d.iresult = ires + (size_t)s * 16;
     d.run = run ? run + s : nullptr;
-    poff += (size_t)4 * kMaxNV * (nb[s] + 1);
+    poff += (size_t)4 * kMaxNV * nb[s];
     for (int k = 0; k < nb[s]; ++k) hsob[(size_t)b0 + k] = s;
     b0 += nb[s];
   }

@@ -38,6 +38,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <type_traits>
 
 #include "fvc_device.cuh"
 #include "fvc_internal.h"
@@ -78,17 +79,18 @@ __device__ __forceinline__ void ff_add(float &s, float &c, float s2, float c2) {
 // not FP64: GB300 runs FP64 at ~2 lanes per clock per SM, and a block of
 // 1024 threads each doing FP64 shuffles and divisions costs microseconds
 // per reduction); warp 0 combines the warps, converts the block's pair to
-// FP64 once, publishes it and arrives on the grid counter (release), waits
-// for every block's arrival (acquire) and sums all partials in block order
-// itself, so every block holds identical totals after two trips to L2.
-// Lane 0 of warp 0 then calls f(totals) -- the place for the iteration's scalar FP64
-// work, which it publishes through shared memory -- and one __syncthreads
-// hands the results to the block.  Returns false when a wait exceeded its
-// bound (gs.err set).
-template <int NV, typename F>
-__device__ __forceinline__ bool grid_allreduce_ff(const GridSync &gs, unsigned int &episode,
-                                                  const CSum (&v)[NV], float2 *red2, F &&f) {
-  __shared__ int s_ok;
+// FP64 once and exchanges it with the other blocks (exchange_totals; kPublish
+// at grid_arrive), so every block holds identical totals.  Lane 0 of warp 0
+// then calls f(totals) -- the place for the iteration's scalar FP64 work,
+// which it publishes through shared memory -- and one __syncthreads hands the
+// results to the block; side() and mid() as in grid_sum_d.  Returns false
+// when a wait exceeded its bound (gs.err set).
+constexpr int kTotCap = 160;  // blocks whose partials one step sums (the device has 152 SMs)
+
+template <int NV, bool kPublish, typename S, typename M, typename F>
+__device__ __forceinline__ bool grid_allreduce_ff(const GridSync &gs, Episode &episode,
+                                                  const CSum (&v)[NV], float2 *red2, double *tot,
+                                                  S &&side, M &&mid, F &&f) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
 #pragma unroll
@@ -102,35 +104,9 @@ __device__ __forceinline__ bool grid_allreduce_ff(const GridSync &gs, unsigned i
     }
     if (lane == 0) red2[q * 32 + warp] = make_float2(s, c);
   }
-  if (threadIdx.x == 0) s_ok = 1;
   __syncthreads();
-  const unsigned int ep = ++episode;
-  if (gs.cluster) {  // one thread-block cluster: cluster_exchange
-    __shared__ double s_slot[2][kMaxNV];
-    if (warp == 0) {
-#pragma unroll
-      for (int q = 0; q < NV; ++q) {
-        const float2 w = (lane < nwarps) ? red2[q * 32 + lane] : make_float2(0.0f, 0.0f);
-        float s = w.x, c = w.y;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const float s2 = __shfl_xor_sync(0xffffffffu, s, o);
-          const float c2 = __shfl_xor_sync(0xffffffffu, c, o);
-          ff_add(s, c, s2, c2);
-        }
-        if (lane == 0) s_slot[ep & 1u][q] = (double)s + (double)c;
-      }
-    }
-    double t[NV];
-    cluster_exchange<NV>(s_slot, ep, t);
-    if (threadIdx.x == 0) f(t);
-    __syncthreads();
-    return true;
-  }
+  double bsum[NV];
   if (warp == 0) {
-    const unsigned int nb = gs.nblocks;
-    double *part = gs.partials + (size_t)(ep & 3u) * kMaxNV * nb;
-    double bsum[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
       const float2 w = (lane < nwarps) ? red2[q * 32 + lane] : make_float2(0.0f, 0.0f);
@@ -143,55 +119,29 @@ __device__ __forceinline__ bool grid_allreduce_ff(const GridSync &gs, unsigned i
       }
       bsum[q] = (double)s + (double)c;
     }
-    bool ok = true;
-    double t[NV];
-    if (nb == 1) {  // one block: its sum is the total (same value)
-#pragma unroll
-      for (int q = 0; q < NV; ++q) t[q] = bsum[q];
-    } else {
-      // publish the block's partials, then wait until every block has
-      if (lane == 0) {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) part[(size_t)q * nb + (blockIdx.x - gs.base)] = bsum[q];
-        red_add_release(gs.count, 1u);
-        const unsigned int target = ep * nb;
-        const uint64_t t0 = global_ns();
-        unsigned int spins = 0;
-        while (ld_acquire(gs.count) < target) {
-          if (*(volatile int *)gs.err != 0) {
-            ok = false;
-            break;
-          }
-          if ((++spins & 255u) == 0 && global_ns() - t0 > kBarrierTimeoutNs) {
-            atomicExch(gs.err, 7 /* FVC_ERR_TIMEOUT */);
-            ok = false;
-            break;
-          }
-          __nanosleep(20);
-        }
-      }
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      // every block sums the partials itself, in block order (identical
-      // totals everywhere; no second round trip through a release flag)
-#pragma unroll
-      for (int q = 0; q < NV; ++q) {
-        double u = 0.0;
-        if (ok) {
-          const double *pp = part + (size_t)q * nb;
-          for (unsigned int b = lane; b < nb; b += 32) u = __dadd_rn(u, __ldcg(pp + b));
-        }
-        t[q] = warp_sum(u);
-      }
-    }
-    if (lane == 0) {
-      if (ok)
-        f(t);
-      else
-        s_ok = 0;
-    }
   }
-  __syncthreads();
-  return s_ok != 0;
+  return exchange_totals<NV, kPublish>(gs, episode, bsum, tot, kTotCap, side, mid, f);
+}
+
+// The exact sum (exact_sum) of compensated FP32 partials; kX false: the sums of
+// grid_allreduce_ff.
+template <int NV, bool kPublish, bool kX, typename S, typename M, typename F>
+__device__ __forceinline__ bool grid_sum_ffx(const GridSync &gs, Episode &episode, ExactState &xs,
+                                             SumWindow<NV> &win, const CSum (&v)[NV],
+                                             float2 *red2, double *tot, S &&side, M &&mid,
+                                             F &&f) {
+  static_assert(NV * kLimbs * 32 * sizeof(int) <= 2 * kTotCap * sizeof(double), "limb sums");
+  constexpr bool kMid = !std::is_same<std::decay_t<M>, NoScalars>::value;
+  if (!kX) return grid_allreduce_ff<NV, kPublish>(gs, episode, v, red2, tot, side, mid, f);
+  auto put = [&](int q, int top, int *part) { return put_limbs(v[q].s, v[q].c, top, part); };
+  auto expo = [&](int q) {  // as an FP64 exponent
+    const int ex = (int)(__float_as_uint(__fadd_rn(v[q].s, v[q].c)) >> 23) & 0xff;
+    return ex == 0xff ? 0x7ff : (ex ? ex : 1) - 127 + 1023;
+  };
+  int *part = reinterpret_cast<int *>(tot);
+  if (kMid)
+    return exact_sum<NV, kPublish, true>(gs, episode, xs, win, part, put, expo, mid, f);
+  return exact_sum<NV, kPublish, false>(gs, episode, xs, win, part, put, expo, side, f);
 }
 
 // (hi, lo) += alpha * p with alpha given as an FP32 pair (ah, al): the
@@ -393,6 +343,7 @@ __device__ __forceinline__ float arow32(const MArgs &a, int s, int lane, int row
       if (k < w) t = fmaf(v[k], yi - yf(c[k]), t);
     return t;
   }
+#pragma unroll 1
   for (int k = 0; k < w; ++k) {
     int c = ld_stream(cp + 32 * k);
     FVC_CHK((unsigned)c < (unsigned)a.A.n, a.A.chk, kChkColumn, c = row);
@@ -421,6 +372,7 @@ struct MPart {
 };
 
 #define MFOR_ROWS(P)                                               \
+  _Pragma("unroll 1")                                              \
   for (int s_ = (P).sb + (P).warp; s_ < (P).se; s_ += (P).nwarps) \
     for (int row = s_ * 32 + (P).lane, once_ = 1; once_ && row < (P).n; once_ = 0)
 
@@ -436,6 +388,7 @@ struct MPart {
 // are visited in the order of MFOR_ROWS, so sums over them are the same.
 template <typename F>
 __device__ __forceinline__ void mfor_rows2(const MPart &P, F &&f) {
+#pragma unroll 1
   for (int s = P.sb + P.warp; s < P.se; s += 2 * P.nwarps) {
     const int ra = s * 32 + P.lane;
     if (ra >= P.n) break;  // later slices of this warp are further on
@@ -452,7 +405,7 @@ __device__ __forceinline__ void mfor_rows2(const MPart &P, F &&f) {
 // FP64 residual sweep: rs = b - A x rounded to FP32.  Returns ||b-Ax||^2,
 // ||b||^2, rs.(rs/m) and ||b-Ax||^2 over the rows the FP32 iteration moves
 // (FP64 sums).
-__device__ __forceinline__ bool residual_sweep(const MArgs &a, unsigned int &ep, bool zero_x,
+__device__ __forceinline__ bool residual_sweep(const MArgs &a, Episode &ep, bool zero_x,
                                                double (&out)[4], double *red) {
   const MPart P(a);
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
@@ -896,6 +849,7 @@ __device__ __forceinline__ CSum cg_phase_a_st(const MArgs &a, const MPart &P, fl
     }
   }
   __syncthreads();
+#pragma unroll 1
   for (int i = 0; i < nch; ++i) {
     if (P.warp == 0) {
       const int jl = i + kWinHalo + 1 + kLandAhead;
@@ -1000,6 +954,7 @@ __device__ __forceinline__ CSum cg_phase_a_st(const MArgs &a, const MPart &P, fl
 #pragma unroll
           for (int k = 0; k < 4; ++k) t = fmaf(w[k], pi - nb[k], t);
         } else {
+#pragma unroll 1
           for (int k = 0; k < wd; ++k) t = fmaf(ws[32 * k], pi - pat(row + (int)cs[32 * k]), t);
         }
         a.q[row] = t;
@@ -1082,6 +1037,7 @@ __device__ __forceinline__ void cg_phase_b_st(const MArgs &a, const MPart &P, fl
   StHdr *H = reinterpret_cast<StHdr *>(smem);
   const int nch = st_chunks(P);
   if (!pre) prefetch_b<kPair, kUpdE>(a, P, d, smem, cnt);
+#pragma unroll 1
   for (int i = 0; i < nch; ++i) {
     if (P.warp == 0 && P.lane == 0 && i + kBStages - 1 < nch)
       issue_b<kPair, kUpdE>(a, P, smem, cnt.sb + i + kBStages - 1, i + kBStages - 1, d);
@@ -1151,13 +1107,16 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
   // every thread after the all-reduce's closing __syncthreads
   __shared__ struct {
     double rz, rr_upd, relres, pend_alpha, alpha, rz_new;
-    double bnorm2, scale, delta2, target2, res0;
+    double bnorm2, scale, delta2, target2, res0, thr, rr;
+    Divisor rzv;  // rz, its reciprocal taken while the p.q sum travels
     float alpha_f, alpha_lo, a1, a1_lo, beta, beta_lo;
     int action, status, updates;
   } sh;
   __shared__ float2 red2[kMaxNV * 32];
+  __shared__ double tot[2 * kTotCap];
   enum { kContinue = 0, kUpdate = 1, kStop = 2 };
-  unsigned int ep = 0;
+  const NoScalars none;
+  Episode ep;
   int it = 0;
   double res[4];
   if (!residual_sweep(a, ep, a.init != 0, res, red)) return;
@@ -1171,6 +1130,8 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
     sh.relres = sqrt(res[0] / scale);
     sh.rz = res[2];
     sh.rr_upd = res[3];  // ||r||^2 (moving rows) at the last reliable update
+    sh.thr = sh.delta2 * sh.rr_upd;
+    sh.rr = 0.0;
     sh.pend_alpha = 0.0;
     sh.beta = 0.0f;
     sh.beta_lo = 0.0f;
@@ -1206,13 +1167,20 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
       else
         prefetch_b<true, false>(a, P, d, st_smem, gch);
     }
-    if (!grid_allreduce_ff<1>(a.gs, ep, pq, red2, [&](const double *t) {
-          const double alpha_d = sh.rz / t[0];
+    // phase B touches own rows only: nothing to publish.  Meanwhile: 1/rz,
+    // the deferred alpha as a pair, the last iteration's history entry
+    auto before_pq = [&] {
+      sh.rzv.set(sh.rz);
+      sh.a1 = (float)sh.pend_alpha;
+      sh.a1_lo = (float)(sh.pend_alpha - (double)sh.a1);
+      if (mlead(a) && a.history && it > 1 && it - 1 <= kHistoryMax)
+        a.history[it - 2] = (float)root(divide(sh.rr, sh.scale));
+    };
+    if (!grid_allreduce_ff<1, false>(a.gs, ep, pq, red2, tot, before_pq, none, [&](const double *t) {
+          const double alpha_d = divide(sh.rz, t[0]);
           sh.alpha = alpha_d;
           sh.alpha_f = (float)alpha_d;
           sh.alpha_lo = (float)(alpha_d - (double)sh.alpha_f);
-          sh.a1 = (float)sh.pend_alpha;
-          sh.a1_lo = (float)(sh.pend_alpha - (double)sh.a1);
         })) {
       if (kStaged) drain_prefetch_b(P, st_smem, gch);
       return;
@@ -1240,20 +1208,19 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
       prefetch_a<kW>(a, P, st_smem, gch);
       a_pre = true;
     }
-    if (!grid_allreduce_ff<2>(a.gs, ep, acc, red2, [&](const double *t) {
+    if (!grid_allreduce_ff<2, true>(a.gs, ep, acc, red2, tot, none, none, [&](const double *t) {
           // the alpha*p of an iteration that did not update e is added later
           if (!was_pending) sh.pend_alpha = sh.alpha;
           const double rz_new = t[0];
           sh.rz_new = rz_new;
-          if (mlead(a) && a.history && it <= kHistoryMax)
-            a.history[it - 1] = (float)sqrt(t[1] / sh.scale);
-          if (!(rz_new == rz_new)) {
+          sh.rr = t[1];
+          if (is_nan_bits(rz_new)) {
             sh.status = FVC_ERR_NAN;
             sh.action = kStop;
-          } else if (t[1] <= sh.delta2 * sh.rr_upd || t[1] <= sh.target2 || it >= a.maxit) {
+          } else if (t[1] <= sh.thr || t[1] <= sh.target2 || it >= a.maxit) {
             sh.action = kUpdate;
           } else {
-            const double beta = rz_new / sh.rz;
+            const double beta = quotient(rz_new, sh.rzv);
             sh.beta = (float)beta;
             sh.beta_lo = (float)(beta - (double)sh.beta);
             sh.rz = rz_new;
@@ -1291,6 +1258,7 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
           sh.action = kStop;
         } else {
           sh.rr_upd = res[3];
+          sh.thr = sh.delta2 * sh.rr_upd;
           // beta from the replaced (true) residual, or with update_beta from
           // the recursive one; the next alpha uses the true r.z
           const double beta = (a.update_beta ? sh.rz_new : res[2]) / sh.rz;
@@ -1313,6 +1281,8 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
   }
   if (a_pre) drain_prefetch_a(P, st_smem, gch);
   if (mlead(a) && threadIdx.x == 0) {
+    if (a.history && it > 0 && it <= kHistoryMax)  // the last iteration's entry
+      a.history[it - 1] = (float)sqrt(sh.rr / sh.scale);
     a.iresult[0] = sh.updates;
     a.iresult[1] = (status == FVC_ERR_NOCONV) ? sh.status : status;
     a.iresult[2] = it;
@@ -1341,21 +1311,29 @@ __global__ void __launch_bounds__(1024, 1) mixed_cg_staged_w4(MArgs a) {
 constexpr int kBcgStall = 100;
 constexpr int kSweepStall = 3;
 
+template <bool kX>
 __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
   __shared__ double red[kMaxNV * 32];
   __shared__ float2 red2[kMaxNV * 32];
+  __shared__ double tot[2 * kTotCap];
   // the inner iteration's scalars: FP64 work of lane 0 of warp 0 inside the
   // all-reduces (GB300 runs FP64 at ~1/64 of the FP32 rate: three FP64
   // divisions in every thread of every iteration kept the FP64 pipe 40%
   // busy), handed to the block as FP32 through shared memory
   __shared__ struct {
-    double rr0, best;
+    double rr0, best, aw;
+    Divisor rv;  // rr0
     float alpha, omega, beta;
     int it_best, go;
   } bs;
+  __shared__ ExactState xs;
+  __shared__ SumWindow<2> w1, w2, w3;
   if (f32_refused(a)) return;
+  const NoScalars none;
+  exact_init(xs);
+  if (threadIdx.x == 0) w1.top[0] = w2.top[0] = w3.top[0] = kNoWindow;
   const MPart P(a);
-  unsigned int ep = 0;
+  Episode ep;
   int sweep = 0, inner_total = 0, status = FVC_ERR_NOCONV;
   double res[4];
   double relres = 0.0, bnorm2 = 0.0, best_rel = 0.0;
@@ -1425,9 +1403,9 @@ __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
       });
       // breakdown (v.r0 or r0.s vanished in FP32): leave the correction as it
       // is and restart from an FP64 residual in the next sweep
-      if (!grid_allreduce_ff<2>(a.gs, ep, c01, red2, [&](const double *q) {
+      if (!grid_sum_ffx<2, false, kX>(a.gs, ep, xs, w1, c01, red2, tot, none, none, [&](const double *q) {
             bs.rr0 = q[0];
-            bs.alpha = (float)(q[0] / q[1]);
+            bs.alpha = (float)divide(q[0], q[1]);
             bs.go = (isfinite(bs.alpha) && bs.alpha != 0.0f) ? 1 : 0;
           }))
         return;
@@ -1472,8 +1450,9 @@ __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
             c23[1].add(ti[u] * ti[u]);
           }
       });
-      if (!grid_allreduce_ff<2>(a.gs, ep, c23, red2, [&](const double *q) {
-            bs.omega = (q[1] > 0.0) ? (float)(q[0] / q[1]) : 0.0f;
+      if (!grid_sum_ffx<2, false, kX>(a.gs, ep, xs, w2, c23, red2, tot, [&] { bs.rv.set(bs.rr0); },
+                                  none, [&](const double *q) {
+            bs.omega = (q[1] > 0.0) ? (float)divide(q[0], q[1]) : 0.0f;
             bs.go = isfinite(bs.omega) ? 1 : 0;
           }))
         return;
@@ -1505,7 +1484,8 @@ __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
       // stop on the inner reduction, a NaN, maxit or w = 0; restarted
       // BiCGSTAB: an inner solve whose residual has not improved for
       // kBcgStall iterations (FP32 stagnation) restarts from an FP64 one
-      if (!grid_allreduce_ff<2>(a.gs, ep, c45, red2, [&](const double *q) {
+      auto before45 = [&] { bs.aw = divide((double)bs.alpha, (double)bs.omega); };
+      if (!grid_sum_ffx<2, false, kX>(a.gs, ep, xs, w3, c45, red2, tot, none, before45, [&](const double *q) {
             const double sz = fabs(q[0]);
             int go = 1;
             if (!(q[0] == q[0]) || sz <= stop2 || inner_total + it >= a.maxit ||
@@ -1517,7 +1497,7 @@ __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
             } else if (it - bs.it_best > kBcgStall) {
               go = 0;
             }
-            bs.beta = (float)((q[1] / bs.rr0) * ((double)bs.alpha / (double)bs.omega));
+            bs.beta = (float)(quotient(q[1], bs.rv) * bs.aw);
             bs.go = go;
           }))
         return;
@@ -1545,7 +1525,9 @@ __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
   }
 }
 
-__global__ void __launch_bounds__(1024, 1) mixed_bicgstab(MArgs a) { mixed_bicgstab_body(a); }
+__global__ void __launch_bounds__(1024, 1) mixed_bicgstab(MArgs a) {
+  mixed_bicgstab_body<true>(a);
+}
 
 // Batched mixed-precision solves: every block runs the mixed CG (code 1)
 // or the mixed BiCGSTAB (code 2) of its system of the block-diagonal
@@ -1572,7 +1554,7 @@ __global__ void __launch_bounds__(kMaxT, 1024 / kMaxT)
   am.history = nullptr;
   if (d.code == 2) {
     am.rsl = nullptr;
-    mixed_bicgstab_body(am);
+    mixed_bicgstab_body<false>(am);
   } else {
     mixed_cg_body<false, 0>(am);
   }
@@ -1773,11 +1755,12 @@ int32_t enqueue_mixed(const DeviceMatrix &A0, Scratch &S, int code, const double
   if (occ <= 0) occ = 1;
   if (o.blocks_per_sm > 0 && o.blocks_per_sm < occ) occ = o.blocks_per_sm;
   const int warps = threads / 32;
-  int blocks = std::max(1, std::min(occ * sm_count_m(), (A.nslices + warps - 1) / warps));
+  int blocks =
+      std::max(1, std::min({occ * sm_count_m(), (A.nslices + warps - 1) / warps, kXBlocks}));
   if (o.max_blocks > 0) blocks = std::min(blocks, o.max_blocks);
   if (ensure_sync(S, (size_t)blocks) != FVC_OK) return FVC_ERR_CUDA;
   if (!launch) return FVC_OK;
-  reset_sync(S, stream);
+  reset_sync(S, stream, (size_t)blocks);
   MArgs a = mixed_args(A, S, b, x);
   a.rsl = (code == 1) ? S.f[9] : nullptr;
   a.gs = make_sync(S, blocks);

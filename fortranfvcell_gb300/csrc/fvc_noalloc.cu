@@ -33,14 +33,14 @@ constexpr int kNoAllocThreads = 1024;
 
 // Layout of the scratch array (doubles):
 //   [0, 5*R)                 r, z, p (two buffers), q
-//   [5R, 5R + 4*kMaxNV*B)    reduction partials
-//   then 4*kMaxNV totals, 16 results, then 16 words of counters
+//   [5R, 5R + 8*kMaxNV*B)    reduction slots (two doubles each)
+//   then 16 results, then 16 doubles of counters
 constexpr size_t kVecDoubles = 5 * (size_t)kNoAllocMaxRows;
-constexpr size_t kPartDoubles = 4 * (size_t)kMaxNV * kNoAllocMaxBlocks;
-constexpr size_t kTotDoubles = 4 * (size_t)kMaxNV;
+constexpr size_t kPartDoubles =
+    4 * (size_t)kMaxNV * kNoAllocMaxBlocks * (sizeof(RedSlot) / sizeof(double));
 constexpr size_t kResDoubles = 16;
-constexpr size_t kCtrDoubles = 16;  // count, flag, err, iresult (as 32-bit words)
-constexpr size_t kScratchDoubles = kVecDoubles + kPartDoubles + kTotDoubles + kResDoubles + kCtrDoubles;
+constexpr size_t kCtrDoubles = 16;  // count, err, iresult (as 32-bit words)
+constexpr size_t kScratchDoubles = kVecDoubles + kPartDoubles + kResDoubles + kCtrDoubles;
 
 // A device holds this array (~5.0 MiB) from the first call on it (the load
 // of this module on that device) until the process exits.
@@ -89,7 +89,7 @@ constexpr int kBadStructure = -1;
 __global__ void __launch_bounds__(kNoAllocThreads, 1) pcg_csrd_noalloc_kernel(NoAllocArgs a) {
   __shared__ double red[kMaxNV * 32];
   const int n = a.n;
-  unsigned int ep = 0;
+  Episode ep;
   // Structure check before any gather: ia(1) = 1, each row's length in
   // [0, n-1], every column in [1, n]; and at least one entry above the
   // diagonal when there are off-diagonals at all.  Symmetric CSRD keeps
@@ -274,13 +274,10 @@ extern "C" int32_t fvc_pcg_csrd_noalloc(const double *d_ad, const double *d_au,
   a.pb = base + 3 * R;
   a.q = base + 4 * R;
   double *part = base + kVecDoubles;
-  double *tot = part + kPartDoubles;
-  double *res = tot + kTotDoubles;
+  double *res = part + kPartDoubles;
   unsigned int *ctr = reinterpret_cast<unsigned int *>(res + kResDoubles);
-  a.gs.partials = part;
-  a.gs.totals = tot;
+  a.gs.slots = reinterpret_cast<RedSlot *>(part);
   a.gs.count = ctr;
-  a.gs.flag = ctr + 8;
   a.gs.err = reinterpret_cast<int *>(ctr + 16);
   a.gs.nblocks = (unsigned int)blocks;
   a.iresult = reinterpret_cast<int *>(ctr + 20);
@@ -289,8 +286,9 @@ extern "C" int32_t fvc_pcg_csrd_noalloc(const double *d_ad, const double *d_au,
   a.maxit = maxit;
   a.init = init ? 1 : 0;
   a.stop_rule = stop_rule;
-  // The array keeps the previous call's contents: counters, flags, error
-  // word and results must start at zero (vectors are written before use).
+  // The array keeps the previous call's contents: the counter, the
+  // error word and the results must start at zero (vectors and slots are
+  // written before use).
   if (cudaMemsetAsync(ctr, 0, kCtrDoubles * sizeof(double), s) != cudaSuccess ||
       cudaMemsetAsync(res, 0, kResDoubles * sizeof(double), s) != cudaSuccess)
     return FVC_ERR_CUDA;
