@@ -1,19 +1,22 @@
 // fvc_cluster.cu -- Jacobi-PCG (src/Iterativos.f:29-106) of a small system
-// on one thread-block cluster, resident in distributed shared memory.
+// on one thread-block cluster, resident in its registers and shared memory.
 //
 // A system of a few thousand rows (the SIMPLE p' system of a 64 x 64 cavity
 // has 4096) leaves a grid-wide persistent kernel latency-bound: every
-// iteration waits twice for all blocks through L2 atomics and reads its
-// vectors from L2.  Here the rows are split over the CTAs of one cluster
-// (up to 16 SMs).  Each CTA copies its rows' SELL slices, diagonal and
-// Jacobi weights into shared memory once and keeps x, r, z, p and q there;
-// the SpMV reads a neighbour row's p from the owning CTA's shared memory
-// over DSMEM, and each reduction is one cluster barrier: every CTA posts its
-// partial in its own shared memory, and after the barrier every CTA sums
-// all partials in rank order itself (identical totals in every CTA, so
-// every CTA takes the same branch).  Per iteration: form p, barrier, SpMV +
-// p.q, reduction, update + r.z, reduction -- three cluster barriers and no
-// global-memory traffic.
+// iteration waits twice for all blocks through L2.  Here the rows are split
+// over the CTAs of one cluster (up to 16 SMs), one row per thread: its matrix
+// row, x, r, p, q and 1/m stay in registers, p also in shared memory, where the
+// SpMV of the other CTAs reads it (DSMEM).  Sums are exact integer sums
+// (fvc_device.cuh), the CTAs' limbs exchanged by one cluster barrier: every
+// CTA posts its limbs in its own shared memory, and after the barrier every
+// CTA adds all of them itself (identical totals in every CTA, so every CTA
+// takes the same branch).  Per iteration: form p, barrier, SpMV + p.q, sum,
+// update + r.z, sum -- three cluster barriers and no global-memory traffic;
+// x += alpha p runs between the arrival and the wait of the last one.
+//
+// What bounds it: chains of dependent FP64 instructions (64 clocks each; two
+// warps of an SM sub-partition share a pipe that takes one per 76 clocks) and
+// the barriers (420 clocks, and 230 for the DSMEM read after each).
 //
 // There is no spin-wait: the only waits are hardware cluster barriers, which
 // every CTA reaches the same number of times (the loop exit depends only on
@@ -35,14 +38,8 @@ namespace fvc {
 namespace {
 
 constexpr int kClMax = 16;        // CTAs per cluster (non-portable above 8)
-constexpr int kClMaxRows = 2048;  // rows per CTA
-// Largest system run on a cluster: measured per PCG iteration on GB300 (16
-// CTAs, 256 rows each) against the grid-wide kernel: 4096 rows 6.65 vs
-// 8.41 us, 6124 rows 7.59 vs 8.41 us, 10000 rows 9.59 vs 8.95 us.  Forming
-// p at every read instead of the p barrier was slower at every size.  The
-// FP64 rate of the cluster's SMs bounds it: 512 or 1024 rows per CTA
-// instead of 256 (8 or 4 CTAs for 4096 rows) took a 64^2 cavity's 200
-// outer iterations from 0.67 s to 0.81 and 1.13 s.
+constexpr int kClMaxRows = 512;   // rows per CTA: one per thread
+// Largest system run on a cluster (16 CTAs of 256 rows and more).
 constexpr int kClMaxN = 8192;
 
 struct ClArgs {
@@ -56,60 +53,120 @@ struct ClArgs {
   int *iresult;     // [0] iterations [1] status
 };
 
-// shared-memory layout of one CTA (R rows, S slots)
+// shared-memory layout of one CTA (R rows, S slots): p and x, and the slots
+// beyond the fourth of a row are read from the staged copy
 struct ClLayout {
   int R, S;
   __host__ __device__ size_t bytes() const {
-    return (size_t)7 * R * sizeof(double) + (size_t)S * (sizeof(double) + sizeof(int)) +
+    return (size_t)2 * R * sizeof(double) + (size_t)S * (sizeof(double) + sizeof(int)) +
            (size_t)(R / 32 + 1) * sizeof(int);
   }
 };
 
 extern __shared__ __align__(16) unsigned char cl_smem[];
 
-template <int NV, typename F>
-__device__ __forceinline__ void cluster_allreduce(cg::cluster_group &cl, unsigned int &ep,
-                                                  double (&v)[NV], double (*part)[kMaxNV],
-                                                  double *red, F &&f) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+// The cluster's state of its sums (shared memory of each CTA): ExactState
+// without the words, and the two sets of posted limbs.
+struct ClSum {
+  ExactState xs;
+  long long post[2][32];
+  int part[3 * kLimbs * 32];
+};
+
+// The exact sum (see exact_sum) over a cluster.  overlap() runs in every
+// thread, side() in thread 32, between the arrival at the cluster barrier and
+// its wait; f(totals) in thread 0.
+template <int NV, typename O, typename S, typename F>
+__device__ __forceinline__ void cluster_sum(cg::cluster_group &cl, unsigned int &ep, ClSum &cs,
+                                            SumWindow<NV> &win, const double (&v)[NV],
+                                            O &&overlap, S &&side, F &&f) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int nb = (int)cl.num_blocks();
+  ExactState &xs = cs.xs;
+  bool first = true, have = true;
 #pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    const double t = warp_sum(v[q]);
-    if (lane == 0) red[q * 32 + warp] = t;
-  }
-  __syncthreads();
-  const unsigned int slot = ep++ & 1u;  // two slots: a CTA one reduction ahead never
-                                       // overwrites a partial still being read
-  if (warp == 0) {
+  for (int q = 0; q < NV; ++q) have = have && win.top[q] != kNoWindow;
+#pragma unroll 1
+  for (;;) {
+    if (!have) {  // the window from the largest partial of the cluster
+      const unsigned int set = ep++ & 1u;
+      __syncthreads();
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      const double t = warp_sum(lane < nwarps ? red[q * 32 + lane] : 0.0);
-      if (lane == 0) part[slot][q] = t;
+      for (int q = 0; q < NV; ++q) {
+        const int m = __reduce_max_sync(0xffffffffu, (__double2hiint(v[q]) >> 20) & 0x7ff);
+        if (lane == 0) cs.part[q * 32 + warp] = m;
+      }
+      __syncthreads();
+      if (warp == 0)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          const int m = __reduce_max_sync(0xffffffffu, lane < nw ? cs.part[q * 32 + lane] : 0);
+          if (lane == 0) cs.post[set][q] = m;
+        }
+      cl.sync();
+      if (warp == 0) {
+        bool nan = false;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          const int m = __reduce_max_sync(
+              0xffffffffu, lane < nb ? (int)*cl.map_shared_rank(&cs.post[set][q], lane) : 0);
+          nan = nan || m == 0x7ff;
+          if (lane == 0) win.top[q] = top_of_partials(m);
+        }
+        if (lane == 0) xs.nan = nan ? 1 : 0;
+      }
+      __syncthreads();
     }
-  }
-  cl.sync();
-  if (warp == 0) {
-    const int nb = (int)cl.num_blocks();
-    double t[NV];
+    const unsigned int set = ep++ & 1u;
+    bool ovf = false;
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double u = 0.0;
-      if (lane < nb) u = *cl.map_shared_rank(&part[slot][q], lane);
-      t[q] = warp_sum(u);
+    for (int q = 0; q < NV; ++q)
+      ovf = put_limbs(v[q], win.top[q], cs.part + q * kLimbs * 32) || ovf;
+    ovf = __any_sync(0xffffffffu, ovf);
+    if (lane == 0) xs.ovf[warp] = ovf ? 1 : 0;
+    if (threadIdx.x < NV) xs.top[threadIdx.x] = win.top[threadIdx.x];
+    if (threadIdx.x == 0) xs.sure = have ? 0 : 1;
+    __syncthreads();
+    if (warp == 0) cs.post[set][lane] = block_limbs(NV, cs.part, xs);
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    if (first) {
+      overlap();
+      if (threadIdx.x == 32) side();
+      __syncwarp();
     }
-    if (lane == 0) f(t);
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    if (warp == 0) {
+      long long d[kClMax], s = 0;
+#pragma unroll
+      for (int c = 0; c < kClMax; ++c)
+        d[c] = (c < nb) ? *cl.map_shared_rank(&cs.post[set][lane], c) : 0;
+#pragma unroll
+      for (int c = 0; c < kClMax; ++c) s += d[c];
+      const long long L = (long long)((unsigned long long)s << 22) >> 22;
+      limb_totals(NV, L, ((s - L) >> 42) != 0, true, xs);
+      if (lane == 0 && xs.flag == 1) {
+        window_set<NV>(win, xs.tot);
+        f(xs.tot);
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    if (xs.flag == 1) return;
+    first = false;
+    have = false;
   }
-  __syncthreads();
 }
 
-__global__ void __launch_bounds__(1024) pcg_cluster(ClArgs a) {
+__global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
   cg::cluster_group cl = cg::this_cluster();
-  __shared__ double red[kMaxNV * 32];
-  __shared__ double part[2][kMaxNV];
-  __shared__ double *rp[kClMax];  // each CTA's p, mapped into the cluster window
-  __shared__ double *rx[kClMax];  // and its x
+  __shared__ ClSum cs;
+  __shared__ SumWindow<1> wpq, wrz;
+  __shared__ SumWindow<2> wrr;
+  __shared__ SumWindow<3> w3;
   __shared__ struct {
-    double d, alpha, beta, conv, crit;
+    double d, alpha, beta, conv, crit2;
+    Divisor dv;
+    long long bound;
     int stop;
   } sh;
   const int rank = (int)cl.block_rank(), nb = (int)cl.num_blocks();
@@ -119,12 +176,13 @@ __global__ void __launch_bounds__(1024) pcg_cluster(ClArgs a) {
   const int ns = (rows + 31) / 32, s0 = r0 / 32;
   const int64_t sbase = a.A.sptr[s0];
   const int S = (int)(a.A.sptr[s0 + ns] - sbase);
-  double *p = reinterpret_cast<double *>(cl_smem);
-  double *x = p + R, *r = x + R, *z = r + R, *q = z + R, *mi = q + R, *dg = mi + R;
-  double *val = dg + R;
+  double *p = reinterpret_cast<double *>(cl_smem);  // read by the other CTAs
+  double *xv = p + R;                               // so is x, before and after the loop
+  double *val = xv + R;
   int *col = reinterpret_cast<int *>(val + S);  // (owner << 16) | local row
   int *sp = col + S;                            // slot offset of each local slice
   const bool has_diag = a.A.diag_mode != DIAG_NONE;
+  if (threadIdx.x == 0) wpq.top[0] = wrz.top[0] = wrr.top[0] = w3.top[0] = kNoWindow;
 #ifdef FVC_CHECK
   // check builds: columns outside [0, n) (whose owner CTA would not be in
   // the cluster) are counted here, redirected to this CTA's first row, and
@@ -142,114 +200,110 @@ __global__ void __launch_bounds__(1024) pcg_cluster(ClArgs a) {
     col[k] = (owner << 16) | (c - owner * R);
     val[k] = a.A.val[sbase + k];
   }
-  for (int i = threadIdx.x; i < R; i += blockDim.x) {
-    const bool own = i < rows;
-    mi[i] = own ? a.minv[r0 + i] : 0.0;
-    dg[i] = (own && has_diag) ? a.A.diag[r0 + i] : 0.0;
-    x[i] = (own && !a.init) ? a.x[r0 + i] : 0.0;
+  // this thread's row (blockDim >= R)
+  const int i = threadIdx.x;
+  const bool own = i < rows;
+  const double mi = own ? a.minv[r0 + i] : 0.0;
+  const double dg = (own && has_diag) ? a.A.diag[r0 + i] : 0.0;
+  const double bi = own ? a.b[r0 + i] : 0.0;
+  double x = (own && !a.init) ? a.x[r0 + i] : 0.0;
+  if (i < R) {
     p[i] = 0.0;
+    xv[i] = x;
   }
-  if (threadIdx.x < nb) {
-    rp[threadIdx.x] = cl.map_shared_rank(p, (int)threadIdx.x);
-    rx[threadIdx.x] = cl.map_shared_rank(x, (int)threadIdx.x);
+  cl.sync();  // every CTA's x in place
+  // its first four slots in registers: values, and where the neighbours' p are
+  int w = 0, base = 0;
+  double v4[4] = {0.0, 0.0, 0.0, 0.0};
+  const double *nb4[4] = {p, p, p, p};
+  if (own) {
+    base = sp[i >> 5] + (i & 31);
+    w = (sp[(i >> 5) + 1] - sp[i >> 5]) >> 5;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k < w) {
+        const int c = col[base + 32 * k], o = c >> 16, l = c & 0xffff;
+        v4[k] = val[base + 32 * k];
+        nb4[k] = (o == rank) ? p + l : cl.map_shared_rank(p, o) + l;
+      }
   }
-  cl.sync();  // every CTA's x and maps in place
-
-  // y_i = (A v)_i over the local row i with the reference's diagonal order;
-  // xf(owner, local) reads v
-  auto spmv_row = [&](int i, auto xf) -> double {
-    const int sl = i >> 5, lane = i & 31;
-    const int base = sp[sl], w = (sp[sl + 1] - base) >> 5;
-    const double xi = xf(rank, i);
-    double t = (a.A.diag_mode == DIAG_FIRST) ? dg[i] * xi : 0.0;
-    if (w <= 4) {
-      int c[4];
-      double v[4];
+  const ptrdiff_t dx = xv - p;  // x beside p in every CTA
+  // (A u)_i in the reference's diagonal order; off: where u lies from p
+  auto spmv_row = [&](double ui, ptrdiff_t off) -> double {
+    double u[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        c[k] = (k < w) ? col[base + 32 * k + lane] : 0;
-        v[k] = (k < w) ? val[base + 32 * k + lane] : 0.0;
-      }
-      double xv[4];
+    for (int k = 0; k < 4; ++k) u[k] = (k < w) ? nb4[k][off] : 0.0;
+    double t = (a.A.diag_mode == DIAG_FIRST) ? dg * ui : 0.0;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) xv[k] = (k < w) ? xf(c[k] >> 16, c[k] & 0xffff) : 0.0;
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (k < w) t = fma(v[k], xv[k], t);
-    } else {
-      for (int k = 0; k < w; ++k) {
-        const int c = col[base + 32 * k + lane];
-        t = fma(val[base + 32 * k + lane], xf(c >> 16, c & 0xffff), t);
-      }
+    for (int k = 0; k < 4; ++k)
+      if (k < w) t = fma(v4[k], u[k], t);
+#pragma unroll 1
+    for (int k = 4; k < w; ++k) {
+      const int c = col[base + 32 * k], o = c >> 16, l = c & 0xffff;
+      const double *q = (o == rank) ? p : cl.map_shared_rank(p, o);
+      t = fma(val[base + 32 * k], q[l + off], t);
     }
-    if (a.A.diag_mode == DIAG_LAST) t = fma(dg[i], xi, t);
+    if (a.A.diag_mode == DIAG_LAST) t = fma(dg, ui, t);
     return t;
   };
-  auto xread = [&](int o, int l) { return (o == rank) ? x[l] : rx[o][l]; };
 
   unsigned int ep = 0;
   const bool rule0 = a.stop_rule == 0;
+  auto none = [] {};
   // r = b - A x ; z = r/m ; p = z ; d = r.z
+  double r = own ? bi - (a.init ? 0.0 : spmv_row(x, dx)) : 0.0;
+  double z = r * mi;
 #ifdef FVC_CHECK
-  double acc[3] = {0.0, 0.0, (threadIdx.x == 0 && s_bad != 0) ? 1.0 : 0.0};
-#else
-  double acc[2] = {0.0, 0.0};
-#endif
-  for (int i = threadIdx.x; i < rows; i += blockDim.x) {
-    const double ax = a.init ? 0.0 : spmv_row(i, xread);
-    const double bi = a.b[r0 + i];
-    const double ri = bi - ax;
-    const double zi = ri * mi[i];
-    r[i] = ri;
-    z[i] = zi;
-    p[i] = zi;
-    acc[0] = fma(ri, zi, acc[0]);
-    acc[1] = fma(bi, bi, acc[1]);
-  }
-#ifdef FVC_CHECK
-  cluster_allreduce<3>(cl, ep, acc, part, red, [&](const double *t) {
+  double acc[3] = {r * z, bi * bi, (threadIdx.x == 0 && s_bad != 0) ? 1.0 : 0.0};
+  __syncthreads();
+  cluster_sum<3>(cl, ep, cs, w3, acc, none, none, [&](const double *t) {
     sh.stop = (t[2] > 0.0) ? 3 : 0;
 #else
-  cluster_allreduce<2>(cl, ep, acc, part, red, [&](const double *t) {
+  double acc[2] = {r * z, bi * bi};
+  cluster_sum<2>(cl, ep, cs, wrr, acc, none, none, [&](const double *t) {
     sh.stop = 0;
 #endif
     sh.d = t[0];
-    sh.conv = rule0 ? a.tol * sqrt(fabs(t[0])) : a.tol * sqrt(t[1]);
-    sh.crit = 0.0;
+    sh.conv = a.tol * root(rule0 ? fabs(t[0]) : t[1]);
+    sh.bound = sqrt_bound(sh.conv);
+    sh.crit2 = 0.0;
+    wrz.top[0] = window_top(t[0]);
+    wrr.top[1] = kNoWindow;
   });
   int j, status = FVC_OK;
-  double beta = 0.0;
+  double beta = 0.0, pi = 0.0;
   const int jmax = (sh.stop == 3) ? 0 : a.maxit;  // 3: a failed check (check builds)
   if (sh.stop == 3) status = FVC_ERR_ARG;
+#pragma unroll 1
   for (j = 1; j <= jmax; ++j) {
-    if (j > 1) {  // p = z + beta p on the own rows, then visible to the cluster
-      for (int i = threadIdx.x; i < rows; i += blockDim.x) p[i] = fma(beta, p[i], z[i]);
-      cl.sync();
-    }
-    double pq[1] = {0.0};
-    for (int i = threadIdx.x; i < rows; i += blockDim.x) {
-      const double qi = spmv_row(i, [&](int o, int l) { return (o == rank) ? p[l] : rp[o][l]; });
-      q[i] = qi;
-      pq[0] = fma(p[i], qi, pq[0]);
-    }
-    cluster_allreduce<1>(cl, ep, pq, part, red, [&](const double *t) { sh.alpha = sh.d / t[0]; });
+    // p = z + beta p on the own rows (the first: p = z), then visible to the cluster
+    pi = fma(beta, pi, z);
+    if (i < R) p[i] = pi;
+    cl.sync();
+    const double qi = own ? spmv_row(pi, 0) : 0.0;
+    const double pq[1] = {pi * qi};
+    cluster_sum<1>(cl, ep, cs, wpq, pq, none, [&] { sh.dv.set(sh.d); },
+                   [&](const double *t) { sh.alpha = quick_quotient(sh.d, t[0]); });
     const double alpha = sh.alpha;
-    double rz[2] = {0.0, 0.0};
-    for (int i = threadIdx.x; i < rows; i += blockDim.x) {
-      x[i] = fma(alpha, p[i], x[i]);
-      const double ri = fma(-alpha, q[i], r[i]);
-      const double zi = ri * mi[i];
-      r[i] = ri;
-      z[i] = zi;
-      rz[0] = fma(ri, zi, rz[0]);
-      rz[1] = fma(ri, ri, rz[1]);
-    }
-    cluster_allreduce<2>(cl, ep, rz, part, red, [&](const double *t) {
-      sh.beta = t[0] / sh.d;
+    r = fma(-alpha, qi, r);
+    z = r * mi;
+    auto step = [&](const double *t) {
+      sh.beta = quotient(t[0], sh.dv);
       sh.d = sh.beta * sh.d;
-      sh.crit = rule0 ? sqrt(fabs(sh.d)) : sqrt(t[1]);
-      sh.stop = (!(sh.crit == sh.crit) || isinf(sh.d)) ? 2 : (sh.crit < sh.conv ? 1 : 0);
-    });
+      const double crit2 = rule0 ? fabs(sh.d) : t[rule0 ? 0 : 1];
+      sh.crit2 = crit2;
+      sh.stop = (is_nan_bits(crit2) || not_finite_bits(sh.d)) ? 2
+                : sqrt_below(crit2, sh.conv, sh.bound)        ? 1
+                                                              : 0;
+    };
+    auto update_x = [&] { x = fma(alpha, pi, x); };
+    if (rule0) {
+      const double rz[1] = {r * z};
+      cluster_sum<1>(cl, ep, cs, wrz, rz, update_x, none, step);
+    } else {
+      const double rr[2] = {r * z, r * r};
+      cluster_sum<2>(cl, ep, cs, wrr, rr, update_x, none, step);
+    }
     if (sh.stop == 2) {
       status = FVC_ERR_NAN;
       break;
@@ -263,21 +317,22 @@ __global__ void __launch_bounds__(1024) pcg_cluster(ClArgs a) {
   }
   if (status == FVC_ERR_ARG) j = 0;
   // x.Ax, |b - Ax|^2, |b|^2 (x complete in every CTA after the barrier)
+  if (i < R) xv[i] = x;
+  if (threadIdx.x == 0) w3.top[0] = kNoWindow;
   cl.sync();
   double e3[3] = {0.0, 0.0, 0.0};
-  for (int i = threadIdx.x; i < rows; i += blockDim.x) {
-    const double ax = spmv_row(i, xread);
-    const double bi = a.b[r0 + i], rr = bi - ax;
-    e3[0] = fma(x[i], ax, e3[0]);
-    e3[1] = fma(rr, rr, e3[1]);
-    e3[2] = fma(bi, bi, e3[2]);
-    a.x[r0 + i] = x[i];
+  if (own) {
+    const double ax = spmv_row(x, dx), rr = bi - ax;
+    e3[0] = x * ax;
+    e3[1] = rr * rr;
+    e3[2] = bi * bi;
+    a.x[r0 + i] = x;
   }
-  cluster_allreduce<3>(cl, ep, e3, part, red, [&](const double *t) {
+  cluster_sum<3>(cl, ep, cs, w3, e3, none, none, [&](const double *t) {
     if (rank == 0) {
       a.result[0] = t[0];
       a.result[1] = sh.conv;
-      a.result[2] = sh.crit;
+      a.result[2] = root(sh.crit2);
       a.result[3] = t[1];
       a.result[4] = t[2];
       a.iresult[0] = j;

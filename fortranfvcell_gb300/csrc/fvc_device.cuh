@@ -537,6 +537,10 @@ __device__ __forceinline__ bool grid_sum_d(const GridSync &gs, Episode &episode,
 static __device__ __noinline__ double divide(double t, double d) { return t / d; }
 static __device__ __noinline__ double root(double v) { return sqrt(v); }
 
+__device__ __forceinline__ bool not_finite_bits(double v) {
+  return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000;
+}
+
 // A divisor whose reciprocal was taken ahead of the dividend.
 struct Divisor {
   double d, r;  // r = 1/d, or 0 when d is too far from 1 for quotient()
@@ -559,6 +563,21 @@ __device__ __forceinline__ double quotient(double t, const Divisor &v) {
   return z;
 }
 
+// t / d from scratch: the reciprocal's hardware approximation (rcp.approx.f64,
+// 20 bits and more), one Newton step, Markstein's correction of t * r as above
+// (about 360 clocks against 570 of the division).  Divisors out of range, and
+// quotients that are not finite, take the division.
+__device__ __forceinline__ double quick_quotient(double t, double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  r = fma(fma(-d, r, 1.0), r, r);
+  const double q = t * r;
+  const double z = fma(fma(-q, d, t), r, q);
+  const int e = (__double2hiint(d) >> 20) & 0x7ff;
+  if (e <= 1023 - 500 || e >= 1023 + 500 || not_finite_bits(z)) return divide(t, d);
+  return z;
+}
+
 // The stopping test sqrt(s) < conv, without the square root while s is
 // clearly above conv^2 (bound from sqrt_bound; s >= 0 or NaN: the bits of
 // nonnegative doubles order like the numbers, a NaN above all of them).
@@ -574,9 +593,6 @@ __device__ __forceinline__ bool sqrt_below(double s, double conv, long long boun
 }
 __device__ __forceinline__ bool is_nan_bits(double v) {
   return (__double_as_longlong(v) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
-}
-__device__ __forceinline__ bool not_finite_bits(double v) {
-  return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000;
 }
 
 // No scalar work beside a sum.
@@ -730,6 +746,11 @@ __device__ __forceinline__ void exact_init(ExactState &xs) {  // a __syncthreads
   for (int i = threadIdx.x; i < 2 * kXWords; i += blockDim.x) (&xs.snap[0][0])[i] = 0;
 }
 
+// The top of a window that holds partials of biased exponents up to m
+__device__ __forceinline__ int top_of_partials(int m) {
+  return max(min(m, 0x7fe), 1) - 1022 + 1;
+}
+
 // The window of a sum from its partials: its top above the largest exponent
 // (ex, biased) of all threads of all blocks, by a maximum exchanged through
 // the reduction slots and a barrier.  Cold: the first sum of a kind, and one
@@ -770,8 +791,7 @@ static __device__ __noinline__ bool window_by_partials(const GridSync &gs, Episo
         m = max(m, (int)__longlong_as_double((long long)ld_slot(slots + (size_t)q * gs.nblocks + b).v));
       m = __reduce_max_sync(0xffffffffu, m);
       nan = nan || m == 0x7ff;
-      // |partial| < 2^(m - 1022)
-      if (lane == 0) top[q] = max(min(m, 0x7fe), 1) - 1022 + 1;
+      if (lane == 0) top[q] = top_of_partials(m);
     }
     if (lane == 0) xs.nan = nan ? 1 : 0;
   }
@@ -779,17 +799,11 @@ static __device__ __noinline__ bool window_by_partials(const GridSync &gs, Episo
   return true;
 }
 
-// Warp 0's part of an exact sum of nv quantities: the block's limbs from its
-// warps' (part), their exchange through the words, the totals into xs.tot and
-// the verdict into xs.flag (0 a wait exceeded its bound, 1 good, 2 the window
-// did not hold it).
-__device__ __forceinline__ void exact_words(unsigned long long *xw, int *err, unsigned int nb,
-                                                unsigned int set, int nv, const int *part,
-                                                ExactState &xs) {
+// Warp 0's part of an exact sum of nv quantities.  First the block's limbs from
+// its warps' (part): lane 8 q + k gets limb k of quantity q with the overflow
+// mark in bits 42 on.
+__device__ __forceinline__ long long block_limbs(int nv, const int *part, const ExactState &xs) {
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  // lane 8 q + k holds limb k of quantity q
-  const int lq = lane >> 3, lk = lane & 7;
-  const bool mine = lq < nv && lk < kLimbs;
   long long w = 0;
 #pragma unroll 1
   for (int q = 0; q < nv; ++q)
@@ -800,14 +814,45 @@ __device__ __forceinline__ void exact_words(unsigned long long *xw, int *err, un
       if (lane == 8 * q + k) w = r;
     }
   const bool o = __any_sync(0xffffffffu, lane < nw && xs.ovf[lane] != 0);
+  return w + ((long long)(o ? 1 : 0) << 42);
+}
+// Then, from the limbs of all blocks (L) and whether any overflowed (bad), the
+// totals into xs.tot and the verdict into xs.flag (0 a wait exceeded its bound,
+// 1 good, 2 the window did not hold it).
+__device__ __forceinline__ void limb_totals(int nv, long long L, bool bad, bool ok,
+                                            ExactState &xs) {
+  const int lane = threadIdx.x & 31, lq = lane >> 3, lk = lane & 7;
+  const bool mine = lq < nv && lk < kLimbs;
+  const int top = xs.top[mine ? lq : 0];
+  // the limbs of a quantity added in FP64
+  double tq = mine ? limb_value(L, lk, top) : 0.0;
+#pragma unroll
+  for (int k = 1; k < 8; k <<= 1) tq = __dadd_rn(tq, __shfl_xor_sync(0xffffffffu, tq, k));
+  if (xs.sure) {
+    bad = false;  // only NaN and Inf overflow a window that follows from the partials
+    if (xs.nan) tq = __longlong_as_double(0x7ff8000000000000ll);
+  } else {
+    bad = mine && (bad || sum_bad(tq, top));
+  }
+  bad = __any_sync(0xffffffffu, bad);
+  ok = __all_sync(0xffffffffu, ok);
+  if (lk == 0 && lq < nv) xs.tot[lq] = tq;
+  if (lane == 0) xs.flag = !ok ? 0 : bad ? 2 : 1;
+  __syncwarp();
+}
+// The exchange over a grid between the two, through the words of this set.
+__device__ __forceinline__ void exact_words(unsigned long long *xw, int *err, unsigned int nb,
+                                            unsigned int set, int nv, const int *part,
+                                            ExactState &xs) {
+  const int lane = threadIdx.x & 31, lq = lane >> 3, lk = lane & 7;
+  const bool mine = lq < nv && lk < kLimbs;
+  const long long w = block_limbs(nv, part, xs);
   long long L = 0;
   bool ok = true, bad = false;
   // (the other lanes poll along on the first word, see wait_count)
   unsigned long long *word = xw + set * kXWords + (mine ? lane : 0);
-  const int top = xs.top[mine ? lq : 0];
   if (mine)  // bits 0-41 the limb, 42-52 blocks that overflowed, 53-63 blocks
-    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(word),
-                 "l"(w + ((long long)(o ? 1 : 0) << 42) + (1ll << 53))
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(w + (1ll << 53))
                  : "memory");
   const unsigned long long prev = xs.snap[set][mine ? lane : 0];
   __syncwarp();
@@ -834,21 +879,7 @@ __device__ __forceinline__ void exact_words(unsigned long long *xw, int *err, un
   }
   if (mine) xs.snap[set][lane] = now;
   __syncwarp();
-  // the limbs of a quantity added in FP64
-  double tq = mine ? limb_value(L, lk, top) : 0.0;
-#pragma unroll
-  for (int k = 1; k < 8; k <<= 1) tq = __dadd_rn(tq, __shfl_xor_sync(0xffffffffu, tq, k));
-  if (xs.sure) {
-    bad = false;  // only NaN and Inf overflow a window that follows from the partials
-    if (xs.nan) tq = __longlong_as_double(0x7ff8000000000000ll);
-  } else {
-    bad = bad || (mine && sum_bad(tq, top));
-  }
-  bad = __any_sync(0xffffffffu, bad);
-  ok = __all_sync(0xffffffffu, ok);
-  if (lk == 0 && lq < nv) xs.tot[lq] = tq;
-  if (lane == 0) xs.flag = !ok ? 0 : bad ? 2 : 1;
-  __syncwarp();
+  limb_totals(nv, L, bad, ok, xs);
 }
 
 // Warps 0 and 1 of the block meet (the values of side() for f()).
