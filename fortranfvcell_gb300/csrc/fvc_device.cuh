@@ -863,9 +863,9 @@ __device__ __forceinline__ void exact_words(unsigned long long *xw, int *err, un
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(word) : "memory");
     const long long d = (long long)(now - prev);
     L = (long long)((unsigned long long)d << 22) >> 22;
-    const long long c = (d - L) >> 42;
-    bad = (c & 2047) != 0;
-    if (__all_sync(0xffffffffu, (unsigned int)(c >> 11) == nb)) break;
+    const unsigned int c = (unsigned int)((unsigned long long)(d - L) >> 42);
+    bad = (c & 2047u) != 0;
+    if (__all_sync(0xffffffffu, (c >> 11) == nb)) break;
     if ((++spins & 63u) == 0) {
       const uint64_t ns = global_ns();
       if (t0 == 0) t0 = ns;

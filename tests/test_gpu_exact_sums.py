@@ -94,6 +94,20 @@ def test_block_counts(orc, system, code, kw):
     assert np.array_equal(got, again)
 
 
+@pytest.mark.parametrize("kw", [dict(block_threads=128), dict(block_threads=256),
+                                dict(max_blocks=1)])
+def test_many_blocks(orc, kw):
+    """More than 1024 blocks (128 threads): the counts of the words' top bits."""
+    from fortranfvcell_gb300 import mesh
+    s = pressure(orc, mesh.square_mesh(430, 430, kind="quad"))
+    s = dict(s, au=-np.ones_like(s["au"]), ad=np.full(s["n"], 4.2))
+    b = np.random.default_rng(11).uniform(-1.0, 1.0, s["n"])
+    got, st = _solve(s, 1, b, 1e-12, **kw)
+    want, so = _solve(s, 1, b, 1e-12)
+    assert np.linalg.norm(got - want) <= 1e-10 * np.linalg.norm(want)
+    assert st.rel_residual <= 1e-9 and so.rel_residual <= 1e-9
+
+
 def test_zero_and_nan_right_hand_sides(system):
     """b = 0: r.z = 0 and p.q = 0, the restated 0/0; a NaN ends the solve."""
     from fortranfvcell_gb300._lib import FVC_ERR_NAN, FvcError
