@@ -1034,27 +1034,25 @@ int32_t run_pcg(const DeviceMatrix &A, Scratch &S, const double *b, double *x, d
     const int32_t rc = run_pcg_cluster(A, S, b, x, tol, maxit, init, o, stream, st);
     if (rc != FVC_ERR_UNSUPPORTED) return rc;
   }
-  // p stored from 262144 rows on: per iteration on GB300 (same bits either
-  // way) 98k rows 14.5 vs 13.0 us, 393k 23.0 vs 23.5, 1.57M 58.8 vs 66.2,
-  // 4.19M 146 vs 161 us (stored vs formed at every read)
+  // p stored from 262144 rows on: per iteration on GB300, stored against
+  // formed at every read, 138k rows 10.5 vs 10.0 us, 260k 13.3 vs 13.1, 360k
+  // 17.0 vs 16.7, 1.05M 34.5 vs 38
   if (A.n >= kStorePRows)
     return run_persistent(pcg_f64<true>, A, S, b, x, tol, maxit, init, o, stream, st, 5, false);
   return run_persistent(pcg_f64<false>, A, S, b, x, tol, maxit, init, o, stream, st, 5, false);
 }
 
 // FP64 BiCGSTAB with z stored once per row from this many rows on (below,
-// the two extra grid barriers cost more than the FP64 they save; the 262k-
-// row enthalpy solves of a 512^2 natural-convection loop gain: 30 outer
-// iterations 2.93 -> 2.77 s; the 65k-row ones of a 256^2 loop lose: 200
-// outer iterations 6.26 -> 6.55 s)
-constexpr int kStoreZRows = 131072;
+// the two extra grid barriers cost more than the FP64 they save).  Per
+// iteration, stored against formed at every read: 52.9k rows 16.8 vs 15.9 us,
+// 90k 18.8 vs 19.5, 122k 21.3 vs 23.5, 260k 28.0 vs 35.4
+constexpr int kStoreZRows = 73728;
 
 // BiCGSTAB on one cluster up to this many rows (a block of 256 threads per
-// eight slices, at most 16 blocks): the grid-wide kernel's grid waits cost
-// more than a cluster's FP64 throughput there.  Per iteration on GB300,
-// cluster against grid-wide: 2025 rows 15.3 vs 18.3 us, 4096 rows 15.3 vs
-// 18.3, 8100 rows 19.9 vs 19.4, 16384 rows 28.8 vs 21.9
-constexpr int kBcgClusterRows = 8192;
+// eight slices, at most 16 blocks); above, the grid-wide kernel.  Per
+// iteration on GB300, cluster against grid-wide: 256 rows 10.0 vs 10.6 us,
+// 1024 rows 13.7 vs 11.5, 4096 rows 13.9 vs 11.8, 8100 rows 18.5 vs 12.2
+constexpr int kBcgClusterRows = 512;
 
 // Enqueues the cluster BiCGSTAB when the system is small enough, the caller
 // left the launch shape automatic and one cluster fits; FVC_ERR_UNSUPPORTED,
