@@ -37,13 +37,12 @@ namespace {
 
 constexpr int MS = 4;
 
-struct Geom;
 struct Mesh {
   int numel, nshared, ld;  // ld = nshared + 1 (ix rows: nodes, then material)
   const double *coor;
   const int32_t *ix, *nelcon, *num, *pedge;
   const double *sedge, *e;
-  const Geom *geo;  // the cells' geometry computed once (null: per kernel)
+  const double *geo;  // the cells' geometry computed once (null: per kernel)
 };
 
 __device__ __forceinline__ int ixa(const Mesh &m, int i, int c) {  // ix(i, c), 1-based
@@ -124,14 +123,6 @@ __device__ double areacell(const double eta[2][MS], int ns) {
   a = a + half_cross(eta[0][0], eta[1][0], eta[0][3], eta[1][3]);
   a = a + half_cross(eta[0][1], eta[1][1], eta[0][2], eta[1][2]);
   return 0.5 * a;
-}
-
-// the neighbour links alone (what the kernels use of the stencil when the
-// geometry comes from the mesh's cache)
-__device__ void gather_links(Stencil &S, const Mesh &m, int nel) {
-  S.ns = nsides(m, nel);
-  for (int j = 1; j <= m.nshared; ++j)
-    S.viz[j - 1] = m.nelcon[(j - 1) + (size_t)(nel - 1) * m.nshared];
 }
 
 // cellGeom2D + ghost centroids + vectorKm2d for the central cell
@@ -218,28 +209,157 @@ __device__ void geom(Geom &G, const Stencil &S) {
   }
 }
 
-// A cell's links and geometry: from the mesh's geometry cache when it has
-// one (geom() of the same stencil, stored once: the same bits), else
-// computed here as the reference's cell routines do
-__device__ __forceinline__ void cell_setup(Stencil &S, Geom &G, const Mesh &m, int nel) {
-  if (m.geo) {
-    gather_links(S, m, nel);
-    G = m.geo[nel - 1];
-  } else {
-    gather(S, m, nel);
-    geom(G, S);
-  }
+// ---- the geometry cache -----------------------------------------------------
+// Per face and cell what the cell kernels take from the geometry, one array
+// per quantity over the cells (a warp's loads are coalesced; 600-byte records
+// per cell went through local memory): beside the geometry itself the
+// combinations that depend on it alone -- interpolation weights, the
+// non-orthogonality products, the Green-Gauss polygon's normals and area --
+// each computed by the same operations, and so to the same bits, as a kernel
+// without the cache computes them.  The kernels are bound by the FP64 pipe (one
+// warp instruction per 76 clocks and SM sub-partition): an operation read
+// instead of recomputed saves 0.4 us per 200k cells, its 8 bytes cost 0.24.
+// 200k cells of a mixed mesh, records against this: gradient 116 -> 22 us,
+// momentum 354 -> 298, p' 168 -> 104.
+enum FaceField : int {
+  kN1, kN2,      // unit normal
+  kMeta,         // face length
+  kKsi1, kKsi2,  // unit vector to the neighbour's centroid
+  kMksi,         // its distance
+  kAlpha,        // mksif / mksi, the neighbour's interpolation weight
+  kNk,           // n . ksi
+  kNkMksi,       // nk mksi
+  kKs1, kKs2,    // mksi ksi
+  kNks,          // n . (mksi ksi)
+  kKm1, kKm2,    // vectorKm2d
+  kDf1, kDf2,    // centroid to face midpoint
+  kCa,           // its component along n
+  kDxc1, kDxc2,  // own minus the neighbour's centroid
+  kDxm1, kDxm2,  // face midpoint minus the neighbour's centroid
+  kGn1, kGn2,    // Green-Gauss polygon: normal of side l
+  kFaceFields
+};
+constexpr int kAreaField = kFaceFields * MS, kGgAreaField = kAreaField + 1;
+constexpr int kCellFields = kGgAreaField + 1;
+constexpr size_t geo_pitch(int numel) { return ((size_t)numel + 31) / 32 * 32; }
+constexpr size_t geo_bytes(int numel) {  // the fields, then the cells' side counts
+  return geo_pitch(numel) * (kCellFields * sizeof(double) + sizeof(int32_t));
 }
 
+// face i (0-based) of the central cell from its Geom
+__device__ double face_field(const Geom &G, const Stencil &S, int f, int i) {
+  const double n1 = G.n[0][i], n2 = G.n[1][i];
+  const double k1 = G.ksi[0][i], k2 = G.ksi[1][i], mk = G.mksi[i];
+  const int s2 = (i + 1) % S.ns;
+  switch (f) {
+    case kN1: return n1;
+    case kN2: return n2;
+    case kMeta: return G.meta[i];
+    case kKsi1: return k1;
+    case kKsi2: return k2;
+    case kMksi: return mk;
+    case kAlpha: return G.mksif[i] / mk;
+    case kNk: return n1 * k1 + n2 * k2;
+    case kNkMksi: return (n1 * k1 + n2 * k2) * mk;
+    case kKs1: return mk * k1;
+    case kKs2: return mk * k2;
+    case kNks: return (mk * k1) * n1 + (mk * k2) * n2;
+    case kKm1: return G.km[0][i];
+    case kKm2: return G.km[1][i];
+    case kDf1: return G.df[0][i];
+    case kDf2: return G.df[1][i];
+    case kCa: return G.ca[i];
+    case kDxc1: return G.xc[0][MS] - G.xc[0][i];
+    case kDxc2: return G.xc[1][MS] - G.xc[1][i];
+    case kDxm1: return G.xm[0][i] - G.xc[0][i];
+    case kDxm2: return G.xm[1][i] - G.xc[1][i];
+    case kGn1: return G.xcg[1][s2] - G.xcg[1][i];
+    default: return -(G.xcg[0][s2] - G.xcg[0][i]);
+  }
+}
+__device__ double gg_area(const Geom &G, int ns) {
+  double eta[2][MS];
+  for (int i = 0; i < 2; ++i)
+    for (int l = 0; l < ns; ++l) eta[i][l] = G.xcg[i][(l + 1) % ns] - G.xcg[i][l];
+  return areacell(eta, ns);
+}
+
+// A cell as the kernels see it: its sides, its neighbours (1-based; <= 0 a
+// boundary face), its geometry from the mesh's cache (kGeo) or computed here
+// as the reference's cell routines do.
+template <bool kGeo>
+struct Cell {
+  int ns, viz[MS];
+  const double *g;
+  size_t pitch;
+  Stencil S;
+  Geom G;
+  __device__ __forceinline__ Cell(const Mesh &m, int nel) {
+    if (kGeo) {
+      pitch = geo_pitch(m.numel);
+      g = m.geo + (nel - 1);
+      ns = reinterpret_cast<const int32_t *>(m.geo + pitch * kCellFields)[nel - 1];
+      for (int j = 0; j < MS; ++j)
+        viz[j] = (j < m.nshared) ? m.nelcon[j + (size_t)(nel - 1) * m.nshared] : 0;
+    } else {
+      gather(S, m, nel);
+      geom(G, S);
+      ns = S.ns;
+      for (int j = 0; j < MS; ++j) viz[j] = (j < m.nshared) ? S.viz[j] : 0;
+    }
+  }
+  __device__ __forceinline__ int neighbour(int i) const {  // of face i, 0-based
+    return i == 0 ? viz[0] : i == 1 ? viz[1] : i == 2 ? viz[2] : viz[3];
+  }
+  __device__ __forceinline__ double face(int f, int i) const {
+    return kGeo ? __ldg(g + (size_t)(f * MS + i) * pitch) : face_field(G, S, f, i);
+  }
+  __device__ __forceinline__ double area() const {
+    return kGeo ? __ldg(g + kAreaField * pitch) : G.area;
+  }
+  __device__ __forceinline__ double polygon_area() const {
+    return kGeo ? __ldg(g + kGgAreaField * pitch) : gg_area(G, S.ns);
+  }
+};
+
+// Four values a loop over the faces writes and later loops read, selected by
+// the face (an indexed array would live in local memory)
+struct Four {
+  double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
+  __device__ __forceinline__ void set(int i, double v) {
+    if (i == 0) v0 = v;
+    if (i == 1) v1 = v;
+    if (i == 2) v2 = v;
+    if (i == 3) v3 = v;
+  }
+  __device__ __forceinline__ double get(int i) const {
+    return i == 0 ? v0 : i == 1 ? v1 : i == 2 ? v2 : v3;
+  }
+};
+
 // every cell's geometry into the cache
-__global__ void geometry_kernel(Mesh m, Geom *out) {
+__global__ void geometry_kernel(Mesh m, double *out) {
   const int nel = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (nel > m.numel) return;
   Stencil S;
   Geom G;
   gather(S, m, nel);
   geom(G, S);
-  out[nel - 1] = G;
+  const size_t pitch = geo_pitch(m.numel);
+  double *o = out + (nel - 1);
+#pragma unroll 1
+  for (int i = 0; i < MS; ++i) {
+    const bool face = i < S.ns, inner = face && S.viz[i] > 0;
+#pragma unroll 1
+    for (int f = 0; f < kFaceFields; ++f) {
+      // a boundary face has no neighbour: only these are read there
+      const bool bnd = f <= kMeta || f == kDf1 || f == kDf2 || f == kCa || f >= kGn1;
+      o[(size_t)(f * MS + i) * pitch] = (inner || (face && bnd)) ? face_field(G, S, f, i) : 0.0;
+    }
+  }
+  o[kAreaField * pitch] = G.area;
+  o[kGgAreaField * pitch] = gg_area(G, S.ns);
+  reinterpret_cast<int32_t *>(out + pitch * kCellFields)[nel - 1] = S.ns;
 }
 
 __device__ double limit(double r, int icod) {
@@ -259,111 +379,101 @@ __device__ double limit(double r, int icod) {
   }
 }
 
-__device__ void green_gauss(const Geom &G, int ns, const double *ug, double &g1, double &g2) {
-  double eta[2][MS], n[2][MS];
-  for (int i = 1; i <= 2; ++i)
-    for (int l = 1; l <= ns; ++l) {
-      const int s1 = l, s2 = (l % ns) + 1;
-      eta[i - 1][l - 1] = G.xcg[i - 1][s2 - 1] - G.xcg[i - 1][s1 - 1];
-    }
-  for (int l = 1; l <= ns; ++l) {
-    n[0][l - 1] = eta[1][l - 1];
-    n[1][l - 1] = -eta[0][l - 1];
-  }
-  const double area = areacell(eta, ns);
-  double um[MS];
-  for (int l = 1; l <= ns; ++l) {
-    const int s1 = l, s2 = (l % ns) + 1;
-    um[l - 1] = 0.5 * (ug[s2 - 1] + ug[s1 - 1]);
-  }
+template <bool kGeo>
+__device__ __forceinline__ void green_gauss(const Cell<kGeo> &C, const Four &ug, double &g1,
+                                            double &g2) {
   double a = 0.0, b = 0.0;
-  for (int i = 1; i <= ns; ++i) {
-    const double uf = um[i - 1];
-    a = a + uf * n[0][i - 1];
-    b = b + uf * n[1][i - 1];
-  }
+#pragma unroll
+  for (int i = 0; i < MS; ++i)
+    if (i < C.ns) {
+      const double uf = 0.5 * (ug.get(i + 1 == C.ns ? 0 : i + 1) + ug.get(i));
+      a = a + uf * C.face(kGn1, i);
+      b = b + uf * C.face(kGn2, i);
+    }
+  const double area = C.polygon_area();
   g1 = a / area;
   g2 = b / area;
 }
 
-// assbly: ld[0..nshared-1] neighbour equations (0 = none), ld[nshared] own
-__device__ void assbly(double *ad, double *au, double *f, const int32_t *ia, const int32_t *ja,
-                       const double *la, double p, const int *ld, int nshared, int matriz,
-                       bool forces, bool matrix) {
-  const int n = ld[nshared];
+// assbly: the equation n of the cell, of its neighbours (0 = none), the
+// coefficients la of the neighbours, the diagonal and the right-hand side p
+template <bool kGeo>
+__device__ __forceinline__ void assbly(const Mesh &m, const Cell<kGeo> &C, int nel, double *ad,
+                                       double *au, double *f, const int32_t *ia,
+                                       const int32_t *ja, const Four &la, double diag, double p,
+                                       int matriz, bool matrix) {
+  const int n = m.num[nel - 1];
+  f[n - 1] = p;
+  if (!matrix) return;
+  ad[n - 1] = diag;
+  int ld[MS];
+#pragma unroll
+  for (int j = 0; j < MS; ++j)
+    ld[j] = (j < C.ns && C.viz[j] > 0) ? m.num[C.viz[j] - 1] : 0;
   if (matriz == 1) {
-    if (matrix) ad[n - 1] = la[nshared];
-    if (forces) f[n - 1] = p;
-    const int ipont = ia[n - 1], iak = ia[n] - ia[n - 1];
-    if (matrix)
-      for (int j = 1; j <= nshared; ++j) {
-        const int l = ld[j - 1];
-        if (l > 0)
-          for (int i = 1; i <= iak; ++i) {
-            const int k = ipont + i - 1;
-            if (l == ja[k - 1]) au[k - 1] = -la[j - 1];
-          }
-      }
-  } else {  // 4: ELLPACK
-    if (forces) f[n - 1] = p;
-    if (matrix) {
-      ad[n - 1] = la[nshared];
-      for (int j = 1; j <= nshared; ++j) {
-        const int l = ld[j - 1];
-        au[(j - 1) + (size_t)(n - 1) * nshared] = (l > 0) ? -la[j - 1] : 0.0;
-      }
+    const int ipont = ia[n - 1], iak = ia[n] - ipont;
+#pragma unroll 1
+    for (int i = 0; i < iak; ++i) {
+      const int k = ipont + i - 1, l = ja[k];
+#pragma unroll
+      for (int j = 0; j < MS; ++j)
+        if (j < m.nshared && ld[j] > 0 && l == ld[j]) au[k] = -la.get(j);
     }
+  } else {  // 4: ELLPACK
+#pragma unroll
+    for (int j = 0; j < MS; ++j)
+      if (j < m.nshared) au[j + (size_t)(n - 1) * m.nshared] = (ld[j] > 0) ? -la.get(j) : 0.0;
   }
 }
 
-__global__ void gradient_kernel(Mesh m, int kind, int comp, const double *__restrict__ u,
+template <bool kGeo>
+__global__ void __launch_bounds__(128) gradient_kernel(Mesh m, int kind, int comp, const double *__restrict__ u,
                                 double *__restrict__ grad, int *err) {
   const int nel = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (nel > m.numel) return;
-  Stencil S;
-  Geom G;
-  cell_setup(S, G, m, nel);
+  const Cell<kGeo> C(m, nel);
   const double uP = u[nel - 1];
   const double go1 = v2(grad, 1, nel), go2 = v2(grad, 2, nel);
-  double ug[MS];
-  for (int i = 1; i <= S.ns; ++i) {
-    const int v = S.viz[i - 1];
+  Four ug;
+#pragma unroll 1
+  for (int i = 1; i <= C.ns; ++i) {
+    const int v = C.neighbour(i - 1);
     if (v > 0) {
-      ug[i - 1] = u[v - 1];
+      ug.set(i - 1, u[v - 1]);
       continue;
     }
     const int pe = pedge(m, i, nel);
     if (kind == 1) {
       if (pe == 0)
-        ug[i - 1] = -uP;
+        ug.set(i - 1, -uP);
       else if (pe == 1 || pe == 2)
-        ug[i - 1] = sedge(m, comp, i, nel);
+        ug.set(i - 1, sedge(m, comp, i, nel));
       else if (pe == 3 || pe == 4)
-        ug[i - 1] = uP;
+        ug.set(i - 1, uP);
       else {
-        atomicExch(err, 1);
-        ug[i - 1] = 0.0;
+        *err = 1;  // (every such cell writes the same)
+        ug.set(i - 1, 0.0);
       }
     } else if (kind == 3) {  // ideal-gas pressure: comp 2 = p', 3 = p
       if (pe == 3) {
-        ug[i - 1] = (comp == 2) ? 0.0 : sedge(m, 3, i, nel);
+        ug.set(i - 1, (comp == 2) ? 0.0 : sedge(m, 3, i, nel));
       } else {
-        const double gama = 2.0 * G.ca[i - 1];
-        ug[i - 1] = uP + gama * (go1 * G.n[0][i - 1] + go2 * G.n[1][i - 1]);
+        const double gama = 2.0 * C.face(kCa, i - 1);
+        ug.set(i - 1, uP + gama * (go1 * C.face(kN1, i - 1) + go2 * C.face(kN2, i - 1)));
       }
     } else {
       if (pe == 3) {
-        ug[i - 1] = 0.0;
+        ug.set(i - 1, 0.0);
       } else if (pe == 6) {
-        ug[i - 1] = uP;
+        ug.set(i - 1, uP);
       } else {
-        const double gama = 2.0 * G.ca[i - 1];
-        ug[i - 1] = uP + gama * (go1 * G.n[0][i - 1] + go2 * G.n[1][i - 1]);
+        const double gama = 2.0 * C.face(kCa, i - 1);
+        ug.set(i - 1, uP + gama * (go1 * C.face(kN1, i - 1) + go2 * C.face(kN2, i - 1)));
       }
     }
   }
   double g1, g2;
-  green_gauss(G, S.ns, ug, g1, g2);
+  green_gauss(C, ug, g1, g2);
   grad[2 * (size_t)(nel - 1)] = g1;
   grad[2 * (size_t)(nel - 1) + 1] = g2;
 }
@@ -379,14 +489,13 @@ struct MomArgs {
   double *ad, *au, *b, *im, *d, *rescell;
 };
 
-__global__ void momentum_kernel(Mesh m, MomArgs a) {
+template <bool kGeo>
+__global__ void __launch_bounds__(128) momentum_kernel(Mesh m, MomArgs a) {
   const int nel = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (nel > m.numel) return;
   const double ZERO = 1.0e-7, eps = 1.0e-14, cnst = 1.0e60;
-  Stencil S;
-  Geom G;
-  cell_setup(S, G, m, nel);
-  const int ns = S.ns, nsh = m.nshared, comp = a.comp;
+  const Cell<kGeo> C(m, nel);
+  const int ns = C.ns, nsh = m.nshared, comp = a.comp;
   const double viscosity = prop(m, nel, 1);
   const double rhoA = prop(m, nel, 2);
   const double cc = prop(m, nel, 6);
@@ -394,51 +503,50 @@ __global__ void momentum_kernel(Mesh m, MomArgs a) {
   const double *u = a.u, *u0 = a.u0, *w = a.w, *g_own = a.g_own, *g_oth = a.g_oth;
   const double *gradp = a.gradp;
   const double uP = u[nel - 1];
-  int ldl[MS + 1];
-  for (int i = 0; i <= MS; ++i) ldl[i] = 0;
-  for (int j = 1; j <= ns; ++j) ldl[j - 1] = (S.viz[j - 1] > 0) ? m.num[S.viz[j - 1] - 1] : 0;
-  ldl[nsh] = m.num[nel - 1];
-  double la[MS + 1];
-  for (int i = 0; i <= MS; ++i) la[i] = 0.0;
   const bool idg = a.idg != 0;
   const double *ro = a.ro;
   if (a.iws == 3) {
-    double mm = (idg ? ro3(ro, 2, nel) : prop(m, nel, 2)) * cc * G.area / a.dt;
+    double mm = (idg ? ro3(ro, 2, nel) : prop(m, nel, 2)) * cc * C.area() / a.dt;
     double p = mm * uP;
-    mm = (idg ? ro3(ro, 1, nel) : prop(m, nel, 2)) * cc * G.area / a.dt;
+    mm = (idg ? ro3(ro, 1, nel) : prop(m, nel, 2)) * cc * C.area() / a.dt;
     if (a.bs) p = 2 * p - 0.5 * mm * u0[nel - 1];
-    assbly(a.ad, a.au, a.b, a.ia, a.ja, la, p, ldl, nsh, a.matriz, true, false);
+    assbly(m, C, nel, a.ad, a.au, a.b, a.ia, a.ja, Four(), 0.0, p, a.matriz, false);
     return;
   }
   const double rhoP = idg ? ro3(ro, 3, nel) : rhoA;  // the cell's current density
   double p = 0.0, pf = 0.0, sp = 0.0, cd = 0.0, cvc = 0.0;
-  double aa[MS + 1];
+  Four aa;
+  const double w1P = v2(w, 1, nel), w2P = v2(w, 2, nel), pP = u0[nel - 1];
+  const double go1P = v2(g_own, 1, nel), go2P = v2(g_own, 2, nel);
+  const double gt1P = v2(g_oth, 1, nel), gt2P = v2(g_oth, 2, nel);
+  const double gp1P = v2(gradp, 1, nel), gp2P = v2(gradp, 2, nel);
+#pragma unroll 1
   for (int i = 1; i <= ns; ++i) {
-    const int v = S.viz[i - 1];
-    const double n1 = G.n[0][i - 1], n2 = G.n[1][i - 1];
-    const double meta = G.meta[i - 1];
+    const int v = C.neighbour(i - 1);
+    const double n1 = C.face(kN1, i - 1), n2 = C.face(kN2, i - 1);
+    const double nc = comp == 1 ? n1 : n2;
+    const double meta = C.face(kMeta, i - 1);
     if (v < 0) {
       const int pe = pedge(m, i, nel);
-      aa[i - 1] = 0.0;
       double ap = viscosity * meta;
       if (comp == 1)
-        p = p + ap * (v2(g_own, comp, nel) * n1 + v2(g_oth, comp, nel) * n2);
+        p = p + ap * (go1P * n1 + gt1P * n2);
       else
-        p = p + ap * (v2(g_own, comp, nel) * n2 + v2(g_oth, comp, nel) * n1);
-      if (idg) p = p - (2.0 / 3.0) * ap * a.div[nel - 1] * G.n[comp - 1][i - 1];
+        p = p + ap * (go2P * n2 + gt2P * n1);
+      if (idg) p = p - (2.0 / 3.0) * ap * a.div[nel - 1] * nc;
       double pface;
       if (pe == 3) {
         pface = sedge(m, 3, i, nel);
       } else {
-        pface = u0[nel - 1];
-        pface = pface + (v2(gradp, 1, nel) * G.df[0][i - 1] + v2(gradp, 2, nel) * G.df[1][i - 1]);
+        pface = pP;
+        pface = pface + (gp1P * C.face(kDf1, i - 1) + gp2P * C.face(kDf2, i - 1));
       }
-      pf = pf + pface * meta * G.n[comp - 1][i - 1];
+      pf = pf + pface * meta * nc;
       if (pe == 0) {
-        ap = viscosity * meta / G.ca[i - 1];
+        ap = viscosity * meta / C.face(kCa, i - 1);
         sp = sp + ap;
       } else if (pe == 1) {
-        ap = viscosity * meta / G.ca[i - 1];
+        ap = viscosity * meta / C.face(kCa, i - 1);
         sp = sp + ap;
         p = p + ap * sedge(m, comp, i, nel);
       } else if (pe == 2) {
@@ -446,7 +554,7 @@ __global__ void momentum_kernel(Mesh m, MomArgs a) {
         const double cv = rhoA * wfn * meta;
         p = p - cv * sedge(m, comp, i, nel);
       } else if (pe == 3) {
-        const double wfn = v2(w, 1, nel) * n1 + v2(w, 2, nel) * n2;
+        const double wfn = w1P * n1 + w2P * n2;
         if (fabs(wfn) > ZERO) {
           if (wfn > 0.0) {
             const double cv = rhoP * wfn * meta;
@@ -457,122 +565,119 @@ __global__ void momentum_kernel(Mesh m, MomArgs a) {
           }
         }
       } else if (pe == 4) {
-        const double wfn = v2(w, 1, nel) * n1 + v2(w, 2, nel) * n2;
+        const double wfn = w1P * n1 + w2P * n2;
         const double cv = rhoP * wfn * meta;
         sp = sp + cv;
       }
     } else {
-      double alpha = G.mksif[i - 1] / G.mksi[i - 1];
-      double kf = alpha / viscosity + (1.0 - alpha) / prop(m, v, 1);
+      const double alpha = C.face(kAlpha, i - 1), beta = 1.0 - alpha;
+      double kf = alpha / viscosity + beta / prop(m, v, 1);
       kf = 1.0 / kf;
-      const double wf1 = (1.0 - alpha) * v2(w, 1, nel) + alpha * v2(w, 1, v);
-      const double wf2 = (1.0 - alpha) * v2(w, 2, nel) + alpha * v2(w, 2, v);
-      double gf1 = (1.0 - alpha) * v2(g_own, 1, nel) + alpha * v2(g_own, 1, v);
-      double gf2 = (1.0 - alpha) * v2(g_own, 2, nel) + alpha * v2(g_own, 2, v);
-      const double k1 = G.ksi[0][i - 1], k2 = G.ksi[1][i - 1], mk = G.mksi[i - 1];
-      const double nk = n1 * k1 + n2 * k2;
+      const double wf1 = beta * w1P + alpha * v2(w, 1, v);
+      const double wf2 = beta * w2P + alpha * v2(w, 2, v);
+      const double go1V = v2(g_own, 1, v), go2V = v2(g_own, 2, v), uV = u[v - 1];
+      const double gl1 = beta * go1P + alpha * go1V, gl2 = beta * go2P + alpha * go2V;
+      double gf1 = gl1, gf2 = gl2;
+      const double k1 = C.face(kKsi1, i - 1), k2 = C.face(kKsi2, i - 1);
+      const double mk = C.face(kMksi, i - 1), nk = C.face(kNk, i - 1);
       const double wfn = wf1 * n1 + wf2 * n2;
       double gfk = gf1 * k1 + gf2 * k2;
-      gf1 = gf1 + ((u[v - 1] - uP) / mk - gfk) * k1;
-      gf2 = gf2 + ((u[v - 1] - uP) / mk - gfk) * k2;
+      const double dgk = (uV - uP) / mk - gfk;
+      gf1 = gf1 + dgk * k1;
+      gf2 = gf2 + dgk * k2;
       const double gfn = gf1 * n1 + gf2 * n2;
       gfk = gf1 * k1 + gf2 * k2;
-      const double dfd = (kf * meta) / (nk * mk);
+      const double dfd = (kf * meta) / C.face(kNkMksi, i - 1);
       cd = kf * meta * (gfn - gfk / nk);
-      aa[i - 1] = dfd;
       p = p + cd;
-      const double rof = idg ? (1.0 - alpha) * ro3(ro, 3, nel) + alpha * ro3(ro, 3, v) : rhoA;
+      const double rof = idg ? beta * rhoP + alpha * ro3(ro, 3, v) : rhoA;
       const double cv = rof * wfn * meta;
       if (cv < 0.0) {
-        const double du = uP - u[v - 1] + eps;
-        const double gpk = v2(g_own, 1, v) * (G.xc[0][MS] - G.xc[0][i - 1]) +
-                           v2(g_own, 2, v) * (G.xc[1][MS] - G.xc[1][i - 1]);
-        alpha = G.mksif[i - 1] / G.mksi[i - 1];
+        const double du = uP - uV + eps;
+        const double gpk = go1V * C.face(kDxc1, i - 1) + go2V * C.face(kDxc2, i - 1);
         const double r = 2.0 * gpk / du - 1.0;
-        cvc = (1.0 - alpha) * limit(r, icod) * du;
+        cvc = beta * limit(r, icod) * du;
       } else {
-        const double du = u[v - 1] - uP + eps;
-        const double gpk = (v2(g_own, 1, nel) * k1 + v2(g_own, 2, nel) * k2) * mk;
-        alpha = G.mksif[i - 1] / G.mksi[i - 1];
+        const double du = uV - uP + eps;
+        const double gpk = (go1P * k1 + go2P * k2) * mk;
         const double r = 2.0 * gpk / du - 1.0;
         cvc = alpha * limit(r, icod) * du;
       }
-      cvc = cvc + gf1 * G.km[0][i - 1] + gf2 * G.km[1][i - 1];
-      aa[i - 1] = aa[i - 1] + fmax(-cv, 0.0);
+      cvc = cvc + gf1 * C.face(kKm1, i - 1) + gf2 * C.face(kKm2, i - 1);
+      aa.set(i - 1, dfd + fmax(-cv, 0.0));
       sp = sp + cv;
       p = p - cv * cvc;
-      alpha = G.mksif[i - 1] / G.mksi[i - 1];
-      const double p1 = u0[nel - 1] + v2(gradp, 1, nel) * G.df[0][i - 1] +
-                        v2(gradp, 2, nel) * G.df[1][i - 1];
-      const double p2 = u0[v - 1] + v2(gradp, 1, v) * (G.xm[0][i - 1] - G.xc[0][i - 1]) +
-                        v2(gradp, 2, v) * (G.xm[1][i - 1] - G.xc[1][i - 1]);
+      const double p1 = pP + gp1P * C.face(kDf1, i - 1) + gp2P * C.face(kDf2, i - 1);
+      const double p2 = u0[v - 1] + v2(gradp, 1, v) * C.face(kDxm1, i - 1) +
+                        v2(gradp, 2, v) * C.face(kDxm2, i - 1);
       const double pface = 0.5 * (p1 + p2);
-      pf = pf + pface * meta * G.n[comp - 1][i - 1];
-      alpha = G.mksif[i - 1] / G.mksi[i - 1];
-      gf1 = (1.0 - alpha) * v2(g_own, comp, nel) + alpha * v2(g_own, comp, v);
-      gf2 = (1.0 - alpha) * v2(g_oth, comp, nel) + alpha * v2(g_oth, comp, v);
+      pf = pf + pface * meta * nc;
+      gf1 = comp == 1 ? gl1 : gl2;
+      gf2 = beta * (comp == 1 ? gt1P : gt2P) + alpha * v2(g_oth, comp, v);
       if (comp == 1)
         p = p + kf * meta * (gf1 * n1 + gf2 * n2);
       else
         p = p + kf * meta * (gf1 * n2 + gf2 * n1);
       if (idg) {  // -2/3 mu div(w) on the face
-        const double gdiv = (1.0 - alpha) * a.div[nel - 1] + alpha * a.div[v - 1];
-        p = p - (2.0 / 3.0) * kf * gdiv * meta * G.n[comp - 1][i - 1];
+        const double gdiv = beta * a.div[nel - 1] + alpha * a.div[v - 1];
+        p = p - (2.0 / 3.0) * kf * gdiv * meta * nc;
       }
     }
   }
   if (!idg && pedge(m, nsh + 1, nel) == -2) sp = sp + cnst;
   double aP = sp;
-  for (int i = 1; i <= ns; ++i) aP = aP + aa[i - 1];
-  double mm = rhoP * cc * G.area / a.dt;
+#pragma unroll
+  for (int i = 0; i < MS; ++i)
+    if (i < ns) aP = aP + aa.get(i);
+  const double area = C.area();
+  double mm = rhoP * cc * area / a.dt;
   if (a.bs) mm = 1.5 * mm;
   aP = aP + mm;
   aP = aP / a.under_u;
   p = p + (1 - a.under_u) * aP * uP;
   if (idg)  // buoyancy (rho - rho_ref) g A with rho_ref = e(2)
-    p = p + (ro3(ro, 3, nel) - rhoA) * a.grav[comp - 1] * G.area;
+    p = p + (ro3(ro, 3, nel) - rhoA) * a.grav[comp - 1] * area;
   double rm = 0.0, anb = 0.0;
-  for (int i = 1; i <= ns; ++i) {
-    rm = rm + aa[i - 1] * ((S.viz[i - 1] > 0) ? u[S.viz[i - 1] - 1] : 0.0);
-    anb = anb + aa[i - 1];
-  }
+#pragma unroll
+  for (int i = 0; i < MS; ++i)
+    if (i < ns) {
+      rm = rm + aa.get(i) * ((C.viz[i] > 0) ? u[C.viz[i] - 1] : 0.0);
+      anb = anb + aa.get(i);
+    }
   a.im[(comp - 1) + 4 * (size_t)(nel - 1)] = rm + p;
   a.im[(comp + 1) + 4 * (size_t)(nel - 1)] = aP;
   if (a.simple_c)
-    a.d[(comp - 1) + 2 * (size_t)(nel - 1)] = G.area / (aP - anb);
+    a.d[(comp - 1) + 2 * (size_t)(nel - 1)] = area / (aP - anb);
   else
-    a.d[(comp - 1) + 2 * (size_t)(nel - 1)] = G.area / aP;
+    a.d[(comp - 1) + 2 * (size_t)(nel - 1)] = area / aP;
   p = p - pf;
   rm = p + rm - aP * uP;
   a.rescell[nel - 1] = rm;
-  for (int i = 1; i <= ns; ++i) la[i - 1] = aa[i - 1];
-  la[nsh] = aP;
-  assbly(a.ad, a.au, a.b, a.ia, a.ja, la, p, ldl, nsh, a.matriz, true, true);
+  assbly(m, C, nel, a.ad, a.au, a.b, a.ia, a.ja, aa, aP, p, a.matriz, true);
 }
 
-__device__ double cell_vel(int intvel, const double *w, const double *grad, const double ddf[2],
-                           const Geom &G, const double *p, int nel, int v, int i, double alpha) {
-  const double n1 = G.n[0][i - 1], n2 = G.n[1][i - 1];
+template <bool kGeo>
+__device__ __forceinline__ double cell_vel(int intvel, const double *w, const double *grad,
+                                           const double ddf[2], const Cell<kGeo> &C,
+                                           const double *p, int nel, int v, int i, double alpha) {
+  const double n1 = C.face(kN1, i - 1), n2 = C.face(kN2, i - 1), meta = C.face(kMeta, i - 1);
   const double vm1 = (1 - alpha) * v2(w, 1, nel) + alpha * v2(w, 1, v);
   const double vm2 = (1 - alpha) * v2(w, 2, nel) + alpha * v2(w, 2, v);
   double wfn = vm1 * n1 + vm2 * n2;
-  if (intvel == 1) return wfn * G.meta[i - 1];
+  if (intvel == 1) return wfn * meta;
   const double gf1 = (1 - alpha) * v2(grad, 1, nel) + alpha * v2(grad, 1, v);
   const double gf2 = (1 - alpha) * v2(grad, 2, nel) + alpha * v2(grad, 2, v);
   if (intvel == 2) {
-    const double gfp1 = ((p[v - 1] - p[nel - 1]) / G.mksi[i - 1]);
-    const double gfp2 = gf1 * G.ksi[0][i - 1] + gf2 * G.ksi[1][i - 1];
+    const double gfp1 = ((p[v - 1] - p[nel - 1]) / C.face(kMksi, i - 1));
+    const double gfp2 = gf1 * C.face(kKsi1, i - 1) + gf2 * C.face(kKsi2, i - 1);
     wfn = wfn + 0.5 * (ddf[0] + ddf[1]) * (gfp2 - gfp1);
-    return wfn * G.meta[i - 1];
+    return wfn * meta;
   }
   const double gfp1 = p[v - 1] - p[nel - 1];
-  const double ks1 = G.mksi[i - 1] * G.ksi[0][i - 1];
-  const double ks2 = G.mksi[i - 1] * G.ksi[1][i - 1];
-  const double nk = ks1 * n1 + ks2 * n2;
-  double gfp2 = gf1 * ks1 + gf2 * ks2;
-  gfp2 = (gfp2 - gfp1) / nk;
+  double gfp2 = gf1 * C.face(kKs1, i - 1) + gf2 * C.face(kKs2, i - 1);
+  gfp2 = (gfp2 - gfp1) / C.face(kNks, i - 1);
   wfn = wfn + 0.5 * (ddf[0] + ddf[1]) * gfp2;
-  return wfn * G.meta[i - 1];
+  return wfn * meta;
 }
 
 struct PcArgs {
@@ -582,44 +687,38 @@ struct PcArgs {
   double *ad, *au, *b, *rescell;
 };
 
-__global__ void pc_kernel(Mesh m, PcArgs a) {
+template <bool kGeo>
+__global__ void __launch_bounds__(128) pc_kernel(Mesh m, PcArgs a) {
   const int nel = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (nel > m.numel) return;
   const double cnst = 1.0e60;
-  Stencil S;
-  Geom G;
-  cell_setup(S, G, m, nel);
-  const int ns = S.ns, nsh = m.nshared;
+  const Cell<kGeo> C(m, nel);
+  const int ns = C.ns, nsh = m.nshared;
   const double rhoA = prop(m, nel, 2);
   const double *w = a.w, *d = a.d;
-  int ldl[MS + 1];
-  for (int i = 0; i <= MS; ++i) ldl[i] = 0;
-  for (int j = 1; j <= ns; ++j) ldl[j - 1] = (S.viz[j - 1] > 0) ? m.num[S.viz[j - 1] - 1] : 0;
-  ldl[nsh] = m.num[nel - 1];
-  double la[MS + 1];
-  for (int i = 0; i <= MS; ++i) la[i] = 0.0;
+  Four la;
   double pp = 0.0, sp = 0.0, kf = 0.0;
+#pragma unroll 1
   for (int i = 1; i <= ns; ++i) {
-    const int v = S.viz[i - 1];
-    const double n1 = G.n[0][i - 1], n2 = G.n[1][i - 1];
+    const int v = C.neighbour(i - 1);
+    const double n1 = C.face(kN1, i - 1), n2 = C.face(kN2, i - 1);
     if (v < 0) {
       const int pe = pedge(m, i, nel);
-      la[i - 1] = 0.0;
       if (pe == 2 || pe == 4) {
         const double wfn = sedge(m, 1, i, nel) * n1 + sedge(m, 2, i, nel) * n2;
-        const double cv = rhoA * wfn * G.meta[i - 1];
+        const double cv = rhoA * wfn * C.face(kMeta, i - 1);
         pp = pp - cv;
       } else if (pe == 3) {
         const double dd1 = v2(d, 1, nel) * n1, dd2 = v2(d, 2, nel) * n2;
         const double ndd = dd1 * n1 + dd2 * n2;
-        const double dfd = (rhoA * ndd * G.meta[i - 1]) / G.ca[i - 1];
+        const double dfd = (rhoA * ndd * C.face(kMeta, i - 1)) / C.face(kCa, i - 1);
         sp = sp + dfd;
         const double wfn = v2(w, 1, nel) * n1 + v2(w, 2, nel) * n2;
-        const double cv = rhoA * wfn * G.meta[i - 1];
+        const double cv = rhoA * wfn * C.face(kMeta, i - 1);
         pp = pp - cv;
       }
     } else {
-      const double alpha = G.mksif[i - 1] / G.mksi[i - 1];
+      const double alpha = C.face(kAlpha, i - 1);
       double ddf[2], ndd;
       if (a.intvel == 5) {
         kf = (1.0 - alpha) * prop(m, nel, 2) + alpha * prop(m, v, 2);
@@ -633,17 +732,18 @@ __global__ void pc_kernel(Mesh m, PcArgs a) {
         const double dd1 = ddf[0] * n1, dd2 = ddf[1] * n2;
         ndd = dd1 * n1 + dd2 * n2;
       }
-      const double nk = n1 * G.ksi[0][i - 1] + n2 * G.ksi[1][i - 1];
-      la[i - 1] = (kf * G.meta[i - 1] * ndd) / (nk * G.mksi[i - 1]);
-      const double wfn = cell_vel(a.intvel, w, a.gradp, ddf, G, a.p, nel, v, i, alpha);
+      la.set(i - 1, (kf * C.face(kMeta, i - 1) * ndd) / C.face(kNkMksi, i - 1));
+      const double wfn = cell_vel(a.intvel, w, a.gradp, ddf, C, a.p, nel, v, i, alpha);
       pp = pp - kf * wfn;
     }
   }
   if (pedge(m, nsh + 1, nel) == -1) sp = sp + cnst;
-  la[nsh] = sp;
-  for (int i = 1; i <= ns; ++i) la[nsh] = la[nsh] + la[i - 1];
+  double diag = sp;
+#pragma unroll
+  for (int i = 0; i < MS; ++i)
+    if (i < ns) diag = diag + la.get(i);
   a.rescell[nel - 1] = pp;
-  assbly(a.ad, a.au, a.b, a.ia, a.ja, la, pp, ldl, nsh, a.matriz, true, true);
+  assbly(m, C, nel, a.ad, a.au, a.b, a.ia, a.ja, la, diag, pp, a.matriz, true);
 }
 
 __global__ void simple_update_kernel(int numel, double *w, double *pre, const double *u1,
@@ -679,57 +779,51 @@ struct PcIdgArgs {
   double *ad, *au, *b, *rescell;
 };
 
-__global__ void pc_idg_kernel(Mesh m, PcIdgArgs a) {
+template <bool kGeo>
+__global__ void __launch_bounds__(128) pc_idg_kernel(Mesh m, PcIdgArgs a) {
   const int nel = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (nel > m.numel) return;
   const double cnst = 1.0e60, ZERO = 1.0e-7;
-  Stencil S;
-  Geom G;
-  cell_setup(S, G, m, nel);
-  const int ns = S.ns, nsh = m.nshared;
+  const Cell<kGeo> C(m, nel);
+  const int ns = C.ns, nsh = m.nshared;
   const double *w = a.w, *d = a.d, *ro = a.ro;
   const double rhoP = ro3(ro, 3, nel), rhoA = prop(m, nel, 2);
-  int ldl[MS + 1];
-  for (int i = 0; i <= MS; ++i) ldl[i] = 0;
-  for (int j = 1; j <= ns; ++j) ldl[j - 1] = (S.viz[j - 1] > 0) ? m.num[S.viz[j - 1] - 1] : 0;
-  ldl[nsh] = m.num[nel - 1];
-  double la[MS + 1];
-  for (int i = 0; i <= MS; ++i) la[i] = 0.0;
+  Four la;
   double pp = 0.0, sp = 0.0, kf = 0.0;
+#pragma unroll 1
   for (int i = 1; i <= ns; ++i) {
-    const int v = S.viz[i - 1];
-    const double n1 = G.n[0][i - 1], n2 = G.n[1][i - 1];
+    const int v = C.neighbour(i - 1);
+    const double n1 = C.face(kN1, i - 1), n2 = C.face(kN2, i - 1);
     if (v < 0) {
       const int pe = pedge(m, i, nel);
-      la[i - 1] = 0.0;
       if (pe == 2) {
         const double wfn = sedge(m, 1, i, nel) * n1 + sedge(m, 2, i, nel) * n2;
-        const double cv = rhoA * wfn * G.meta[i - 1];
+        const double cv = rhoA * wfn * C.face(kMeta, i - 1);
         pp = pp - cv;
       } else if (pe == 3) {
         const double ddf1 = v2(d, 1, nel), ddf2 = v2(d, 2, nel);
         if (a.intvel == 2) {
           const double dd1 = ddf1 * n1, dd2 = ddf2 * n2;
           const double ndd = dd1 * n1 + dd2 * n2;
-          const double dfd = (rhoP * ndd * G.meta[i - 1]) / G.ca[i - 1];
+          const double dfd = (rhoP * ndd * C.face(kMeta, i - 1)) / C.face(kCa, i - 1);
           sp = sp + dfd;
         } else if (a.intvel == 5) {
           const double ndd = 0.5 * (ddf1 + ddf2);
-          const double dfd = (rhoP * G.meta[i - 1] * ndd) / G.ca[i - 1];
+          const double dfd = (rhoP * C.face(kMeta, i - 1) * ndd) / C.face(kCa, i - 1);
           sp = sp + dfd;
         }
         const double wfn = v2(w, 1, nel) * n1 + v2(w, 2, nel) * n2;
         double cv = 0.0;
         if (fabs(wfn) > ZERO) {
           if (wfn > 0.0)
-            cv = rhoP * wfn * G.meta[i - 1];
+            cv = rhoP * wfn * C.face(kMeta, i - 1);
           else if (wfn < 0.0)
-            cv = rhoA * wfn * G.meta[i - 1];
+            cv = rhoA * wfn * C.face(kMeta, i - 1);
         }
         pp = pp - cv;
       }
     } else {
-      const double alpha = G.mksif[i - 1] / G.mksi[i - 1];
+      const double alpha = C.face(kAlpha, i - 1);
       kf = (1.0 - alpha) * ro3(ro, 3, nel) + alpha * ro3(ro, 3, v);
       double ddf[2];
       ddf[0] = (1.0 - alpha) * v2(d, 1, nel) + alpha * v2(d, 1, v);
@@ -741,23 +835,24 @@ __global__ void pc_idg_kernel(Mesh m, PcIdgArgs a) {
         const double dd1 = ddf[0] * n1, dd2 = ddf[1] * n2;
         ndd = dd1 * n1 + dd2 * n2;
       }
-      const double nk = n1 * G.ksi[0][i - 1] + n2 * G.ksi[1][i - 1];
-      la[i - 1] = (kf * G.meta[i - 1] * ndd) / (nk * G.mksi[i - 1]);
-      const double wfn = cell_vel(a.intvel, w, a.gradp, ddf, G, a.p, nel, v, i, alpha);
+      la.set(i - 1, (kf * C.face(kMeta, i - 1) * ndd) / C.face(kNkMksi, i - 1));
+      const double wfn = cell_vel(a.intvel, w, a.gradp, ddf, C, a.p, nel, v, i, alpha);
       pp = pp - kf * wfn;
     }
   }
   if (pedge(m, nsh + 1, nel) == -1) sp = sp + cnst;
-  la[nsh] = sp;
-  for (int i = 1; i <= ns; ++i) la[nsh] = la[nsh] + la[i - 1];
+  double diag = sp;
+#pragma unroll
+  for (int i = 0; i < MS; ++i)
+    if (i < ns) diag = diag + la.get(i);
   double cvc;
   if (a.bs)
     cvc = (1.5 * ro3(ro, 3, nel) - 2.0 * ro3(ro, 2, nel) + 0.5 * ro3(ro, 1, nel));
   else
     cvc = (ro3(ro, 3, nel) - ro3(ro, 2, nel));
-  pp = pp - G.area * cvc / a.dt;
+  pp = pp - C.area() * cvc / a.dt;
   a.rescell[nel - 1] = fabs(pp);
-  assbly(a.ad, a.au, a.b, a.ia, a.ja, la, pp, ldl, nsh, a.matriz, true, true);
+  assbly(m, C, nel, a.ad, a.au, a.b, a.ia, a.ja, la, diag, pp, a.matriz, true);
 }
 
 // EnthalpyForTemp (IdealGas.f:20-50): to_temp: t = tRef + h/cP, else
@@ -814,22 +909,22 @@ __device__ __forceinline__ double esedge(const double *se, int nsh, int i, int c
   return se[(i - 1) + (size_t)(c - 1) * (nsh + 1)];
 }
 
-__global__ void energy_gradient_kernel(Mesh m, int lib, const int32_t *__restrict__ pe,
+template <bool kGeo>
+__global__ void __launch_bounds__(128) energy_gradient_kernel(Mesh m, int lib, const int32_t *__restrict__ pe,
                                        const double *__restrict__ se,
                                        const double *__restrict__ u, double *__restrict__ grad) {
   const int nel = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (nel > m.numel) return;
-  Stencil S;
-  Geom G;
-  cell_setup(S, G, m, nel);
+  const Cell<kGeo> C(m, nel);
   const double uP = u[nel - 1];
   const double go1 = v2(grad, 1, nel), go2 = v2(grad, 2, nel);
   const double cesp = prop(m, nel, 4), tref = prop(m, nel, 5);
-  double ug[MS];
-  for (int i = 1; i <= S.ns; ++i) {
-    const int v = S.viz[i - 1];
+  Four ug;
+#pragma unroll 1
+  for (int i = 1; i <= C.ns; ++i) {
+    const int v = C.neighbour(i - 1);
     if (v > 0) {
-      ug[i - 1] = u[v - 1];
+      ug.set(i - 1, u[v - 1]);
       continue;
     }
     const int pcode = epedge(pe, m.nshared, i, nel);
@@ -837,29 +932,28 @@ __global__ void energy_gradient_kernel(Mesh m, int lib, const int32_t *__restric
     if (lib == 3) {  // CellibTrans.f:131-144
       if (pcode == 2) {
         const int enthalpia = (int)(cesp * (sface - tref));
-        ug[i - 1] = (double)enthalpia;
+        ug.set(i - 1, (double)enthalpia);
       } else {
-        const double gama = 2.0 * G.ca[i - 1];
-        ug[i - 1] = uP + gama * (go1 * G.n[0][i - 1] + go2 * G.n[1][i - 1]);
+        const double gama = 2.0 * C.face(kCa, i - 1);
+        ug.set(i - 1, uP + gama * (go1 * C.face(kN1, i - 1) + go2 * C.face(kN2, i - 1)));
       }
     } else {  // CellibTrans.f:460-464
-      ug[i - 1] = (pcode == 2) ? 2.0 * sface - uP : uP;
+      ug.set(i - 1, (pcode == 2) ? 2.0 * sface - uP : uP);
     }
   }
   double g1, g2;
-  green_gauss(G, S.ns, ug, g1, g2);
+  green_gauss(C, ug, g1, g2);
   grad[2 * (size_t)(nel - 1)] = g1;
   grad[2 * (size_t)(nel - 1) + 1] = g2;
 }
 
-__global__ void energy_kernel(Mesh m, EnArgs a) {
+template <bool kGeo>
+__global__ void __launch_bounds__(128) energy_kernel(Mesh m, EnArgs a) {
   const int nel = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (nel > m.numel) return;
   const double ZERO = 1.0e-14, eps = 1.0e-14;
-  Stencil S;
-  Geom G;
-  cell_setup(S, G, m, nel);
-  const int ns = S.ns, nsh = m.nshared, lib = a.lib;
+  const Cell<kGeo> C(m, nel);
+  const int ns = C.ns, nsh = m.nshared, lib = a.lib;
   const double kc = prop(m, nel, 3);
   const double cesp = prop(m, nel, 4);
   const double tref = prop(m, nel, 5);
@@ -868,47 +962,41 @@ __global__ void energy_kernel(Mesh m, EnArgs a) {
   const int spec_mass = (int)prop(m, nel, 2);  // lib 4: an integer in the reference
   const double *u = a.u, *ro = a.ro, *w = a.w, *grad = a.grad;
   const double uP = u[nel - 1];
-  int ldl[MS + 1];
-  for (int i = 0; i <= MS; ++i) ldl[i] = 0;
-  for (int j = 1; j <= ns; ++j) ldl[j - 1] = (S.viz[j - 1] > 0) ? m.num[S.viz[j - 1] - 1] : 0;
-  ldl[nsh] = m.num[nel - 1];
-  double la[MS + 1];
-  for (int i = 0; i <= MS; ++i) la[i] = 0.0;
   if (a.iws == 4) {  // label 400: time term and volume source
-    double mm = ro3(ro, 2, nel) * cc * G.area / a.dt;
+    double mm = ro3(ro, 2, nel) * cc * C.area() / a.dt;
     double p = mm * uP;
     if (a.bs) {
-      mm = ro3(ro, 1, nel) * cc * G.area / a.dt;
+      mm = ro3(ro, 1, nel) * cc * C.area() / a.dt;
       p = 2 * p - 0.5 * mm * a.u0[nel - 1];
     }
-    if (epedge(a.pe, nsh, nsh + 1, nel) != 0) p = p + esedge(a.se, nsh, nsh + 1, nel) * G.area;
-    assbly(a.ad, a.au, a.b, a.ia, a.ja, la, p, ldl, nsh, a.matriz, true, false);
+    if (epedge(a.pe, nsh, nsh + 1, nel) != 0) p = p + esedge(a.se, nsh, nsh + 1, nel) * C.area();
+    assbly(m, C, nel, a.ad, a.au, a.b, a.ia, a.ja, Four(), 0.0, p, a.matriz, false);
     return;
   }
   const double roc = ro3(ro, 3, nel);
   double rof = roc;  // lib 4 carries it from face to face
   double p = 0.0, sp = 0.0, cd = 0.0, cvc = 0.0;
-  double aa[MS];
+  Four aa;
+#pragma unroll 1
   for (int i = 1; i <= ns; ++i) {
-    const int v = S.viz[i - 1];
-    const double n1 = G.n[0][i - 1], n2 = G.n[1][i - 1];
-    const double meta = G.meta[i - 1];
+    const int v = C.neighbour(i - 1);
+    const double n1 = C.face(kN1, i - 1), n2 = C.face(kN2, i - 1);
+    const double meta = C.face(kMeta, i - 1);
     if (v < 0) {
       const int pcode = epedge(a.pe, nsh, i, nel);
       const double sface = esedge(a.se, nsh, i, nel);
-      aa[i - 1] = 0.0;
       const double wfn = v2(w, 1, nel) * n1 + v2(w, 2, nel) * n2;
       double cv = (lib == 3 ? roc : rof) * wfn * meta;
       if (pcode == 0) {
         p = p + sface * meta;
       } else if (pcode == 1) {
         if (lib == 3) {
-          const double ap = (kc / cesp) * meta / G.ca[i - 1];
+          const double ap = (kc / cesp) * meta / C.face(kCa, i - 1);
           sp = sp + ap;
           const int enthalpia = (int)(cesp * (sface - tref));
           p = p + ap * enthalpia;
         } else {
-          const double ap = kc * meta / G.ca[i - 1];
+          const double ap = kc * meta / C.face(kCa, i - 1);
           sp = sp + ap;
           p = p + ap * sface;
         }
@@ -935,7 +1023,7 @@ __global__ void energy_kernel(Mesh m, EnArgs a) {
         sp = sp + cv;
       }
     } else {
-      double alpha = G.mksif[i - 1] / G.mksi[i - 1];
+      const double alpha = C.face(kAlpha, i - 1);
       double kf;
       if (lib == 3)
         kf = alpha / (kc / cesp) + (1.0 - alpha) / (prop(m, v, 3) / prop(m, v, 4));
@@ -946,8 +1034,8 @@ __global__ void energy_kernel(Mesh m, EnArgs a) {
       const double wf2 = (1.0 - alpha) * v2(w, 2, nel) + alpha * v2(w, 2, v);
       double gf1 = (1.0 - alpha) * v2(grad, 1, nel) + alpha * v2(grad, 1, v);
       double gf2 = (1.0 - alpha) * v2(grad, 2, nel) + alpha * v2(grad, 2, v);
-      const double k1 = G.ksi[0][i - 1], k2 = G.ksi[1][i - 1], mk = G.mksi[i - 1];
-      const double nk = n1 * k1 + n2 * k2;
+      const double k1 = C.face(kKsi1, i - 1), k2 = C.face(kKsi2, i - 1);
+      const double mk = C.face(kMksi, i - 1), nk = C.face(kNk, i - 1);
       const double wfn = wf1 * n1 + wf2 * n2;
       const double uv = u[v - 1];
       double gfk = gf1 * k1 + gf2 * k2;
@@ -955,9 +1043,8 @@ __global__ void energy_kernel(Mesh m, EnArgs a) {
       gf2 = gf2 + ((uv - uP) / mk - gfk) * k2;
       const double gfn = gf1 * n1 + gf2 * n2;
       gfk = gf1 * k1 + gf2 * k2;
-      const double dfd = (kf * meta) / (nk * mk);
+      const double dfd = (kf * meta) / C.face(kNkMksi, i - 1);
       cd = kf * meta * (gfn - gfk / nk);
-      aa[i - 1] = dfd;
       p = p + cd;
       if (lib == 3) {
         rof = (1.0 - alpha) * ro3(ro, 3, nel) + alpha * ro3(ro, 3, v);
@@ -972,36 +1059,35 @@ __global__ void energy_kernel(Mesh m, EnArgs a) {
       const double cv = rof * wfn * meta;
       if (cv < 0.0) {
         const double du = uP - uv + eps;
-        const double gpk = v2(grad, 1, v) * (G.xc[0][MS] - G.xc[0][i - 1]) +
-                           v2(grad, 2, v) * (G.xc[1][MS] - G.xc[1][i - 1]);
-        alpha = G.mksif[i - 1] / G.mksi[i - 1];
+        const double gpk = v2(grad, 1, v) * C.face(kDxc1, i - 1) +
+                           v2(grad, 2, v) * C.face(kDxc2, i - 1);
         const double r = 2.0 * gpk / du - 1.0;
         cvc = (1.0 - alpha) * limit(r, icod) * du;
       } else {
         const double du = uv - uP + eps;
         const double gpk = (v2(grad, 1, nel) * k1 + v2(grad, 2, nel) * k2) * mk;
-        alpha = G.mksif[i - 1] / G.mksi[i - 1];
         const double r = 2.0 * gpk / du - 1.0;
         cvc = alpha * limit(r, icod) * du;
       }
-      cvc = cvc + gf1 * G.km[0][i - 1] + gf2 * G.km[1][i - 1];
-      aa[i - 1] = aa[i - 1] + fmax(-cv, 0.0);
+      cvc = cvc + gf1 * C.face(kKm1, i - 1) + gf2 * C.face(kKm2, i - 1);
+      aa.set(i - 1, dfd + fmax(-cv, 0.0));
       sp = sp + cv;
       p = p - cv * cvc;
     }
   }
   double aP = sp;
-  for (int i = 1; i <= ns; ++i) aP = aP + aa[i - 1];
-  double mm = ro3(ro, 3, nel) * cc * G.area / a.dt;
+#pragma unroll
+  for (int i = 0; i < MS; ++i)
+    if (i < ns) aP = aP + aa.get(i);
+  double mm = ro3(ro, 3, nel) * cc * C.area() / a.dt;
   if (a.bs) mm = 1.5 * mm;
   aP = aP + mm;
   double rm = p - aP * uP;
-  for (int i = 1; i <= ns; ++i)
-    rm = rm + aa[i - 1] * ((S.viz[i - 1] > 0) ? u[S.viz[i - 1] - 1] : 0.0);
+#pragma unroll
+  for (int i = 0; i < MS; ++i)
+    if (i < ns) rm = rm + aa.get(i) * ((C.viz[i] > 0) ? u[C.viz[i] - 1] : 0.0);
   a.rescell[nel - 1] = rm;
-  for (int i = 1; i <= ns; ++i) la[i - 1] = aa[i - 1];
-  la[nsh] = aP;
-  assbly(a.ad, a.au, a.b, a.ia, a.ja, la, p, ldl, nsh, a.matriz, true, true);
+  assbly(m, C, nel, a.ad, a.au, a.b, a.ia, a.ja, aa, aP, p, a.matriz, true);
 }
 
 Mesh view(const fvc_cell_mesh *m) {
@@ -1016,7 +1102,7 @@ Mesh view(const fvc_cell_mesh *m) {
   v.pedge = m->pedge;
   v.sedge = m->sedge;
   v.e = m->e;
-  v.geo = static_cast<const Geom *>(m->geometry);
+  v.geo = static_cast<const double *>(m->geometry);
   return v;
 }
 
@@ -1041,7 +1127,10 @@ int32_t gradient_async(const fvc_cell_mesh *m, int kind, int comp, const double 
   if (!mesh_ok(m) || !u || !grad || !d_err || kind < 1 || kind > 3 || comp < 1 || comp > 3 ||
       (kind == 3 && comp == 1))
     return FVC_ERR_ARG;
-  gradient_kernel<<<grid(m->numel), kThreads, 0, s>>>(view(m), kind, comp, u, grad, d_err);
+  if (m->geometry)
+    gradient_kernel<true><<<grid(m->numel), kThreads, 0, s>>>(view(m), kind, comp, u, grad, d_err);
+  else
+    gradient_kernel<false><<<grid(m->numel), kThreads, 0, s>>>(view(m), kind, comp, u, grad, d_err);
   count_launch();
   return cudaPeekAtLastError() == cudaSuccess ? FVC_OK : FVC_ERR_CUDA;
 }
@@ -1054,7 +1143,10 @@ int32_t gradient(const fvc_cell_mesh *m, int kind, int comp, const double *u, do
   int *err = nullptr;
   if (cudaMallocAsync(&err, sizeof(int), s) != cudaSuccess) return FVC_ERR_CUDA;
   cudaMemsetAsync(err, 0, sizeof(int), s);
-  gradient_kernel<<<grid(m->numel), kThreads, 0, s>>>(view(m), kind, comp, u, grad, err);
+  if (m->geometry)
+    gradient_kernel<true><<<grid(m->numel), kThreads, 0, s>>>(view(m), kind, comp, u, grad, err);
+  else
+    gradient_kernel<false><<<grid(m->numel), kThreads, 0, s>>>(view(m), kind, comp, u, grad, err);
   count_launch();
   int herr = 0;
   cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s);
@@ -1116,7 +1208,10 @@ int32_t fvc_cells_momentum(const fvc_cell_mesh *m, int32_t comp, int32_t iws, co
   a.div = nullptr;
   a.grav[0] = a.grav[1] = 0.0;
   cudaStream_t s = (cudaStream_t)stream;
-  fvc::cells::momentum_kernel<<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
+  if (m->geometry)
+    fvc::cells::momentum_kernel<true><<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
+  else
+    fvc::cells::momentum_kernel<false><<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
   fvc::count_launch();
   return cudaPeekAtLastError() == cudaSuccess ? FVC_OK : FVC_ERR_CUDA;
 }
@@ -1164,7 +1259,10 @@ int32_t fvc_cells_momentum_ideal_gas(const fvc_cell_mesh *m, int32_t comp, int32
   a.d = d;
   a.rescell = rescell;
   cudaStream_t s = (cudaStream_t)stream;
-  fvc::cells::momentum_kernel<<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
+  if (m->geometry)
+    fvc::cells::momentum_kernel<true><<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
+  else
+    fvc::cells::momentum_kernel<false><<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
   fvc::count_launch();
   return cudaPeekAtLastError() == cudaSuccess ? FVC_OK : FVC_ERR_CUDA;
 }
@@ -1193,7 +1291,10 @@ int32_t fvc_cells_pressure_correction(const fvc_cell_mesh *m, const double *w, c
   a.b = b;
   a.rescell = rescell;
   cudaStream_t s = (cudaStream_t)stream;
-  fvc::cells::pc_kernel<<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
+  if (m->geometry)
+    fvc::cells::pc_kernel<true><<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
+  else
+    fvc::cells::pc_kernel<false><<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
   fvc::count_launch();
   return cudaPeekAtLastError() == cudaSuccess ? FVC_OK : FVC_ERR_CUDA;
 }
@@ -1226,7 +1327,10 @@ int32_t fvc_cells_pressure_correction_ideal_gas(const fvc_cell_mesh *m, const do
   a.b = b;
   a.rescell = rescell;
   cudaStream_t s = (cudaStream_t)stream;
-  fvc::cells::pc_idg_kernel<<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
+  if (m->geometry)
+    fvc::cells::pc_idg_kernel<true><<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
+  else
+    fvc::cells::pc_idg_kernel<false><<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
   fvc::count_launch();
   return cudaPeekAtLastError() == cudaSuccess ? FVC_OK : FVC_ERR_CUDA;
 }
@@ -1278,7 +1382,11 @@ int32_t fvc_cells_energy_gradient(const fvc_cell_mesh *m, int32_t lib, const int
   if (!fvc::cells::mesh_geom_ok(m) || (lib != 3 && lib != 4) || !pedge || !sedge || !u || !grad)
     return FVC_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  fvc::cells::energy_gradient_kernel<<<grid(m->numel), kThreads, 0, s>>>(
+  if (m->geometry)
+    fvc::cells::energy_gradient_kernel<true><<<grid(m->numel), kThreads, 0, s>>>(
+      fvc::cells::view(m), lib, pedge, sedge, u, grad);
+  else
+    fvc::cells::energy_gradient_kernel<false><<<grid(m->numel), kThreads, 0, s>>>(
       fvc::cells::view(m), lib, pedge, sedge, u, grad);
   fvc::count_launch();
   return cudaPeekAtLastError() == cudaSuccess ? FVC_OK : FVC_ERR_CUDA;
@@ -1315,7 +1423,10 @@ int32_t fvc_cells_energy(const fvc_cell_mesh *m, int32_t lib, int32_t iws, const
   a.b = b;
   a.rescell = rescell;
   cudaStream_t s = (cudaStream_t)stream;
-  fvc::cells::energy_kernel<<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
+  if (m->geometry)
+    fvc::cells::energy_kernel<true><<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
+  else
+    fvc::cells::energy_kernel<false><<<grid(m->numel), kThreads, 0, s>>>(fvc::cells::view(m), a);
   fvc::count_launch();
   return cudaPeekAtLastError() == cudaSuccess ? FVC_OK : FVC_ERR_CUDA;
 }
@@ -1335,8 +1446,8 @@ int32_t fvc_cells_geometry_create(const fvc_cell_mesh *m, void **geometry) {
       !m->ix || !m->nelcon)
     return FVC_ERR_ARG;
   *geometry = nullptr;
-  fvc::cells::Geom *g = nullptr;
-  if (cudaMalloc(&g, sizeof(fvc::cells::Geom) * (size_t)m->numel) != cudaSuccess)
+  double *g = nullptr;
+  if (cudaMalloc(&g, fvc::cells::geo_bytes(m->numel)) != cudaSuccess)
     return FVC_ERR_CUDA;
   fvc::cells::Mesh v = fvc::cells::view(m);
   v.geo = nullptr;

@@ -453,7 +453,7 @@ typedef struct {
 
 /* The geometry of every cell of m (centroids, face normals, lengths and
  * midpoints, ghost centroids, the reference's cellGeom2D / vectorKm2d
- * quantities) computed once into a DEVICE buffer (*geometry, 600 bytes per
+ * quantities) computed once into a DEVICE buffer (*geometry, 756 bytes per
  * cell), for fvc_cell_mesh.geometry.  It depends only on coor, ix and
  * nelcon, which must hold their values when it is called (it runs on the
  * default stream and waits for the device).  Free it with
