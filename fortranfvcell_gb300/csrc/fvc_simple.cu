@@ -26,6 +26,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 #include <cuda_runtime.h>
 
 #include "fvc_internal.h"
@@ -1135,14 +1136,49 @@ int32_t gradient_async(const fvc_cell_mesh *m, int kind, int comp, const double 
   return cudaPeekAtLastError() == cudaSuccess ? FVC_OK : FVC_ERR_CUDA;
 }
 
+// The error words of the gradient calls in flight (a call waits for its
+// kernel, so it needs one while it runs): static device words, all zero
+// between calls.  An allocation per call, whose memory the stream's pool gives
+// back at the call's synchronisation, cost 190 us, of which the kernel is 40
+// at 200k cells.  More calls at once than there are words allocate theirs.
+constexpr int kErrWords = 64;
+__device__ int g_err_words[kErrWords];
+std::mutex g_err_mutex;
+uint64_t g_err_used = 0;
+
+// One of the words, given back at the end of its scope
+struct ErrWord {
+  int index = -1;
+  ErrWord() {
+    std::lock_guard<std::mutex> lock(g_err_mutex);
+    for (int i = 0; i < kErrWords && index < 0; ++i)
+      if (!(g_err_used >> i & 1)) index = i;
+    if (index >= 0) g_err_used |= 1ull << index;
+  }
+  ~ErrWord() {
+    if (index < 0) return;
+    std::lock_guard<std::mutex> lock(g_err_mutex);
+    g_err_used &= ~(1ull << index);
+  }
+  ErrWord(const ErrWord &) = delete;
+  ErrWord &operator=(const ErrWord &) = delete;
+};
+
 int32_t gradient(const fvc_cell_mesh *m, int kind, int comp, const double *u, double *grad,
                  cudaStream_t s) {
   if (!mesh_ok(m) || !u || !grad || kind < 1 || kind > 3 || comp < 1 || comp > 3 ||
       (kind == 3 && comp == 1))
     return FVC_ERR_ARG;
+  const ErrWord word;
   int *err = nullptr;
-  if (cudaMallocAsync(&err, sizeof(int), s) != cudaSuccess) return FVC_ERR_CUDA;
-  cudaMemsetAsync(err, 0, sizeof(int), s);
+  if (word.index >= 0) {
+    if (cudaGetSymbolAddress(reinterpret_cast<void **>(&err), g_err_words) != cudaSuccess)
+      return FVC_ERR_CUDA;
+    err += word.index;
+  } else {
+    if (cudaMallocAsync(&err, sizeof(int), s) != cudaSuccess) return FVC_ERR_CUDA;
+    cudaMemsetAsync(err, 0, sizeof(int), s);
+  }
   if (m->geometry)
     gradient_kernel<true><<<grid(m->numel), kThreads, 0, s>>>(view(m), kind, comp, u, grad, err);
   else
@@ -1150,8 +1186,12 @@ int32_t gradient(const fvc_cell_mesh *m, int kind, int comp, const double *u, do
   count_launch();
   int herr = 0;
   cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s);
-  cudaFreeAsync(err, s);
+  if (word.index < 0) cudaFreeAsync(err, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return FVC_ERR_CUDA;
+  if (herr && word.index >= 0) {  // back to zero for the word's next call
+    cudaMemsetAsync(err, 0, sizeof(int), s);
+    if (cudaStreamSynchronize(s) != cudaSuccess) return FVC_ERR_CUDA;
+  }
   return herr ? FVC_ERR_UNSUPPORTED : FVC_OK;
 }
 
