@@ -84,7 +84,7 @@ struct __align__(16) RedSlot {
 struct GridSync {
   unsigned int *count;     // [0] arrivals of the sums and barriers; [8] (its
                            // own 32-byte sector) publications (exchange_totals)
-  unsigned long long *xw;  // words of the exact sums (exact_sum), whole grids only
+  unsigned long long *xw;  // words of the exact sums (exact_sum)
   int *err;                // sticky error (FVC_ERR_TIMEOUT on a stuck wait)
   RedSlot *slots;          // 4 sets x kMaxNV x nblocks
   unsigned int nblocks;    // blocks that synchronise through this state
@@ -772,13 +772,15 @@ static __device__ __noinline__ bool window_by_partials(const GridSync &gs, Episo
     for (int q = 0; q < nv; ++q) {
       int m = 0;
       for (int w = 0; w < nw; ++w) m = max(m, part[q * 32 + w]);
-      st_slot(slots + (size_t)q * gs.nblocks + blockIdx.x, (double)m, ep);
+      st_slot(slots + (size_t)q * gs.nblocks + (blockIdx.x - gs.base), (double)m, ep);
     }
-    // (one block counts no arrivals, see grid_barrier)
-    if (gs.nblocks > 1) red_add_release(gs.count, 1u);
+    // (one block and a cluster count no arrivals, see grid_barrier)
+    if (gs.nblocks > 1 && !gs.cluster) red_add_release(gs.count, 1u);
   }
+  if (gs.cluster) cooperative_groups::this_cluster().sync();
   if (warp == 0) {
-    const bool ok = gs.nblocks == 1 || wait_count<true>(gs.count, gs.err, ep * gs.nblocks);
+    const bool ok =
+        gs.nblocks == 1 || gs.cluster || wait_count<true>(gs.count, gs.err, ep * gs.nblocks);
     if (lane == 0) s_ok = ok ? 1 : 0;
   }
   __syncthreads();
@@ -849,6 +851,11 @@ __device__ __forceinline__ void exact_words(unsigned long long *xw, int *err, un
   const long long w = block_limbs(nv, part, xs);
   long long L = 0;
   bool ok = true, bad = false;
+  if (nb == 1) {  // its limbs are the total
+    L = (long long)((unsigned long long)w << 22) >> 22;
+    limb_totals(nv, L, w != L, true, xs);
+    return;
+  }
   // (the other lanes poll along on the first word, see wait_count)
   unsigned long long *word = xw + set * kXWords + (mine ? lane : 0);
   if (mine)  // bits 0-41 the limb, 42-52 blocks that overflowed, 53-63 blocks
@@ -932,8 +939,11 @@ __device__ __forceinline__ bool exact_sum(const GridSync &gs, Episode &episode, 
       if (lane == 0 && first) side();
       if (kJoin && first) join_warps01();
     } else if (kPublish && warp == 2 && first) {
-      if (lane == 0) red_add_release(gs.count + 8, 1u);
-      const bool ok = wait_count<true>(gs.count + 8, gs.err, episode.pub * gs.nblocks);
+      bool ok = true;  // (one block publishes by the __syncthreads)
+      if (gs.nblocks > 1) {
+        if (lane == 0) red_add_release(gs.count + 8, 1u);
+        ok = wait_count<true>(gs.count + 8, gs.err, episode.pub * gs.nblocks);
+      }
       if (lane == 0) xs.pub_ok = ok ? 1 : 0;
     }
     __syncthreads();

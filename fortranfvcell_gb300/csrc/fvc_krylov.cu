@@ -595,9 +595,9 @@ __global__ void __launch_bounds__(kMaxT, 1024 / kMaxT) krylov_batched(KArgs a, c
   ak.tol = d.tol;
   ak.init = d.init;
   if (d.code == 2)
-    bicgstab_run<kMaxT, false, true, false>(ak, P, d.gs, d.result, d.iresult, rank == 0);
+    bicgstab_run<kMaxT, false, true>(ak, P, d.gs, d.result, d.iresult, rank == 0);
   else
-    pcg_run<true, kMaxT, false>(ak, P, d.gs, d.result, d.iresult, rank == 0);
+    pcg_run<true, kMaxT>(ak, P, d.gs, d.result, d.iresult, rank == 0);
   cluster_close(d.gs);
 }
 
@@ -1250,7 +1250,9 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
     // device, else groups, where a large system can spread over more than
     // 16 blocks (the enthalpy systems of those SIMPLE cases in FP64: 256
     // cases 184 ms on clusters against 233 ms in groups; 64 cases 83
-    // against 52 ms)
+    // against 52 ms).  In FP64 twice over: 150 systems of 32^2 to 100^2 cells
+    // 11.4 ms on clusters, 10.0 in groups (mixed 10.0 and 11.1), 900 of 32^2
+    // to 64^2 17.6 and 19.7 (mixed 16.1 and 17.0)
     int most_rows = 0;
     for (int s = 0; s < nsys; ++s)
       most_rows = std::max(most_rows, row_start[s + 1] - row_start[s]);
@@ -1261,7 +1263,8 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
     int occ256 = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &occ256, mixed ? mixed_batched_kernel(256) : krylov_batched_kernel(256), 256, 0);
-    if (want < (long)std::max(occ256, 1) * sm_count()) adaptive = false;
+    const long fill = (long)std::max(occ256, 1) * sm_count();
+    if (want < (mixed ? fill : 2 * fill)) adaptive = false;
   }
   int csize = (o.cluster_size == 1)   ? 0
               : (o.cluster_size >= 2) ? o.cluster_size
@@ -1270,9 +1273,20 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
   // groups: 128-thread blocks by default, twice the co-resident blocks of
   // 256, so the one-block minimum of the small systems takes a smaller share
   // (the u, v, T and p' systems of 256 heated cavities, 1024 systems: 184 ms
-  // at 128 threads, 215 at 256, 386 at 512); clusters: 256
+  // at 128 threads, 215 at 256, 386 at 512); clusters: 256.  Few systems
+  // (kSparse blocks or more each) leave half of the thread slots empty: eight
+  // blocks of 128 threads on an SM delay one another's sums by more than the
+  // rows they share save, 48 systems of 24^2 to 140^2 cells, mixed, 13.4 ms
+  // at eight a SM, 9.5 at four, 48 triangle meshes of 12^2 to 60^2 in FP64 5.9
+  // and 5.15 (but 150 systems 9.95 and 11.7); and with kSparse blocks of 256
+  // threads each those serve better, two to an SM: 20 systems of up to 100^2,
+  // mixed, 8.3 ms against 8.8 of four of 128, 12 of up to 140^2 16.7 and 18.3
+  constexpr int kSparse = 8;
+  const bool few = nsys * kSparse <= 4 * sm_count();
   auto threads_for = [&](int cs) {
-    return (o.block_threads > 0) ? block_threads_for(o.block_threads, 0, 1) : cs > 0 ? 256 : 128;
+    return (o.block_threads > 0)                               ? block_threads_for(o.block_threads, 0, 1)
+           : cs > 0 || nsys * kSparse <= 2 * sm_count() ? 256
+                                                               : 128;
   };
   int threads = threads_for(csize);
   if (mixed) {
@@ -1316,6 +1330,7 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, 0);
     if (occ <= 0) occ = 1;
     if (o.blocks_per_sm > 0 && o.blocks_per_sm < occ) occ = o.blocks_per_sm;
+    else if (few && o.blocks_per_sm <= 0 && o.block_threads <= 0) occ = std::min(occ, 512 / threads);
     cap = occ * sm_count();
     if (o.max_blocks > 0) cap = std::min(cap, o.max_blocks);
     if (nsys > cap) {
@@ -1327,7 +1342,10 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
   // blocks per system in proportion to its work: slices x the expected
   // iterations (the caller's hint, else sqrt(rows), the growth of the
   // iteration count with the mesh size) x the SpMVs per iteration (2 for
-  // BiCGSTAB); at most one slice per warp.  Water-filling: a system whose share is
+  // BiCGSTAB; without a hint 1/2: a transport system takes some 50 iterations
+  // where a pressure system takes 9 sqrt(rows), and its blocks idle when it is
+  // done.  24 systems of each kind, 24^2 to 140^2 cells: FP64 13.1 -> 8.9 ms);
+  // at most one slice per warp.  Water-filling: a system whose share is
   // below one block gets one, the others share the rest, and blocks left
   // over by rounding go to the largest remainders.
   const int warps = threads / 32;
@@ -1339,8 +1357,9 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
     const int rows = row_start[s + 1] - row_start[s];
     slices[s] = (rows + 31) / 32;
     most[s] = (slices[s] + warps - 1) / warps;
-    const double its = (its_hint && its_hint[s] > 0.0) ? its_hint[s] : std::sqrt((double)rows);
-    wt[s] = slices[s] * its * ((codes && codes[s] == 2) ? 2.0 : 1.0);
+    const bool hinted = its_hint && its_hint[s] > 0.0;
+    const double its = hinted ? its_hint[s] : std::sqrt((double)rows);
+    wt[s] = slices[s] * its * ((codes && codes[s] == 2) ? (hinted ? 2.0 : 0.5) : 1.0);
     wleft += wt[s];
   }
   // clusters: csize blocks each (adaptive: each system's own size), one
@@ -1418,10 +1437,12 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
     --total;
   }
   // one device buffer: per system a 64-byte counter sector, the error word,
-  // the reduction slots (groups: clusters have none); then results,
-  // descriptors and the block map.  ctr_bytes: what every launch zeroes of it
-  const size_t part_off = (size_t)nsys * 64 + 64;
-  const size_t ctr_bytes = part_off + (csize > 0 ? 0 : slot_bytes((size_t)total));
+  // per system the words of its exact sums, the reduction slots; then
+  // results, descriptors and the block map.  ctr_bytes: what every launch
+  // zeroes of it
+  const size_t xw_off = ((size_t)nsys * 64 + 64 + 511) / 512 * 512;
+  const size_t part_off = xw_off + (size_t)nsys * kXBytes;
+  const size_t ctr_bytes = part_off + slot_bytes((size_t)total);
   const size_t res_bytes = (size_t)nsys * 16 * sizeof(double);
   const size_t ires_bytes = (size_t)nsys * 16 * sizeof(int);
   const size_t sys_bytes = (size_t)nsys * sizeof(BatchSys);
@@ -1456,8 +1477,8 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
     d.inner_tol = (o.inner_tol > 0) ? o.inner_tol : kInnerTolDefault;
     d.gs.count = ctr + (size_t)s * 16;
     d.gs.err = err;
-    d.gs.slots = csize > 0 ? nullptr : part + poff;
-    d.gs.xw = nullptr;
+    d.gs.slots = part + poff;
+    d.gs.xw = reinterpret_cast<unsigned long long *>(buf + xw_off + (size_t)s * kXBytes);
     d.gs.nblocks = (unsigned int)nb[s];
     // a cluster launch numbers its blocks from 0: the base within the segment
     d.gs.base = (unsigned int)(csize > 0 ? b0 - seg_off[seg] : b0);

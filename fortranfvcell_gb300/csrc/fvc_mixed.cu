@@ -1085,7 +1085,7 @@ __device__ __forceinline__ bool f32_refused(const MArgs &a) {
   return true;
 }
 
-template <bool kStaged, int kW>
+template <bool kStaged, int kW, bool kX>
 __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
   __shared__ double red[kMaxNV * 32];
   extern __shared__ __align__(128) unsigned char st_smem[];
@@ -1114,6 +1114,13 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
   } sh;
   __shared__ float2 red2[kMaxNV * 32];
   __shared__ double tot[2 * kTotCap];
+  __shared__ ExactState xs;
+  __shared__ SumWindow<1> wpq;
+  __shared__ SumWindow<2> wrz;
+  if (kX) {
+    exact_init(xs);
+    if (threadIdx.x == 0) wpq.top[0] = wrz.top[0] = kNoWindow;
+  }
   enum { kContinue = 0, kUpdate = 1, kStop = 2 };
   const NoScalars none;
   Episode ep;
@@ -1176,7 +1183,7 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
       if (mlead(a) && a.history && it > 1 && it - 1 <= kHistoryMax)
         a.history[it - 2] = (float)root(divide(sh.rr, sh.scale));
     };
-    if (!grid_allreduce_ff<1, false>(a.gs, ep, pq, red2, tot, before_pq, none, [&](const double *t) {
+    if (!grid_sum_ffx<1, false, kX>(a.gs, ep, xs, wpq, pq, red2, tot, before_pq, none, [&](const double *t) {
           const double alpha_d = divide(sh.rz, t[0]);
           sh.alpha = alpha_d;
           sh.alpha_f = (float)alpha_d;
@@ -1208,7 +1215,7 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
       prefetch_a<kW>(a, P, st_smem, gch);
       a_pre = true;
     }
-    if (!grid_allreduce_ff<2, true>(a.gs, ep, acc, red2, tot, none, none, [&](const double *t) {
+    if (!grid_sum_ffx<2, true, kX>(a.gs, ep, xs, wrz, acc, red2, tot, none, none, [&](const double *t) {
           // the alpha*p of an iteration that did not update e is added later
           if (!was_pending) sh.pend_alpha = sh.alpha;
           const double rz_new = t[0];
@@ -1292,18 +1299,18 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
   }
 }
 
-__global__ void __launch_bounds__(1024, 1) mixed_cg(MArgs a) { mixed_cg_body<false, 0>(a); }
+__global__ void __launch_bounds__(1024, 1) mixed_cg(MArgs a) { mixed_cg_body<false, 0, false>(a); }
 
 // Staged forms: 1024 threads, kStSmem bytes of dynamic shared memory, and
 // the 16-bit column offsets (col16) present; _w3/_w4 when every slice has
 // width 3 / 4 in the padded uniform layout (ell_w; cells of triangle /
 // quadrilateral meshes).
-__global__ void __launch_bounds__(1024, 1) mixed_cg_staged(MArgs a) { mixed_cg_body<true, 0>(a); }
+__global__ void __launch_bounds__(1024, 1) mixed_cg_staged(MArgs a) { mixed_cg_body<true, 0, false>(a); }
 __global__ void __launch_bounds__(1024, 1) mixed_cg_staged_w3(MArgs a) {
-  mixed_cg_body<true, 3>(a);
+  mixed_cg_body<true, 3, false>(a);
 }
 __global__ void __launch_bounds__(1024, 1) mixed_cg_staged_w4(MArgs a) {
-  mixed_cg_body<true, 4>(a);
+  mixed_cg_body<true, 4, false>(a);
 }
 
 // The reference's Jacobi BiCGSTAB (Iterativos.f:140-234) in FP32 on the
@@ -1311,7 +1318,6 @@ __global__ void __launch_bounds__(1024, 1) mixed_cg_staged_w4(MArgs a) {
 constexpr int kBcgStall = 100;
 constexpr int kSweepStall = 3;
 
-template <bool kX>
 __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
   __shared__ double red[kMaxNV * 32];
   __shared__ float2 red2[kMaxNV * 32];
@@ -1403,7 +1409,7 @@ __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
       });
       // breakdown (v.r0 or r0.s vanished in FP32): leave the correction as it
       // is and restart from an FP64 residual in the next sweep
-      if (!grid_sum_ffx<2, false, kX>(a.gs, ep, xs, w1, c01, red2, tot, none, none, [&](const double *q) {
+      if (!grid_sum_ffx<2, false, true>(a.gs, ep, xs, w1, c01, red2, tot, none, none, [&](const double *q) {
             bs.rr0 = q[0];
             bs.alpha = (float)divide(q[0], q[1]);
             bs.go = (isfinite(bs.alpha) && bs.alpha != 0.0f) ? 1 : 0;
@@ -1450,7 +1456,7 @@ __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
             c23[1].add(ti[u] * ti[u]);
           }
       });
-      if (!grid_sum_ffx<2, false, kX>(a.gs, ep, xs, w2, c23, red2, tot, [&] { bs.rv.set(bs.rr0); },
+      if (!grid_sum_ffx<2, false, true>(a.gs, ep, xs, w2, c23, red2, tot, [&] { bs.rv.set(bs.rr0); },
                                   none, [&](const double *q) {
             bs.omega = (q[1] > 0.0) ? (float)divide(q[0], q[1]) : 0.0f;
             bs.go = isfinite(bs.omega) ? 1 : 0;
@@ -1485,7 +1491,7 @@ __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
       // BiCGSTAB: an inner solve whose residual has not improved for
       // kBcgStall iterations (FP32 stagnation) restarts from an FP64 one
       auto before45 = [&] { bs.aw = divide((double)bs.alpha, (double)bs.omega); };
-      if (!grid_sum_ffx<2, false, kX>(a.gs, ep, xs, w3, c45, red2, tot, none, before45, [&](const double *q) {
+      if (!grid_sum_ffx<2, false, true>(a.gs, ep, xs, w3, c45, red2, tot, none, before45, [&](const double *q) {
             const double sz = fabs(q[0]);
             int go = 1;
             if (!(q[0] == q[0]) || sz <= stop2 || inner_total + it >= a.maxit ||
@@ -1526,7 +1532,7 @@ __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
 }
 
 __global__ void __launch_bounds__(1024, 1) mixed_bicgstab(MArgs a) {
-  mixed_bicgstab_body<true>(a);
+  mixed_bicgstab_body(a);
 }
 
 // Batched mixed-precision solves: every block runs the mixed CG (code 1)
@@ -1554,9 +1560,9 @@ __global__ void __launch_bounds__(kMaxT, 1024 / kMaxT)
   am.history = nullptr;
   if (d.code == 2) {
     am.rsl = nullptr;
-    mixed_bicgstab_body<false>(am);
+    mixed_bicgstab_body(am);
   } else {
-    mixed_cg_body<false, 0>(am);
+    mixed_cg_body<false, 0, true>(am);
   }
   cluster_close(d.gs);
 }

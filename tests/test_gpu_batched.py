@@ -183,3 +183,39 @@ def test_batched_mixed_precision_reaches_tolerance(orc):
     for s, r in zip(systems, pk["rows"]):
         xm, x64 = xs["mixed"][r], xs["fp64"][r]
         assert np.linalg.norm(xm - x64) <= 1e-4 * np.linalg.norm(x64), s["n"]
+
+
+@pytest.mark.parametrize("nsys", [10, 60, 90])
+def test_batched_group_shapes(orc, nsys):
+    """Few, some and many systems (256-thread blocks two to an SM, 128-thread
+    blocks four and eight to an SM), the right-hand sides of the PCG systems
+    many orders apart: each system's sums keep to its own scale.  Bars as
+    above."""
+    base = batch(orc)
+    codes = [2 if k % 2 else 1 for k in range(nsys)]
+    scale = [1.0 if k % 2 else 10.0 ** (40 * (k % 5 - 2)) for k in range(nsys)]
+    refs, systems = {}, []
+    for k in range(nsys):
+        i = k % len(base)
+        s = dict(base[i])
+        if codes[k] == 2:
+            u = unsymmetric(s, seed=i)
+            s.update(ad=u["ad"], au=u["au"])
+        if i not in refs:
+            x = np.zeros(s["n"])
+            status, so = orc.solver(s["ad"].copy(), s["au"].copy(), s["au"].copy(), x,
+                                    s["b"].copy(), s["ia"], s["ja"], s["n"], s["nad"], True,
+                                    1e-10 if codes[k] == 1 else 1e-11, 20000, codes[k], 1)
+            assert status == 0
+            refs[i] = x, so
+        s["b"] = s["b"] * scale[k]
+        systems.append(s)
+    rc, st, xs = solve_batch(systems, 0.0, 20000, codes=codes,
+                             tols=[1e-10 if c == 1 else 1e-11 for c in codes])
+    assert rc == 0
+    for k in range(nsys):
+        want, so = refs[k % len(base)]
+        err = np.linalg.norm(xs[k] / scale[k] - want) / np.linalg.norm(want)
+        assert err <= (REL_TOL if codes[k] == 1 else 1e-9), (k, err)
+        if codes[k] == 1:
+            assert abs(st[k].iterations - so.iterations) <= ITS_TOL, k
