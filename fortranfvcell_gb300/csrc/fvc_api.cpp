@@ -1027,6 +1027,8 @@ void context_free_batched(fvc_context *c, BatchPlan &P) {
 
 int context_default_init(int code, int matriz) { return default_init(code, matriz); }
 
+void context_order_sums(fvc_context *c) { c->S.ordered = true; }
+
 int32_t context_prepare(fvc_context *c, int code, const fvc_opts &o) {
   if (!c || !c->has_matrix) return FVC_ERR_ARG;
   cudaSetDevice(c->device);

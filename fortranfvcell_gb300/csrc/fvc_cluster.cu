@@ -70,16 +70,55 @@ extern __shared__ __align__(16) unsigned char cl_smem[];
 struct ClSum {
   ExactState xs;
   long long post[2][32];
-  int part[3 * kLimbs * 32];
+  alignas(8) int part[3 * kLimbs * 32];
 };
+
+// The same sum added in FP64 in a fixed order (Scratch::ordered): a shuffle
+// tree per warp, one over the warps, one over the CTAs.
+template <int NV, typename O, typename S, typename F>
+__device__ __forceinline__ void cluster_sum_ordered(cg::cluster_group &cl, unsigned int &ep,
+                                                    ClSum &cs, const double (&v)[NV], O &&overlap,
+                                                    S &&side, F &&f) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const unsigned int set = ep++ & 1u;
+  double *part = reinterpret_cast<double *>(cs.part);
+  double *post = reinterpret_cast<double *>(cs.post[set]);
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    const double t = warp_sum(v[q]);
+    if (lane == 0) part[q * 32 + warp] = t;
+  }
+  __syncthreads();
+  if (warp == 0)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      const double t = warp_sum(lane < nw ? part[q * 32 + lane] : 0.0);
+      if (lane == 0) post[q] = t;
+    }
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  overlap();
+  if (threadIdx.x == 32) side();
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  if (warp == 0) {
+    const int nb = (int)cl.num_blocks();
+    double t[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+      t[q] = warp_sum(lane < nb ? *cl.map_shared_rank(post + q, lane) : 0.0);
+    if (lane == 0) f(t);
+  }
+  __syncthreads();
+}
 
 // The exact sum (see exact_sum) over a cluster.  overlap() runs in every
 // thread, side() in thread 32, between the arrival at the cluster barrier and
 // its wait; f(totals) in thread 0.
-template <int NV, typename O, typename S, typename F>
+template <bool kOrdered, int NV, typename O, typename S, typename F>
 __device__ __forceinline__ void cluster_sum(cg::cluster_group &cl, unsigned int &ep, ClSum &cs,
                                             SumWindow<NV> &win, const double (&v)[NV],
                                             O &&overlap, S &&side, F &&f) {
+  if (kOrdered) return cluster_sum_ordered<NV>(cl, ep, cs, v, overlap, side, f);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int nb = (int)cl.num_blocks();
   ExactState &xs = cs.xs;
@@ -157,6 +196,7 @@ __device__ __forceinline__ void cluster_sum(cg::cluster_group &cl, unsigned int 
   }
 }
 
+template <bool kOrdered>
 __global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
   cg::cluster_group cl = cg::this_cluster();
   __shared__ ClSum cs;
@@ -256,11 +296,11 @@ __global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
 #ifdef FVC_CHECK
   double acc[3] = {r * z, bi * bi, (threadIdx.x == 0 && s_bad != 0) ? 1.0 : 0.0};
   __syncthreads();
-  cluster_sum<3>(cl, ep, cs, w3, acc, none, none, [&](const double *t) {
+  cluster_sum<kOrdered, 3>(cl, ep, cs, w3, acc, none, none, [&](const double *t) {
     sh.stop = (t[2] > 0.0) ? 3 : 0;
 #else
   double acc[2] = {r * z, bi * bi};
-  cluster_sum<2>(cl, ep, cs, wrr, acc, none, none, [&](const double *t) {
+  cluster_sum<kOrdered, 2>(cl, ep, cs, wrr, acc, none, none, [&](const double *t) {
     sh.stop = 0;
 #endif
     sh.d = t[0];
@@ -282,8 +322,10 @@ __global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
     cl.sync();
     const double qi = own ? spmv_row(pi, 0) : 0.0;
     const double pq[1] = {pi * qi};
-    cluster_sum<1>(cl, ep, cs, wpq, pq, none, [&] { sh.dv.set(sh.d); },
-                   [&](const double *t) { sh.alpha = quick_quotient(sh.d, t[0]); });
+    cluster_sum<kOrdered, 1>(cl, ep, cs, wpq, pq, none, [&] { sh.dv.set(sh.d); },
+                   [&](const double *t) {
+                     sh.alpha = kOrdered ? divide(sh.d, t[0]) : quick_quotient(sh.d, t[0]);
+                   });
     const double alpha = sh.alpha;
     r = fma(-alpha, qi, r);
     z = r * mi;
@@ -299,10 +341,10 @@ __global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
     auto update_x = [&] { x = fma(alpha, pi, x); };
     if (rule0) {
       const double rz[1] = {r * z};
-      cluster_sum<1>(cl, ep, cs, wrz, rz, update_x, none, step);
+      cluster_sum<kOrdered, 1>(cl, ep, cs, wrz, rz, update_x, none, step);
     } else {
       const double rr[2] = {r * z, r * r};
-      cluster_sum<2>(cl, ep, cs, wrr, rr, update_x, none, step);
+      cluster_sum<kOrdered, 2>(cl, ep, cs, wrr, rr, update_x, none, step);
     }
     if (sh.stop == 2) {
       status = FVC_ERR_NAN;
@@ -328,7 +370,7 @@ __global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
     e3[2] = bi * bi;
     a.x[r0 + i] = x;
   }
-  cluster_sum<3>(cl, ep, cs, w3, e3, none, none, [&](const double *t) {
+  cluster_sum<kOrdered, 3>(cl, ep, cs, w3, e3, none, none, [&](const double *t) {
     if (rank == 0) {
       a.result[0] = t[0];
       a.result[1] = sh.conv;
@@ -394,10 +436,13 @@ int32_t enqueue_pcg_cluster(const DeviceMatrix &A, Scratch &S, const double *b, 
   const ClLayout L{R, smax};
   const size_t smem = L.bytes();
   if (smem > 200 * 1024) return FVC_ERR_UNSUPPORTED;
+  auto *kern = S.ordered ? pcg_cluster<true> : pcg_cluster<false>;
   static bool attrs_set = false;
   if (!attrs_set) {
-    cudaFuncSetAttribute(pcg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(pcg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (auto *k : {pcg_cluster<false>, pcg_cluster<true>}) {
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
     attrs_set = true;
   }
   const int threads = std::min(1024, std::max(128, (R + 127) / 128 * 128));
@@ -415,7 +460,7 @@ int32_t enqueue_pcg_cluster(const DeviceMatrix &A, Scratch &S, const double *b, 
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, pcg_cluster, &cfg) != cudaSuccess ||
+  if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess ||
       clusters < 1) {
     cudaGetLastError();
     return FVC_ERR_UNSUPPORTED;
@@ -434,7 +479,7 @@ int32_t enqueue_pcg_cluster(const DeviceMatrix &A, Scratch &S, const double *b, 
   a.stop_rule = o.stop_rule;
   a.result = S.result;
   a.iresult = S.iresult;
-  const cudaError_t ce = cudaLaunchKernelEx(&cfg, pcg_cluster, a);
+  const cudaError_t ce = cudaLaunchKernelEx(&cfg, kern, a);
   count_launch();
   if (ce != cudaSuccess) {
     fprintf(stderr, "fvcgpu: cluster PCG launch failed: %s\n", cudaGetErrorString(ce));

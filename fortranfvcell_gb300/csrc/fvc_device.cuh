@@ -326,8 +326,8 @@ __device__ __forceinline__ bool grid_allreduce(const GridSync &gs, Episode &epis
   return true;
 }
 
-// The exchange of the grid-wide sums of the solvers (grid_sum_d and
-// grid_allreduce_ff).  Thread 0 puts its block's partial of each quantity
+// The exchange of the grid-wide sums of the mixed-precision CG
+// (grid_allreduce_ff) and of grid_allreduce.  Thread 0 puts its block's partial of each quantity
 // into its slots and counts itself in; every block then waits for all and
 // sums all partials itself in a fixed order, so that every block holds
 // identical totals.
@@ -398,21 +398,6 @@ __device__ __forceinline__ bool exchange_totals(const GridSync &gs, Episode &epi
   __shared__ double s_t[NV];
   if (kPublish) ++episode.pub;
   const unsigned int ep = ++episode.n;
-  if (gs.cluster) {
-    __shared__ double s_slot[2][kMaxNV];
-    if (threadIdx.x == 0) {
-#pragma unroll
-      for (int q = 0; q < NV; ++q) s_slot[ep & 1u][q] = bsum[q];
-    }
-    if (threadIdx.x == 32) side();
-    __syncwarp();
-    cluster_sync_mid(mid);
-    double t[NV];
-    cluster_exchange<NV>(s_slot, ep, t);
-    if (threadIdx.x == 0) f(t);
-    __syncthreads();
-    return true;
-  }
   if (gs.nblocks == 1) {  // one block: its sum is the total (same value)
     if (threadIdx.x == 0) {
       mid();
@@ -474,27 +459,22 @@ __device__ __forceinline__ bool exchange_totals(const GridSync &gs, Episode &epi
   return true;
 }
 
-// Grid-wide deterministic sum of NV FP64 values per thread, for the FP64
-// solvers.  GB300 issues one FP64 warp instruction per 76 clocks and SM
-// sub-partition, whatever the active lanes, with 64 clocks of latency, so
-// the chain of dependent additions is what a sum costs.  The values go to
-// shared memory (buf: NV x blockDim doubles); four warps (one per
-// sub-partition) add blockDim / 128 values per lane in two chains and
-// finish with a shuffle tree; lane 0 of warp 0 adds the four (a fixed
-// order; blockDim.x must be a multiple of 128; 10 dependent additions for
-// 1024 threads).  The blocks' partials travel through grid_arrive /
-// grid_collect (or the cluster).  Lane 0 of warp 0 then calls f(totals) --
-// the place for the iteration's scalar FP64 work (one thread instead of
-// 1024) -- and one __syncthreads hands its results (through shared memory)
-// to the block.  Scalar work that needs nothing of this sum (a division is
-// 570 clocks) hides in the wait: thread 0 calls mid() between its arrival
-// and its wait, for values f uses; thread 32 calls side(), for values of
-// later phases.  Returns false when a wait exceeded its bound (gs.err set).
-template <int NV, bool kPublish, typename S, typename M, typename F>
-__device__ __forceinline__ bool grid_sum_d(const GridSync &gs, Episode &episode,
-                                           const double (&v)[NV], double *buf, S &&side, M &&mid,
-                                           F &&f) {
-  __shared__ double s_part[NV][4];
+// Deterministic sum of NV FP64 values per thread over one cluster (or one
+// block) in a fixed order, which the cluster BiCGSTAB keeps (see
+// Scratch::ordered): four warps add blockDim / 128 values per lane (buf: NV x
+// blockDim doubles; blockDim.x a multiple of 128), warp 0 adds the four per
+// lane and finishes with a shuffle tree, the CTAs follow in rank order
+// (cluster_exchange).  Thread 0 then calls f(totals) -- the place for the
+// iteration's scalar FP64 work -- and one __syncthreads hands its results
+// (through shared memory) to the block.  Scalar work that needs nothing of
+// this sum (a division is 570 clocks) hides in the wait: thread 0 calls mid()
+// between its arrival and its wait, for values f uses; thread 32 calls side(),
+// for values of later phases.
+template <int NV, typename S, typename M, typename F>
+__device__ __forceinline__ void ordered_sum(const GridSync &gs, Episode &episode,
+                                            const double (&v)[NV], double *buf, S &&side, M &&mid,
+                                            F &&f) {
+  __shared__ double s_part[NV][128], s_slot[2][kMaxNV];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int bd = blockDim.x, per = bd >> 7;  // values per lane of the first level
 #pragma unroll
@@ -505,27 +485,32 @@ __device__ __forceinline__ bool grid_sum_d(const GridSync &gs, Episode &episode,
     for (int q = 0; q < NV; ++q) {
       const double *b = buf + q * bd + warp * (bd >> 2) + lane;
       double u = b[0];
-      if (per > 1) {
-        double u2 = b[32];
-#pragma unroll 1
-        for (int k = 2; k < per; k += 2) {
-          u = __dadd_rn(u, b[32 * k]);
-          if (k + 1 < per) u2 = __dadd_rn(u2, b[32 * k + 32]);
-        }
-        u = __dadd_rn(u, u2);
-      }
-      u = warp_sum(u);
-      if (lane == 0) s_part[q][warp] = u;
+      for (int k = 1; k < per; ++k) u = __dadd_rn(u, b[32 * k]);
+      s_part[q][threadIdx.x] = u;
     }
   }
   __syncthreads();
-  double bsum[NV];
-  if (threadIdx.x == 0)
+  const unsigned int ep = ++episode.n;
+  double t[NV];
+  if (warp == 0)
 #pragma unroll
-    for (int q = 0; q < NV; ++q)
-      bsum[q] = __dadd_rn(__dadd_rn(s_part[q][0], s_part[q][1]),
-                          __dadd_rn(s_part[q][2], s_part[q][3]));
-  return exchange_totals<NV, kPublish>(gs, episode, bsum, buf, bd, side, mid, f);
+    for (int q = 0; q < NV; ++q) {
+      double u = s_part[q][lane];
+#pragma unroll
+      for (int k = 1; k < 4; ++k) u = __dadd_rn(u, s_part[q][32 * k + lane]);
+      t[q] = warp_sum(u);
+      if (lane == 0) s_slot[ep & 1u][q] = t[q];
+    }
+  if (threadIdx.x == 32) side();
+  __syncwarp();
+  if (gs.cluster) {
+    cluster_sync_mid(mid);
+    cluster_exchange<NV>(s_slot, ep, t);
+  } else if (threadIdx.x == 0) {
+    mid();
+  }
+  if (threadIdx.x == 0) f(t);
+  __syncthreads();
 }
 
 // ---- scalar work of the recurrences ---------------------------------------
@@ -899,7 +884,7 @@ __device__ __forceinline__ void join_warps01() {
 // the limbs of the warp's values of quantity q (put_limbs), expo(q) gives the
 // value's biased FP64 exponent.  part: shared memory for NV * kLimbs * 32
 // ints.  win: the window of this kind of sum.  Thread 0 calls f(totals) as in
-// grid_sum_d; thread 32 calls side() while warp 0 exchanges (kJoin: for values
+// ordered_sum; thread 32 calls side() while warp 0 exchanges (kJoin: for values
 // f uses).  kPublish: as in exchange_totals.  Returns false when a wait
 // exceeded its bound (gs.err set).
 template <int NV, bool kPublish, bool kJoin, typename C, typename X, typename S, typename F>

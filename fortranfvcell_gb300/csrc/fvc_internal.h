@@ -65,6 +65,12 @@ struct Scratch {
   int *iresult = nullptr;
   double *trace = nullptr;      // per residual replacement: (iteration, ||r||/||b||)
   float *history = nullptr;     // per iteration: recursive ||r||/||b|| (first kHistoryMax)
+  // FP64 solves that fit one cluster add their sums in FP64 in a fixed order
+  // instead of exactly.  Set for the systems of a SIMPLE loop with energy: the
+  // last bits of a sum move its enthalpy by up to 1e-6 at a tolerance of 1e-10
+  // (BiCGSTAB stops an iteration earlier or later, both within the tolerance),
+  // so that a loop continued from a saved state would leave its old path.
+  bool ordered = false;
 };
 
 constexpr int kTraceMax = 256;
@@ -235,5 +241,7 @@ int32_t context_enqueue_batched(fvc_context *c, const BatchPlan &P, const double
 void context_free_batched(fvc_context *c, BatchPlan &P);
 // src/Solver.f's warm-start rule for (code, matriz): 1 zeroes x first
 int context_default_init(int code, int matriz);
+// Scratch::ordered of the context's solves
+void context_order_sums(fvc_context *c);
 
 }  // namespace fvc

@@ -105,15 +105,18 @@ __device__ __forceinline__ void finish(const KArgs &a, int iters, int status,
   finish_to(a.result, a.iresult, blockIdx.x == 0, iters, status, conv, crit, inner);
 }
 
-// The sums of the solver bodies: exact ones over a whole grid (kX), those of
-// grid_sum_d for the groups and clusters of a batch and the cluster kernels.
+// The sums of the solver bodies: exact ones (kX), or ordered_sum's (the
+// cluster BiCGSTAB).
 // side: scalars of later phases, mid: scalars f uses (thread 0 or 32).
 template <bool kX, int NV, bool kPublish, typename S, typename M, typename F>
 __device__ __forceinline__ bool sum_rows(const GridSync &gs, Episode &ep, ExactState &xs,
                                          SumWindow<NV> &win, const double (&v)[NV], double *buf,
                                          S &&side, M &&mid, F &&f) {
   constexpr bool kMid = !std::is_same<std::decay_t<M>, NoScalars>::value;
-  if (!kX) return grid_sum_d<NV, kPublish>(gs, ep, v, buf, side, mid, f);
+  if (!kX) {
+    ordered_sum<NV>(gs, ep, v, buf, side, mid, f);
+    return true;
+  }
   if (kMid) return grid_sum_x<NV, kPublish, true>(gs, ep, xs, win, v, buf, mid, f);
   return grid_sum_x<NV, kPublish, false>(gs, ep, xs, win, v, buf, side, f);
 }
@@ -1053,6 +1056,9 @@ constexpr int kStoreZRows = 73728;
 // iteration on GB300, cluster against grid-wide: 256 rows 10.0 vs 10.6 us,
 // 1024 rows 13.7 vs 11.5, 4096 rows 13.9 vs 11.8, 8100 rows 18.5 vs 12.2
 constexpr int kBcgClusterRows = 512;
+// ... and of a context whose sums keep their order (Scratch::ordered): as far
+// as one cluster is the better half of the time
+constexpr int kBcgOrderedRows = 8192;
 
 // Enqueues the cluster BiCGSTAB when the system is small enough, the caller
 // left the launch shape automatic and one cluster fits; FVC_ERR_UNSUPPORTED,
@@ -1060,7 +1066,7 @@ constexpr int kBcgClusterRows = 512;
 int32_t enqueue_bicgstab_cluster(const DeviceMatrix &A, Scratch &S, const double *b, double *x,
                                  double tol, int maxit, int init, const fvc_opts &o,
                                  cudaStream_t stream, bool launch) {
-  if (A.n <= 0 || A.n > kBcgClusterRows || o.block_threads != 0 || o.blocks_per_sm != 0 ||
+  if (A.n <= 0 || A.n > (S.ordered ? kBcgOrderedRows : kBcgClusterRows) || o.block_threads != 0 || o.blocks_per_sm != 0 ||
       o.max_blocks != 0)
     return FVC_ERR_UNSUPPORTED;
   constexpr int threads = 256;

@@ -83,7 +83,7 @@ __device__ __forceinline__ void ff_add(float &s, float &c, float s2, float c2) {
 // at grid_arrive), so every block holds identical totals.  Lane 0 of warp 0
 // then calls f(totals) -- the place for the iteration's scalar FP64 work,
 // which it publishes through shared memory -- and one __syncthreads hands the
-// results to the block; side() and mid() as in grid_sum_d.  Returns false
+// results to the block; side() and mid() as in ordered_sum.  Returns false
 // when a wait exceeded its bound (gs.err set).
 constexpr int kTotCap = 160;  // blocks whose partials one step sums (the device has 152 SMs)
 

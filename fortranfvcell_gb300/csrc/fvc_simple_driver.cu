@@ -929,6 +929,7 @@ int32_t fvc_simple_energy(fvc_simple *s, const int32_t *pedge_e, const double *s
     if ((rc = fvc_cells_ideal_gas_density((int)n, s->ro, s->temp, 1, row, 1.0, 1.0,
                                           s->stream)) != FVC_OK)
       return rc;
+  for (fvc_context *c : {s->ctx_u, s->ctx_pc, s->ctx_e}) fvc::context_order_sums(c);
   s->gas = true;
   if ((rc = time_term_gas(s)) != FVC_OK) return rc;
   return cudaStreamSynchronize(s->stream) == cudaSuccess ? FVC_OK : FVC_ERR_CUDA;
