@@ -16,7 +16,12 @@
 //
 // What bounds it: chains of dependent FP64 instructions (64 clocks each; two
 // warps of an SM sub-partition share a pipe that takes one per 76 clocks) and
-// the barriers (420 clocks, and 230 for the DSMEM read after each).
+// the barriers (420 clocks, and 230 for the DSMEM read after each).  Of the
+// 7,000 clocks of an iteration at 2304 rows each sum takes some 1,900, the SpMV
+// 1,100, the scalars between 300 (alpha) and 400 (beta, the stopping test).
+// Per iteration, against rows in shared memory and sums in FP64: 256 rows 3.3
+// us, 1024 rows 3.3, 2304 rows 3.5 against 6.4, 4096 rows 3.6 against 6.7, 8100
+// rows 4.4 against 8.4.
 //
 // There is no spin-wait: the only waits are hardware cluster barriers, which
 // every CTA reaches the same number of times (the loop exit depends only on
@@ -39,7 +44,8 @@ namespace {
 
 constexpr int kClMax = 16;        // CTAs per cluster (non-portable above 8)
 constexpr int kClMaxRows = 512;   // rows per CTA: one per thread
-// Largest system run on a cluster (16 CTAs of 256 rows and more).
+// Largest system run on a cluster: per iteration against the grid-wide kernel
+// (128-thread blocks), 4096 rows 3.6 and 5.6 us, 8100 rows 4.4 and 6.1.
 constexpr int kClMaxN = 8192;
 
 struct ClArgs {
@@ -65,12 +71,21 @@ struct ClLayout {
 
 extern __shared__ __align__(16) unsigned char cl_smem[];
 
+// sqrt_bound's bound with room for the roundings between t[0] and beta d
+__device__ __forceinline__ long long far_bound(long long bound) {
+  return bound >= 0x7ff0000000000000ll ? 0x7fffffffffffffffll : bound + 16;
+}
+__device__ __forceinline__ bool middling(double v) {
+  const int e = (__double2hiint(v) >> 20) & 0x7ff;
+  return e > 1023 - 500 && e < 1023 + 500;
+}
+
 // The cluster's state of its sums (shared memory of each CTA): ExactState
 // without the words, and the two sets of posted limbs.
 struct ClSum {
   ExactState xs;
   long long post[2][32];
-  alignas(8) int part[3 * kLimbs * 32];
+  alignas(8) int part[6 * 32];  // ordered: 3 x 32 doubles
 };
 
 // The same sum added in FP64 in a fixed order (Scratch::ordered): a shuffle
@@ -157,16 +172,10 @@ __device__ __forceinline__ void cluster_sum(cg::cluster_group &cl, unsigned int 
       __syncthreads();
     }
     const unsigned int set = ep++ & 1u;
-    bool ovf = false;
 #pragma unroll
-    for (int q = 0; q < NV; ++q)
-      ovf = put_limbs(v[q], win.top[q], cs.part + q * kLimbs * 32) || ovf;
-    ovf = __any_sync(0xffffffffu, ovf);
-    if (lane == 0) xs.ovf[warp] = ovf ? 1 : 0;
-    if (threadIdx.x < NV) xs.top[threadIdx.x] = win.top[threadIdx.x];
-    if (threadIdx.x == 0) xs.sure = have ? 0 : 1;
+    for (int q = 0; q < NV; ++q) put_limbs(v[q], win.top[q], xs.acc[set] + 8 * q);
     __syncthreads();
-    if (warp == 0) cs.post[set][lane] = block_limbs(NV, cs.part, xs);
+    if (warp == 0) cs.post[set][lane] = block_limbs(xs.acc[set]);
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     if (first) {
       overlap();
@@ -175,17 +184,27 @@ __device__ __forceinline__ void cluster_sum(cg::cluster_group &cl, unsigned int 
     }
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     if (warp == 0) {
-      long long d[kClMax], s = 0;
+      // every lane reads kClMax / kG CTAs' words, the lanes add theirs
+      constexpr int kG = NV == 1 ? 4 : NV == 2 ? 2 : 1, kW = 32 / kG;
+      long long d[kClMax / kG], s = 0;
 #pragma unroll
-      for (int c = 0; c < kClMax; ++c)
-        d[c] = (c < nb) ? *cl.map_shared_rank(&cs.post[set][lane], c) : 0;
+      for (int i = 0; i < kClMax / kG; ++i) {
+        const int c = i * kG + lane / kW;
+        d[i] = (c < nb) ? *cl.map_shared_rank(&cs.post[set][lane % kW], c) : 0;
+      }
 #pragma unroll
-      for (int c = 0; c < kClMax; ++c) s += d[c];
+      for (int i = 0; i < kClMax / kG; ++i) s += d[i];
+#pragma unroll
+      for (int o = kW; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       const long long L = (long long)((unsigned long long)s << 22) >> 22;
-      limb_totals(NV, L, ((s - L) >> 42) != 0, true, xs);
-      if (lane == 0 && xs.flag == 1) {
-        window_set<NV>(win, xs.tot);
-        f(xs.tot);
+      double t[NV];
+      const int r = limb_totals<NV>(L, ((s - L) >> 42) != 0, true, !have, win, xs, t);
+      if (lane == 0) {
+        xs.flag = r;
+        if (r == 1) {
+          window_set<NV>(win, t);
+          f(t);
+        }
       }
       __syncwarp();
     }
@@ -206,7 +225,7 @@ __global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
   __shared__ struct {
     double d, alpha, beta, conv, crit2;
     Divisor dv;
-    long long bound;
+    long long bound, far;  // of the stopping test
     int stop;
   } sh;
   const int rank = (int)cl.block_rank(), nb = (int)cl.num_blocks();
@@ -222,6 +241,7 @@ __global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
   int *col = reinterpret_cast<int *>(val + S);  // (owner << 16) | local row
   int *sp = col + S;                            // slot offset of each local slice
   const bool has_diag = a.A.diag_mode != DIAG_NONE;
+  exact_init(cs.xs);
   if (threadIdx.x == 0) wpq.top[0] = wrz.top[0] = wrr.top[0] = w3.top[0] = kNoWindow;
 #ifdef FVC_CHECK
   // check builds: columns outside [0, n) (whose owner CTA would not be in
@@ -306,6 +326,7 @@ __global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
     sh.d = t[0];
     sh.conv = a.tol * root(rule0 ? fabs(t[0]) : t[1]);
     sh.bound = sqrt_bound(sh.conv);
+    sh.far = far_bound(sh.bound);
     sh.crit2 = 0.0;
     wrz.top[0] = window_top(t[0]);
     wrr.top[1] = kNoWindow;
@@ -319,7 +340,10 @@ __global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
     // p = z + beta p on the own rows (the first: p = z), then visible to the cluster
     pi = fma(beta, pi, z);
     if (i < R) p[i] = pi;
-    cl.sync();
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    if (threadIdx.x == 0 && j > 1) sh.d = sh.beta * sh.d;  // read after the next __syncthreads
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     const double qi = own ? spmv_row(pi, 0) : 0.0;
     const double pq[1] = {pi * qi};
     cluster_sum<kOrdered, 1>(cl, ep, cs, wpq, pq, none, [&] { sh.dv.set(sh.d); },
@@ -329,14 +353,25 @@ __global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
     const double alpha = sh.alpha;
     r = fma(-alpha, qi, r);
     z = r * mi;
+    // beta = r.z / d ; the next d = beta d, formed while the next barrier is
+    // waited for; the reference's stopping test.  Far from its bound the test
+    // needs neither d nor a root: beta d is t[0] to two roundings (exponents
+    // within +-500 of 1)
     auto step = [&](const double *t) {
-      sh.beta = quotient(t[0], sh.dv);
-      sh.d = sh.beta * sh.d;
-      const double crit2 = rule0 ? fabs(sh.d) : t[rule0 ? 0 : 1];
+      const double b = quotient(t[0], sh.dv);
+      sh.beta = b;
+      const double c = rule0 ? t[0] : t[rule0 ? 0 : 1];
+      if (middling(t[0]) && middling(b) && __double_as_longlong(c) > sh.far && !is_nan_bits(c)) {
+        sh.stop = 0;
+        if (!rule0) sh.crit2 = c;
+        return;
+      }
+      const double d = b * sh.d;
+      const double crit2 = rule0 ? fabs(d) : c;
       sh.crit2 = crit2;
-      sh.stop = (is_nan_bits(crit2) || not_finite_bits(sh.d)) ? 2
-                : sqrt_below(crit2, sh.conv, sh.bound)        ? 1
-                                                              : 0;
+      sh.stop = (is_nan_bits(crit2) || not_finite_bits(d)) ? 2
+                : sqrt_below(crit2, sh.conv, sh.bound)     ? 1
+                                                           : 0;
     };
     auto update_x = [&] { x = fma(alpha, pi, x); };
     if (rule0) {
@@ -356,6 +391,7 @@ __global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
   if (j > a.maxit && status == FVC_OK) {
     j = a.maxit;
     status = FVC_ERR_NOCONV;
+    if (rule0 && j > 0 && threadIdx.x == 0) sh.crit2 = fabs(sh.beta * sh.d);
   }
   if (status == FVC_ERR_ARG) j = 0;
   // x.Ax, |b - Ax|^2, |b|^2 (x complete in every CTA after the barrier)
@@ -388,9 +424,13 @@ __global__ void __launch_bounds__(kClMaxRows, 1) pcg_cluster(ClArgs a) {
 // The cluster layout of an n-row system: CTAs, rows per CTA (a multiple of
 // 32, at most kClMaxRows, over at most kClMax CTAs).  False when the system
 // does not fit one cluster.
-bool cluster_shape(int n, int &nb, int &R) {
+// One warp of rows per SM sub-partition while 16 CTAs hold them (an FP64
+// instruction of a warp takes its sub-partition's pipe for 76 clocks), two for
+// ordered sums, whose order the split is part of.
+bool cluster_shape(int n, bool ordered, int &nb, int &R) {
   if (n <= 0 || n > kClMaxN) return false;
-  nb = std::min(kClMax, std::max(1, (n + 255) / 256));
+  const int per = ordered ? 256 : 128;
+  nb = std::min(kClMax, std::max(1, (n + per - 1) / per));
   R = ((n + nb - 1) / nb + 31) / 32 * 32;
   if (R > kClMaxRows) return false;
   nb = (n + R - 1) / R;
@@ -403,12 +443,14 @@ bool cluster_shape(int n, int &nb, int &R) {
 // layout, from the host copy of the slice pointers; -1 when the system does
 // not fit one cluster.
 int cluster_slots_max(int n, int nslices, const int64_t *sptr) {
-  int nb = 0, R = 0;
-  if (!sptr || !cluster_shape(n, nb, R)) return -1;
-  int smax = 0;
-  for (int c = 0; c < nb; ++c) {
-    const int s0 = c * R / 32, s1 = std::min(nslices, (c + 1) * R / 32);
-    smax = std::max(smax, (int)(sptr[s1] - sptr[s0]));
+  int smax = sptr ? 0 : -1;
+  for (const bool ordered : {false, true}) {  // the larger serves both
+    int nb = 0, R = 0;
+    if (!sptr || !cluster_shape(n, ordered, nb, R)) return -1;
+    for (int c = 0; c < nb; ++c) {
+      const int s0 = c * R / 32, s1 = std::min(nslices, (c + 1) * R / 32);
+      smax = std::max(smax, (int)(sptr[s1] - sptr[s0]));
+    }
   }
   return smax;
 }
@@ -423,7 +465,7 @@ int32_t enqueue_pcg_cluster(const DeviceMatrix &A, Scratch &S, const double *b, 
   const int n = A.n;
   if (n <= 0 || A.diag_mode == DIAG_NONE || !A.jinv) return FVC_ERR_UNSUPPORTED;
   int nb = 0, R = 0;
-  if (!cluster_shape(n, nb, R)) return FVC_ERR_UNSUPPORTED;
+  if (!cluster_shape(n, S.ordered, nb, R)) return FVC_ERR_UNSUPPORTED;
   int smax = A.cl_smax;
   if (smax < 0) {  // a matrix loaded without the host-side count
     std::vector<int64_t> sptr((size_t)A.nslices + 1);

@@ -549,14 +549,16 @@ __device__ __forceinline__ double quotient(double t, const Divisor &v) {
 }
 
 // t / d from scratch: the reciprocal's hardware approximation (rcp.approx.f64,
-// 20 bits and more), one Newton step, Markstein's correction of t * r as above
-// (about 360 clocks against 570 of the division).  Divisors out of range, and
+// 20 bits and more) r, one Newton step for it and for t r side by side,
+// Markstein's correction as above (about 300 clocks against 570 of the
+// division).  Divisors out of range, and
 // quotients that are not finite, take the division.
 __device__ __forceinline__ double quick_quotient(double t, double d) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  r = fma(fma(-d, r, 1.0), r, r);
-  const double q = t * r;
+  const double h = fma(-d, r, 1.0), q0 = t * r;
+  r = fma(h, r, r);
+  const double q = fma(h, q0, q0);
   const double z = fma(fma(-q, d, t), r, q);
   const int e = (__double2hiint(d) >> 20) & 0x7ff;
   if (e <= 1023 - 500 || e >= 1023 + 500 || not_finite_bits(z)) return divide(t, d);
@@ -592,8 +594,9 @@ struct NoScalars {
 // Every thread splits its FP64 partial into kLimbs signed limbs of kLimbBits
 // bits of one fixed-point window that all blocks know (its top lies
 // kWindowHead bits above the total of the same sum one iteration ago); a
-// warp adds a limb with one redux, a block its warps' with another, and the
-// blocks add theirs into one 64-bit word per limb with relaxed atomics.
+// warp adds a limb with one redux, the warps of a block theirs in shared
+// memory by atomics (a second redux over the warps took 330 clocks, this 60),
+// and the blocks into one 64-bit word per limb with relaxed atomics.
 // Integer addition is associative, so the total does not depend on the
 // order: deterministic, and exact but for the bits below the window (less
 // than 2^-53.7 of the total, see sum_bad) and the limbs' addition in FP64.  The word's upper bits count the
@@ -619,12 +622,11 @@ constexpr int kXBlocks = 2047;            // most blocks a word's count serves
 // A block's state of the exact sums (shared memory).
 struct ExactState {
   unsigned long long snap[2][kXWords];
-  int ovf[32];
-  double tot[kMaxNV];
-  int top[kMaxNV];  // the window of the running sum
+  // the block's sums (two sets alternate, all zero between uses): limb k of
+  // quantity q at 8 q + k, the warps with a value above the window at 8 q + 6
+  int acc[2][32];
   int flag, pub_ok;
-  int sure;  // that window follows from the partials
-  int nan;   // and some partial was NaN or Inf: so is the total
+  int nan;  // some partial was NaN or Inf: so is the total
 };
 // The window of one kind of sum: its top, an exponent of two, per quantity.
 template <int NV>
@@ -644,7 +646,7 @@ __device__ __forceinline__ void window_set(SumWindow<NV> &w, const double *t) {
 }
 
 // A warp's values +-m 2^e (m < 2^53; up to two per lane) as limbs of the window
-// with the given top, added over the warp and left in part[32 k + warp] for
+// with the given top, added over the warp and then to the block's acc[k] for
 // limb k.  True in the lanes whose value does not fit.
 __device__ __forceinline__ bool add_limbs(int (&l)[kLimbs], unsigned long long m, int e, int neg,
                                           int top) {
@@ -670,27 +672,26 @@ __device__ __forceinline__ bool add_limbs(int (&l)[kLimbs], unsigned long long m
   for (int k = 0; k < kLimbs; ++k) l[k] += (x[k] ^ -neg) + neg;
   return s > kWindowBits - 53 - 1;
 }
-__device__ __forceinline__ void warp_limbs(const int (&l)[kLimbs], int *part) {
+__device__ __forceinline__ void warp_limbs(const int (&l)[kLimbs], bool ovf, int *acc) {
   const int lane = threadIdx.x & 31;
-  int mine = 0;
+  int mine = __any_sync(0xffffffffu, ovf) ? 1 : 0;  // lane kLimbs
 #pragma unroll
   for (int k = 0; k < kLimbs; ++k) {
     const int r = __reduce_add_sync(0xffffffffu, l[k]);
     if (lane == k) mine = r;
   }
-  if (lane < kLimbs) part[32 * lane + (threadIdx.x >> 5)] = mine;
+  if (lane <= kLimbs) atomicAdd(acc + lane, mine);
 }
-__device__ __forceinline__ bool put_limbs(double v, int top, int *part) {
+__device__ __forceinline__ void put_limbs(double v, int top, int *acc) {
   int l[kLimbs] = {0, 0, 0, 0, 0, 0};
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   const int ex = (int)(b >> 52) & 0x7ff;
   const unsigned long long m = (b & 0xfffffffffffffull) | ((unsigned long long)(ex != 0) << 52);
   const bool ovf = add_limbs(l, m, (ex ? ex : 1) - 1075, (int)(b >> 63), top);
-  warp_limbs(l, part);
-  return ovf;
+  warp_limbs(l, ovf, acc);
 }
 // The value of an FP32 pair, its parts renormalised so that they do not overlap
-__device__ __forceinline__ bool put_limbs(float s, float c, int top, int *part) {
+__device__ __forceinline__ void put_limbs(float s, float c, int top, int *acc) {
   int l[kLimbs] = {0, 0, 0, 0, 0, 0};
   const float hi = __fadd_rn(s, c);
   const float lo = __fsub_rn(c, __fsub_rn(hi, s));
@@ -704,12 +705,11 @@ __device__ __forceinline__ bool put_limbs(float s, float c, int top, int *part) 
     const int e = ex == 0xff ? 4096 : (ex ? ex : 1) - 150;
     ovf = add_limbs(l, (unsigned long long)m, e, (int)(b >> 31), top) || ovf;
   }
-  warp_limbs(l, part);
-  return ovf;
+  warp_limbs(l, ovf, acc);
 }
 
-// Limb k of a total in FP64: L 2^(21 k) units of the window, exact (|L| <
-// 2^41) unless it leaves FP64's exponents (then 0 or Inf).
+// L 2^(21 k) units of the window in FP64, rounded once, unless it leaves
+// FP64's exponents (then 0 or Inf).
 __device__ __forceinline__ double limb_value(long long L, int k, int top) {
   const double v = (double)L;
   const int hi = __double2hiint(v), sh = top - kWindowBits + kLimbBits * k;
@@ -728,7 +728,10 @@ __device__ __forceinline__ bool sum_bad(double t, int top) {
 
 __device__ __forceinline__ void exact_init(ExactState &xs) {  // a __syncthreads must follow
 #pragma unroll 1
-  for (int i = threadIdx.x; i < 2 * kXWords; i += blockDim.x) (&xs.snap[0][0])[i] = 0;
+  for (int i = threadIdx.x; i < 2 * kXWords; i += blockDim.x) {
+    (&xs.snap[0][0])[i] = 0;
+    (&xs.acc[0][0])[i] = 0;
+  }
 }
 
 // The top of a window that holds partials of biased exponents up to m
@@ -786,60 +789,57 @@ static __device__ __noinline__ bool window_by_partials(const GridSync &gs, Episo
   return true;
 }
 
-// Warp 0's part of an exact sum of nv quantities.  First the block's limbs from
-// its warps' (part): lane 8 q + k gets limb k of quantity q with the overflow
-// mark in bits 42 on.
-__device__ __forceinline__ long long block_limbs(int nv, const int *part, const ExactState &xs) {
-  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  long long w = 0;
-#pragma unroll 1
-  for (int q = 0; q < nv; ++q)
-#pragma unroll
-    for (int k = 0; k < kLimbs; ++k) {
-      const int r =
-          __reduce_add_sync(0xffffffffu, lane < nw ? part[(q * kLimbs + k) * 32 + lane] : 0);
-      if (lane == 8 * q + k) w = r;
-    }
-  const bool o = __any_sync(0xffffffffu, lane < nw && xs.ovf[lane] != 0);
-  return w + ((long long)(o ? 1 : 0) << 42);
+// Warp 0's part of an exact sum.  First the block's limbs: lane 8 q + k gets
+// limb k of quantity q with the overflow mark in bits 42 on; acc is zero again.
+__device__ __forceinline__ long long block_limbs(int *acc) {
+  const int lane = threadIdx.x & 31;
+  const int w = acc[lane];
+  acc[lane] = 0;
+  const bool o = __any_sync(0xffffffffu, (lane & 7) == kLimbs && w != 0);
+  return ((lane & 7) < kLimbs ? w : 0) + ((long long)(o ? 1 : 0) << 42);
 }
 // Then, from the limbs of all blocks (L) and whether any overflowed (bad), the
-// totals into xs.tot and the verdict into xs.flag (0 a wait exceeded its bound,
-// 1 good, 2 the window did not hold it).
-__device__ __forceinline__ void limb_totals(int nv, long long L, bool bad, bool ok,
-                                            ExactState &xs) {
+// totals t (in every lane) and the verdict: 0 a wait exceeded its bound, 1
+// good, 2 the window did not hold it (never where it follows from the
+// partials, sure).  Two limbs are added as integers (|L| < 2^41), the three
+// pairs in FP64.
+template <int NV>
+__device__ __forceinline__ int limb_totals(long long L, bool bad, bool ok, bool sure,
+                                           const SumWindow<NV> &win, const ExactState &xs,
+                                           double (&t)[NV]) {
   const int lane = threadIdx.x & 31, lq = lane >> 3, lk = lane & 7;
-  const bool mine = lq < nv && lk < kLimbs;
-  const int top = xs.top[mine ? lq : 0];
-  // the limbs of a quantity added in FP64
-  double tq = mine ? limb_value(L, lk, top) : 0.0;
+  const bool mine = lq < NV && lk < kLimbs;
+  const int top = win.top[lq < NV ? lq : 0];
+  if (!mine) L = 0;
+  L += __shfl_down_sync(0xffffffffu, L, 1) << kLimbBits;
+  double tq = (lk & 1) ? 0.0 : limb_value(L, lk, top);
 #pragma unroll
-  for (int k = 1; k < 8; k <<= 1) tq = __dadd_rn(tq, __shfl_xor_sync(0xffffffffu, tq, k));
-  if (xs.sure) {
-    bad = false;  // only NaN and Inf overflow a window that follows from the partials
+  for (int k = 2; k < 8; k <<= 1) tq = __dadd_rn(tq, __shfl_xor_sync(0xffffffffu, tq, k));
+  if (sure) {
+    bad = false;  // only NaN and Inf overflow such a window
     if (xs.nan) tq = __longlong_as_double(0x7ff8000000000000ll);
   } else {
-    bad = mine && (bad || sum_bad(tq, top));
+    bad = mine && (bad || ((lk & 1) == 0 && sum_bad(tq, top)));
   }
   bad = __any_sync(0xffffffffu, bad);
   ok = __all_sync(0xffffffffu, ok);
-  if (lk == 0 && lq < nv) xs.tot[lq] = tq;
-  if (lane == 0) xs.flag = !ok ? 0 : bad ? 2 : 1;
-  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < NV; ++q) t[q] = __shfl_sync(0xffffffffu, tq, 8 * q);
+  return !ok ? 0 : bad ? 2 : 1;
 }
 // The exchange over a grid between the two, through the words of this set.
-__device__ __forceinline__ void exact_words(unsigned long long *xw, int *err, unsigned int nb,
-                                            unsigned int set, int nv, const int *part,
-                                            ExactState &xs) {
+template <int NV>
+__device__ __forceinline__ int exact_words(unsigned long long *xw, int *err, unsigned int nb,
+                                           unsigned int set, bool sure, const SumWindow<NV> &win,
+                                           ExactState &xs, double (&t)[NV]) {
   const int lane = threadIdx.x & 31, lq = lane >> 3, lk = lane & 7;
-  const bool mine = lq < nv && lk < kLimbs;
-  const long long w = block_limbs(nv, part, xs);
+  const bool mine = lq < NV && lk < kLimbs;
+  const long long w = block_limbs(xs.acc[set]);
   long long L = 0;
   bool ok = true, bad = false;
   if (nb == 1) {  // its limbs are the total
     L = (long long)((unsigned long long)w << 22) >> 22;
-    limb_totals(nv, L, w != L, true, xs);
-    return;
+    return limb_totals<NV>(L, w != L, true, sure, win, xs, t);
   }
   // (the other lanes poll along on the first word, see wait_count)
   unsigned long long *word = xw + set * kXWords + (mine ? lane : 0);
@@ -870,8 +870,7 @@ __device__ __forceinline__ void exact_words(unsigned long long *xw, int *err, un
     }
   }
   if (mine) xs.snap[set][lane] = now;
-  __syncwarp();
-  limb_totals(nv, L, bad, ok, xs);
+  return limb_totals<NV>(L, bad, ok, sure, win, xs, t);
 }
 
 // Warps 0 and 1 of the block meet (the values of side() for f()).
@@ -880,10 +879,9 @@ __device__ __forceinline__ void join_warps01() {
   asm volatile("barrier.sync 1, 64;" ::: "memory");
 }
 
-// Grid-wide deterministic sum of NV values per thread: put(q, top, part) leaves
+// Grid-wide deterministic sum of NV values per thread: put(q, top, acc) adds
 // the limbs of the warp's values of quantity q (put_limbs), expo(q) gives the
-// value's biased FP64 exponent.  part: shared memory for NV * kLimbs * 32
-// ints.  win: the window of this kind of sum.  Thread 0 calls f(totals) as in
+// value's biased FP64 exponent.  part: shared memory for NV * 32 ints.  win: the window of this kind of sum.  Thread 0 calls f(totals) as in
 // ordered_sum; thread 32 calls side() while warp 0 exchanges (kJoin: for values
 // f uses).  kPublish: as in exchange_totals.  Returns false when a wait
 // exceeded its bound (gs.err set).
@@ -905,20 +903,19 @@ __device__ __forceinline__ bool exact_sum(const GridSync &gs, Episode &episode, 
       if (!window_by_partials(gs, episode, xs, win.top, NV, ex, part)) return false;
     }
     const unsigned int set = (episode.x++) & 1u;
-    bool ovf = false;
 #pragma unroll
-    for (int q = 0; q < NV; ++q) ovf = put(q, win.top[q], part + q * kLimbs * 32) || ovf;
-    ovf = __any_sync(0xffffffffu, ovf);
-    if (lane == 0) xs.ovf[warp] = ovf ? 1 : 0;
-    if (threadIdx.x < NV) xs.top[threadIdx.x] = win.top[threadIdx.x];
-    if (threadIdx.x == 0) xs.sure = have ? 0 : 1;
+    for (int q = 0; q < NV; ++q) put(q, win.top[q], xs.acc[set] + 8 * q);
     __syncthreads();
     if (warp == 0) {
-      exact_words(gs.xw, gs.err, gs.nblocks, set, NV, part, xs);
+      double t[NV];
+      const int r = exact_words<NV>(gs.xw, gs.err, gs.nblocks, set, !have, win, xs, t);
       if (kJoin && first) join_warps01();
-      if (lane == 0 && xs.flag == 1) {
-        window_set<NV>(win, xs.tot);
-        f(xs.tot);
+      if (lane == 0) {
+        xs.flag = r;
+        if (r == 1) {
+          window_set<NV>(win, t);
+          f(t);
+        }
       }
     } else if (warp == 1) {
       if (lane == 0 && first) side();
@@ -947,7 +944,7 @@ __device__ __forceinline__ bool grid_sum_x(const GridSync &gs, Episode &episode,
                                            S &&side, F &&f) {
   return exact_sum<NV, kPublish, kJoin>(
       gs, episode, xs, win, reinterpret_cast<int *>(buf),
-      [&](int q, int top, int *part) { return put_limbs(v[q], top, part); },
+      [&](int q, int top, int *acc) { put_limbs(v[q], top, acc); },
       [&](int q) { return (__double2hiint(v[q]) >> 20) & 0x7ff; }, side, f);
 }
 

@@ -130,10 +130,10 @@ __device__ __forceinline__ bool grid_sum_ffx(const GridSync &gs, Episode &episod
                                              SumWindow<NV> &win, const CSum (&v)[NV],
                                              float2 *red2, double *tot, S &&side, M &&mid,
                                              F &&f) {
-  static_assert(NV * kLimbs * 32 * sizeof(int) <= 2 * kTotCap * sizeof(double), "limb sums");
+  static_assert(NV * 32 * sizeof(int) <= 2 * kTotCap * sizeof(double), "exponents");
   constexpr bool kMid = !std::is_same<std::decay_t<M>, NoScalars>::value;
   if (!kX) return grid_allreduce_ff<NV, kPublish>(gs, episode, v, red2, tot, side, mid, f);
-  auto put = [&](int q, int top, int *part) { return put_limbs(v[q].s, v[q].c, top, part); };
+  auto put = [&](int q, int top, int *acc) { put_limbs(v[q].s, v[q].c, top, acc); };
   auto expo = [&](int q) {  // as an FP64 exponent
     const int ex = (int)(__float_as_uint(__fadd_rn(v[q].s, v[q].c)) >> 23) & 0xff;
     return ex == 0xff ? 0x7ff : (ex ? ex : 1) - 127 + 1023;
