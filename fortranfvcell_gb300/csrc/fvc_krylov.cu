@@ -54,6 +54,7 @@ struct KArgs {
   int stop_rule;
   double *result;  // [0] energy [1] conv [2] final_crit [3] |b-Ax|^2 [4] |b|^2
   int *iresult;    // [0] iterations [1] status [2] inner iterations
+  int cap, capm;   // rows per thread whose own vectors / matrix lie in shared memory (Resident)
 };
 
 // Slice range of this block and the lane/warp decomposition.
@@ -86,8 +87,80 @@ struct Part {
 // code, and the BiCGSTAB of 262k rows took 2 % longer.)
 #define FOR_ROWS(P)                                          \
   _Pragma("unroll 1")                                        \
-  for (int s_ = (P).sb + (P).warp; s_ < (P).se; s_ += (P).nwarps) \
+  for (int s_ = (P).sb + (P).warp, it_ = 0; s_ < (P).se; s_ += (P).nwarps, ++it_) \
     for (int row = s_ * 32 + (P).lane, once_ = 1; once_ && row < (P).n; once_ = 0)
+
+// What only a row's own thread reads stays in shared memory: its matrix row for
+// the thread's first `capm` rows (up to four stored entries), the solver's own
+// vectors for the first `cap`; the other rows' lie in global memory.
+extern __shared__ double resident_smem[];
+template <int kVec>
+struct Resident {
+  int cap, capm;
+  __device__ __forceinline__ explicit Resident(const KArgs &a) : cap(a.cap), capm(a.capm) {}
+  // vector vec (g in global memory) at the thread's it-th row
+  __device__ __forceinline__ double &operator()(int vec, int it, double *g, int row) const {
+    return it < cap ? resident_smem[(vec * cap + it) * blockDim.x + threadIdx.x] : g[row];
+  }
+  // entry k of the it-th row: its value (k = 4: the diagonal) and column
+  __device__ __forceinline__ double &val(int k, int it) const {
+    return resident_smem[(kVec * cap + k * capm + it) * blockDim.x + threadIdx.x];
+  }
+  __device__ __forceinline__ int &col(int k, int it) const {
+    return reinterpret_cast<int *>(resident_smem +
+                                   (kVec * cap + 5 * capm) * blockDim.x)[(k * capm + it) *
+                                                                             blockDim.x +
+                                                                         threadIdx.x];
+  }
+  // Copies row `row` of A (kT: of A^T) in; a row of more than four entries
+  // stays where it is (its first column -2), absent entries get column -1.
+  template <bool kT>
+  __device__ __forceinline__ void load(const SellView<double> &A, int s, int it, int lane,
+                                       int row) const {
+    if (it >= capm) return;
+    const int64_t base = A.sptr[s] + lane;
+    const int w = (int)((A.sptr[s + 1] - A.sptr[s]) >> 5);
+    FVC_CHK(w >= 0 && w <= A.n, A.chk, kChkSliceWidth, col(0, it) = -2; return);
+    if (A.diag_mode != DIAG_NONE) val(4, it) = A.diag[row];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      int c = w > 4 ? -2 : -1;
+      if (w <= 4 && k < w) {
+        c = A.col[base + 32 * k];
+        FVC_CHK((unsigned)c < (unsigned)A.n, A.chk, kChkColumn, c = row);
+        int64_t m = base + 32 * k;
+        if (kT) m = A.mirror[m];
+#ifdef FVC_CHECK
+        const int64_t nslots = A.sptr[A.nslices];
+        FVC_CHK(m >= 0 && m < nslots, A.chk, kChkMirror, m = base);
+#endif
+        val(k, it) = A.val[m];
+      }
+      col(k, it) = c;
+    }
+  }
+  // (A x)_row (kT: (A^T x)_row), in the order of row_fma
+  template <bool kT, typename XF>
+  __device__ __forceinline__ double product(const SellView<double> &A, int s, int it, int lane,
+                                            int row, XF xf) const {
+    if (it < capm && col(0, it) != -2) {
+      int c[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) c[k] = col(k, it);
+      const bool first = kT ? A.diag_mode != DIAG_NONE : A.diag_mode == DIAG_FIRST;
+      const bool last = !kT && A.diag_mode == DIAG_LAST;
+      double xi = 0.0, t = 0.0;
+      if (first || last) xi = xf(row);
+      if (first) t = val(4, it) * xi;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (c[k] >= 0) t = fma(val(k, it), xf(c[k]), t);
+      if (last) t = fma(val(4, it), xi, t);
+      return t;
+    }
+    return row_fma<kT>(A, s, lane, row, xf);
+  }
+};
 
 __device__ __forceinline__ void finish_to(double *result, int *iresult, bool lead, int iters,
                                           int status, double conv, double crit, int inner) {
@@ -164,7 +237,7 @@ __device__ __forceinline__ void epilogue_to(const KArgs &a, const Part &P, doubl
 template <bool kStoreP, int kMaxT = 1024, bool kX = true>
 __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const GridSync &gs,
                                         double *result, int *iresult, bool lead) {
-  __shared__ double buf[3 * kMaxT];
+  __shared__ double buf[48];  // (window_by_partials: 3 x 32 ints)
   // scalars of the recurrence, updated by lane 0 of warp 0 inside the
   // all-reduces and read by every thread after them
   __shared__ struct {
@@ -180,26 +253,37 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
   exact_init(xs);
   if (threadIdx.x == 0) wpq.top[0] = wrz.top[0] = wrr.top[0] = kNoWindow;
   __syncthreads();
-  double *r = a.v0, *z = a.v1, *q = a.v4, *x = a.x;
+  double *z = a.v1;
+  // own: r, x, and q which takes z's place between the sums (kStoreP: no other
+  // thread reads z)
+  const Resident<3> own(a);
+#define R_ own(0, it_, a.v0, row)
+#define Q_ own(1, it_, a.v4, row)
+#define X_ own(2, it_, a.x, row)
   const NoScalars none;
   const double *minv = a.minv, *b = a.b;
   const bool rule0 = a.stop_rule == 0;
   Episode ep;
 
+  FOR_ROWS(P) own.load<false>(a.A, s_, it_, P.lane, row);
   // r = b - A x ; z = r/m ; p = z ; d = r.z  (x = 0 when init)
   double acc[2] = {0.0, 0.0};
   FOR_ROWS(P) {
     double ax;
     if (a.init) {
       ax = 0.0;
-      x[row] = 0.0;
+      X_ = 0.0;
     } else {
-      ax = sell_row_fma(a.A, s_, P.lane, row, [&](int k) { return x[k]; });
+      ax = own.product<false>(a.A, s_, it_, P.lane, row, [&](int k) { return a.x[k]; });
+      if (it_ < own.cap) X_ = a.x[row];
     }
     const double ri = b[row] - ax;
     const double zi = ri * minv[row];
-    r[row] = ri;
-    z[row] = zi;
+    R_ = ri;
+    if (kStoreP)
+      Q_ = zi;
+    else
+      z[row] = zi;
     a.v2[row] = zi;
     acc[0] = fma(ri, zi, acc[0]);
     acc[1] = fma(b[row], b[row], acc[1]);
@@ -224,14 +308,14 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
     // q = A p  (p = z + beta*p formed on the fly for j >= 2); p.q
     double pq[1] = {0.0};
     if (kStoreP && j > 1) {
-      FOR_ROWS(P) pcur[row] = fma(beta, pcur[row], z[row]);
+      FOR_ROWS(P) pcur[row] = fma(beta, pcur[row], Q_);
       if (!grid_barrier(gs, ep)) return;
     }
     if (kStoreP) {
       FOR_ROWS(P) {
         const double *pc = pcur;
-        const double qi = sell_row_fma(a.A, s_, P.lane, row, [&](int k) { return pc[k]; });
-        q[row] = qi;
+        const double qi = own.product<false>(a.A, s_, it_, P.lane, row, [&](int k) { return pc[k]; });
+        Q_ = qi;
         pq[0] = fma(pc[row], qi, pq[0]);
       }
     } else {
@@ -240,25 +324,29 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
         auto pf = [&](int k) { return fma(beta, pp[k], z[k]); };
         const double pi = pf(row);
         pcur[row] = pi;
-        const double qi = sell_row_fma(a.A, s_, P.lane, row, pf);
-        q[row] = qi;
+        const double qi = own.product<false>(a.A, s_, it_, P.lane, row, pf);
+        Q_ = qi;
         pq[0] = fma(pi, qi, pq[0]);
       }
     }
     // what follows touches own rows only: nothing to publish
     if (!sum_rows<kX, 1, false>(
             gs, ep, xs, wpq, pq, buf, [&] { sh.dv.set(sh.d); }, none,
-            [&](const double *t) { sh.alpha = divide(sh.d, t[0]); }))
+            [&](const double *t) { sh.alpha = quick_quotient(sh.d, t[0]); }))
       return;
     const double alpha = sh.alpha;
     // x += alpha p ; r -= alpha q ; z = r/m ; r.z (and r.r for stop_rule 1)
     double rz[1] = {0.0}, rr2[2] = {0.0, 0.0};
     FOR_ROWS(P) {
-      x[row] = fma(alpha, pcur[row], x[row]);
-      const double ri = fma(-alpha, q[row], r[row]);
+      double &x = X_, &r = R_, &q = Q_;
+      x = fma(alpha, pcur[row], x);
+      const double ri = fma(-alpha, q, r);
       const double zi = ri * minv[row];
-      r[row] = ri;
-      z[row] = zi;
+      r = ri;
+      if (kStoreP)
+        q = zi;
+      else
+        z[row] = zi;
       if (rule0) {
         rz[0] = fma(ri, zi, rz[0]);
       } else {
@@ -297,6 +385,12 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
     status = FVC_ERR_NOCONV;
   }
   finish_to(result, iresult, lead, j, status, sh.conv, root(sh.rr), 0);
+  FOR_ROWS(P) {
+    if (it_ < own.cap) a.x[row] = X_;
+  }
+#undef R_
+#undef Q_
+#undef X_
   if (!grid_barrier(gs, ep)) return;  // x of every row before the epilogue's SpMV
   __shared__ SumWindow<3> we;
   if (threadIdx.x == 0) we.top[0] = kNoWindow;
@@ -341,7 +435,7 @@ __global__ void __launch_bounds__(1024, 1) pcg_f64(KArgs a) {
 template <int kMaxT = 1024, bool kT = false, bool kStoreZ = false, bool kX = true>
 __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, const GridSync &gs,
                                              double *result, int *iresult, bool lead) {
-  __shared__ double buf[3 * kMaxT];
+  __shared__ double buf[kX ? 48 : 3 * kMaxT];
   __shared__ struct {
     double d, conv, rr0, alpha, w, aw, beta, crit2;
     Divisor dv, rv;   // d, and this iteration's s.r
@@ -351,8 +445,16 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
     int fresh;    // this iteration started from r0 = s (the start or a restart)
     int brk;      // r.v = 0 or r.s = 0 in phase 1 (alpha = 0 this iteration)
   } sh;
-  double *r = a.v0, *t = a.v7, *x = a.x;
   double *scur = a.v1, *snxt = a.v2, *pold = a.v3, *pnew = a.v4, *vold = a.v5, *vnew = a.v6;
+  // own: r, t, x, and with the stored z, which alone is gathered, s, p and v
+  // (in one buffer each)
+  const Resident<kStoreZ ? 6 : 3> own(a);
+#define R_ own(0, it_, a.v0, row)
+#define T_ own(1, it_, a.v7, row)
+#define X_ own(2, it_, a.x, row)
+#define S_ own(3, it_, a.v1, row)
+#define P_ own(4, it_, a.v3, row)
+#define V_ own(5, it_, a.v5, row)
   __shared__ ExactState xs;
   __shared__ SumWindow<2> w1, w2;
   __shared__ SumWindow<3> w3;
@@ -364,21 +466,30 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
   Episode ep;
   const NoScalars none;
 
+  FOR_ROWS(P) own.template load<kT>(a.A, s_, it_, P.lane, row);
   // r = b - A x ; p = s = r ; d = r.(r/m)   (x = 0 when init)
   double acc[2] = {0.0, 0.0}, acc3[3];
   FOR_ROWS(P) {
     double ax;
     if (a.init) {
       ax = 0.0;
-      x[row] = 0.0;
+      X_ = 0.0;
     } else {
-      ax = row_fma<kT>(a.A, s_, P.lane, row, [&](int k) { return x[k]; });
+      ax = own.template product<kT>(a.A, s_, it_, P.lane, row, [&](int k) { return a.x[k]; });
+      if (it_ < own.cap) X_ = a.x[row];
     }
     const double ri = b[row] - ax;
-    r[row] = ri;
-    scur[row] = ri;
-    pold[row] = 0.0;  // the first p = s + 0 (0 - 0 v): no case of its own
-    vold[row] = 0.0;
+    R_ = ri;
+    // the first p = s + 0 (0 - 0 v): no case of its own
+    if (kStoreZ) {
+      S_ = ri;
+      P_ = 0.0;
+      V_ = 0.0;
+    } else {
+      scur[row] = ri;
+      pold[row] = 0.0;
+      vold[row] = 0.0;
+    }
     acc[0] = fma(ri, ri * minv[row], acc[0]);
     acc[1] = fma(b[row], b[row], acc[1]);
   }
@@ -404,17 +515,19 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
     if (kStoreZ) {
       double *zp = a.v8;
       FOR_ROWS(P) {
-        if (restart) r[row] = scur[row];
-        const double pi = fma(beta, fma(-w, vold[row], pold[row]), scur[row]);
-        pnew[row] = pi;
+        const double si = S_;
+        double &p = P_;
+        if (restart) R_ = si;
+        const double pi = fma(beta, fma(-w, V_, p), si);
+        p = pi;
         zp[row] = pi * minv[row];
       }
       if (!grid_barrier(gs, ep)) return;
       FOR_ROWS(P) {
-        const double vi = row_fma<kT>(a.A, s_, P.lane, row, [&](int k) { return zp[k]; });
-        vnew[row] = vi;
-        const double ri = r[row];
-        acc[0] = fma(scur[row], ri, acc[0]);
+        const double vi = own.template product<kT>(a.A, s_, it_, P.lane, row, [&](int k) { return zp[k]; });
+        V_ = vi;
+        const double ri = R_;
+        acc[0] = fma(S_, ri, acc[0]);
         acc[1] = fma(vi, ri, acc[1]);
       }
     } else {
@@ -422,13 +535,13 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
         const double *po = pold, *vo = vold, *sc = scur;
         // after a breakdown beta = 0 (p = s) and the shadow residual is s:
         // each row rewrites its own r before it reads it
-        if (restart) r[row] = sc[row];
+        if (restart) R_ = sc[row];
         auto pf = [&](int k) { return fma(beta, fma(-w, vo[k], po[k]), sc[k]); };
         pnew[row] = pf(row);
         const double vi =
-            row_fma<kT>(a.A, s_, P.lane, row, [&](int k) { return pf(k) * minv[k]; });
+            own.template product<kT>(a.A, s_, it_, P.lane, row, [&](int k) { return pf(k) * minv[k]; });
         vnew[row] = vi;
-        const double ri = r[row];
+        const double ri = R_;
         acc[0] = fma(sc[row], ri, acc[0]);
         acc[1] = fma(vi, ri, acc[1]);
       }
@@ -440,7 +553,7 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
     if (!sum_rows<kX, 2, !kStoreZ>(gs, ep, xs, w1, acc, buf, none, none, [&](const double *q) {
           sh.rr0 = q[0];
           sh.brk = (q[0] == 0.0 || q[1] == 0.0) ? 1 : 0;
-          sh.alpha = sh.brk ? 0.0 : divide(q[0], q[1]);
+          sh.alpha = sh.brk ? 0.0 : quick_quotient(q[0], q[1]);
         }))
       return;
     alpha = sh.alpha;
@@ -450,15 +563,16 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
     if (kStoreZ) {
       double *zs = a.v9;
       FOR_ROWS(P) {
-        const double s1 = fma(-alpha, vnew[row], scur[row]);
-        snxt[row] = s1;
+        double &s = S_;
+        const double s1 = fma(-alpha, V_, s);
+        s = s1;
         zs[row] = s1 * minv[row];
       }
       if (!grid_barrier(gs, ep)) return;
       FOR_ROWS(P) {
-        const double ti = row_fma<kT>(a.A, s_, P.lane, row, [&](int k) { return zs[k]; });
-        t[row] = ti;
-        acc[0] = fma(ti, snxt[row], acc[0]);
+        const double ti = own.template product<kT>(a.A, s_, it_, P.lane, row, [&](int k) { return zs[k]; });
+        T_ = ti;
+        acc[0] = fma(ti, S_, acc[0]);
         acc[1] = fma(ti, ti, acc[1]);
       }
     } else {
@@ -467,8 +581,8 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
         auto sf = [&](int k) { return fma(-alpha, vn[k], sc[k]); };
         snxt[row] = sf(row);
         const double ti =
-            row_fma<kT>(a.A, s_, P.lane, row, [&](int k) { return sf(k) * minv[k]; });
-        t[row] = ti;
+            own.template product<kT>(a.A, s_, it_, P.lane, row, [&](int k) { return sf(k) * minv[k]; });
+        T_ = ti;
         acc[0] = fma(ti, snxt[row], acc[0]);
         acc[1] = fma(ti, ti, acc[1]);
       }
@@ -478,7 +592,7 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
     // (phase 3 touches own rows only: nothing to publish)
     if (!sum_rows<kX, 2, false>(
             gs, ep, xs, w2, acc, buf, [&] { sh.rv.set(sh.rr0); }, none,
-            [&](const double *q) { sh.w = (q[1] != 0.0) ? divide(q[0], q[1]) : 0.0; }))
+            [&](const double *q) { sh.w = (q[1] != 0.0) ? quick_quotient(q[0], q[1]) : 0.0; }))
       return;
     w = sh.w;
     // phase 3: x += alpha z ; x += w z' ; s'' = s' - w t ; s''.z' ; r.s'' ; s''.s''
@@ -486,15 +600,16 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
     acc3[1] = 0.0;
     acc3[2] = 0.0;
     FOR_ROWS(P) {
-      const double mi = minv[row];
-      const double s1 = snxt[row];
+      double &x = X_, &s = kStoreZ ? S_ : snxt[row];
+      const double mi = kStoreZ ? 0.0 : minv[row];
+      const double s1 = s;
       const double z1 = kStoreZ ? a.v9[row] : s1 * mi;
-      double xi = fma(alpha, kStoreZ ? a.v8[row] : pnew[row] * mi, x[row]);
-      x[row] = fma(w, z1, xi);
-      const double si = fma(-w, t[row], s1);
-      snxt[row] = si;
+      double xi = fma(alpha, kStoreZ ? a.v8[row] : pnew[row] * mi, x);
+      x = fma(w, z1, xi);
+      const double si = fma(-w, T_, s1);
+      s = si;
       acc3[0] = fma(si, z1, acc3[0]);
-      acc3[1] = fma(r[row], si, acc3[1]);
+      acc3[1] = fma(R_, si, acc3[1]);
       acc3[2] = fma(si, si, acc3[2]);
     }
     auto before3 = [&] { sh.aw = divide(sh.alpha, sh.w); };
@@ -545,6 +660,15 @@ __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, cons
     status = FVC_ERR_NOCONV;
   }
   finish_to(result, iresult, lead, j, status, sh.conv, root(sh.crit2), 0);
+  FOR_ROWS(P) {
+    if (it_ < own.cap) a.x[row] = X_;
+  }
+#undef R_
+#undef T_
+#undef X_
+#undef S_
+#undef P_
+#undef V_
   if (!grid_barrier(gs, ep)) return;  // x of every row before the epilogue's SpMV
   if (threadIdx.x == 0) w3.top[0] = kNoWindow;
   __syncthreads();
@@ -573,7 +697,12 @@ __global__ void __launch_bounds__(1024, 1) bicgstab_f64_z(KArgs a) {
                                   blockIdx.x == 0);
 }
 
-// BiCGSTAB on A^T x = b over A's storage (a.A.mirror set)
+// BiCGSTAB on A^T x = b over A's storage (a.A.mirror set), from kStoreZRows on
+// with the stored z
+__global__ void __launch_bounds__(1024, 1) bicgstab_f64_tz(KArgs a) {
+  bicgstab_run<1024, true, true>(a, Part(a.A.nslices, a.A.n), a.gs, a.result, a.iresult,
+                                 blockIdx.x == 0);
+}
 __global__ void __launch_bounds__(1024, 1) bicgstab_f64_t(KArgs a) {
   bicgstab_run<1024, true>(a, Part(a.A.nslices, a.A.n), a.gs, a.result, a.iresult,
                            blockIdx.x == 0);
@@ -882,6 +1011,17 @@ int32_t ensure_vectors(Scratch &S, size_t n, int nvec, size_t nblocks, bool gmre
   return ensure_sync(S, nblocks);
 }
 
+// Shared memory of a block for what Resident keeps, of the 227 KB; the rest is
+// left to L1 for the gathered vector.  Per iteration on GB300 with nothing
+// kept, the vectors, and the matrix before the vectors: PCG 10k rows 5.9, 5.7,
+// 5.4 us, 66k rows 7.6, 7.5, 7.2, 176k rows 11.7, 11.8, 10.8, 490k rows 21.0,
+// 20.4, 19.4, 1.05M rows 36.3, 36.7, 34.5, 3.2M rows 109, 103, 107; BiCGSTAB
+// 10k rows 11.3, 11.2, 10.4, 176k rows 24.9, 24.2, 22.2, 490k rows 42.2, 40.3,
+// 36.7, 1.05M rows 71.5, 69.3, 65.5, 3.2M rows 236, 222, 229: the vectors first
+// where a thread has more than ten rows.
+constexpr size_t kResidentBytes = 216 * 1024;
+constexpr size_t kMatrixFirst = 10;
+
 // Enqueues one persistent solve on `stream` and returns without waiting:
 // the scratch exists afterwards, so a second call of the same shape makes
 // no allocation and may run inside a stream capture.  launch = false stops
@@ -889,9 +1029,33 @@ int32_t ensure_vectors(Scratch &S, size_t n, int nvec, size_t nblocks, bool gmre
 template <typename K>
 int32_t enqueue_persistent(K kernel, const DeviceMatrix &A, Scratch &S, const double *b,
                            double *x, double tol, int maxit, int init, const fvc_opts &o,
-                           cudaStream_t stream, int nvec, bool gmres, bool launch = true) {
+                           cudaStream_t stream, int nvec, bool gmres, bool launch = true,
+                           int nres = 0) {
   if (A.n <= 0) return FVC_ERR_ARG;
   Launch L = persistent_launch(kernel, A, o);
+  int cap = 0, capm = 0;
+  size_t smem = 0;
+  if (nres > 0 && L.blocks <= sm_count()) {
+    const int spb = (A.nslices + L.blocks - 1) / L.blocks, warps = L.threads / 32;
+    const size_t need = (spb + warps - 1) / warps, vec = (size_t)nres * 8 * L.threads,
+                 mat = (size_t)56 * L.threads;
+    size_t left = kResidentBytes;
+    if (need > kMatrixFirst) {
+      cap = (int)std::min(need, left / vec);
+      left -= cap * vec;
+    }
+    capm = (int)std::min(need, left / mat);
+    left -= capm * mat;
+    if (need <= kMatrixFirst) cap = (int)std::min(need, left / vec);
+    smem = cap * vec + capm * mat;
+    if (smem > 40 * 1024 &&
+        cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem) != cudaSuccess) {
+      cudaGetLastError();
+      cap = capm = 0;
+      smem = 0;
+    }
+  }
   int32_t rc = ensure_vectors(S, (size_t)A.n, nvec, (size_t)L.blocks, gmres);
   if (rc != FVC_OK || !launch) return rc;
   reset_sync(S, stream, (size_t)L.blocks);
@@ -920,9 +1084,11 @@ int32_t enqueue_persistent(K kernel, const DeviceMatrix &A, Scratch &S, const do
   a.stop_rule = o.stop_rule;
   a.result = S.result;
   a.iresult = S.iresult;
+  a.cap = cap;
+  a.capm = capm;
   void *args[] = {&a};
   cudaError_t ce = cudaLaunchCooperativeKernel((const void *)kernel, dim3(L.blocks), dim3(L.threads),
-                                               args, 0, stream);
+                                               args, smem, stream);
   count_launch();
   if (ce != cudaSuccess) {
     fprintf(stderr, "fvcgpu: cooperative launch failed: %s\n", cudaGetErrorString(ce));
@@ -967,13 +1133,13 @@ int32_t read_stats(const Scratch &S, cudaStream_t stream, cudaEvent_t e0, cudaEv
 template <typename K>
 int32_t run_persistent(K kernel, const DeviceMatrix &A, Scratch &S, const double *b, double *x,
                        double tol, int maxit, int init, const fvc_opts &o, cudaStream_t stream,
-                       fvc_stats *st, int nvec, bool gmres) {
+                       fvc_stats *st, int nvec, bool gmres, int nres = 0) {
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaEventRecord(e0, stream);
   const int32_t rc =
-      enqueue_persistent(kernel, A, S, b, x, tol, maxit, init, o, stream, nvec, gmres);
+      enqueue_persistent(kernel, A, S, b, x, tol, maxit, init, o, stream, nvec, gmres, true, nres);
   cudaEventRecord(e1, stream);
   if (rc != FVC_OK) {
     cudaEventDestroy(e0);
@@ -1038,18 +1204,18 @@ int32_t run_pcg(const DeviceMatrix &A, Scratch &S, const double *b, double *x, d
     if (rc != FVC_ERR_UNSUPPORTED) return rc;
   }
   // p stored from 262144 rows on: per iteration on GB300, stored against
-  // formed at every read, 138k rows 10.5 vs 10.0 us, 260k 13.3 vs 13.1, 360k
-  // 17.0 vs 16.7, 1.05M 34.5 vs 38
+  // formed at every read, 66k rows 7.8 vs 7.2 us, 176k 11.1 vs 10.8, 262k 12.7
+  // vs 13.1, 490k 19.3 vs 21.5, 1.05M 34.5 vs 40.1
   if (A.n >= kStorePRows)
-    return run_persistent(pcg_f64<true>, A, S, b, x, tol, maxit, init, o, stream, st, 5, false);
-  return run_persistent(pcg_f64<false>, A, S, b, x, tol, maxit, init, o, stream, st, 5, false);
+    return run_persistent(pcg_f64<true>, A, S, b, x, tol, maxit, init, o, stream, st, 5, false, 3);
+  return run_persistent(pcg_f64<false>, A, S, b, x, tol, maxit, init, o, stream, st, 5, false, 3);
 }
 
 // FP64 BiCGSTAB with z stored once per row from this many rows on (below,
 // the two extra grid barriers cost more than the FP64 they save).  Per
-// iteration, stored against formed at every read: 52.9k rows 16.8 vs 15.9 us,
-// 90k 18.8 vs 19.5, 122k 21.3 vs 23.5, 260k 28.0 vs 35.4
-constexpr int kStoreZRows = 73728;
+// iteration, stored against formed at every read: 10k rows 12.0 vs 10.4 us,
+// 65.5k 15.5 vs 15.7, 90k 16.7 vs 17.8, 176k 22.2 vs 26.0, 262k 25.1 vs 32.8
+constexpr int kStoreZRows = 65536;
 
 // BiCGSTAB on one cluster up to this many rows (a block of 256 threads per
 // eight slices, at most 16 blocks); above, the grid-wide kernel.  Per
@@ -1142,15 +1308,17 @@ int32_t run_bicgstab(const DeviceMatrix &A, Scratch &S, const double *b, double 
     return read_stats(S, stream, e0, e1, true, st);
   }
   if (A.n >= kStoreZRows)
-    return run_persistent(bicgstab_f64_z, A, S, b, x, tol, maxit, init, o, stream, st, 10, false);
-  return run_persistent(bicgstab_f64, A, S, b, x, tol, maxit, init, o, stream, st, 8, false);
+    return run_persistent(bicgstab_f64_z, A, S, b, x, tol, maxit, init, o, stream, st, 10, false, 6);
+  return run_persistent(bicgstab_f64, A, S, b, x, tol, maxit, init, o, stream, st, 8, false, 3);
 }
 
 int32_t run_bicgstab_transposed(const DeviceMatrix &A, Scratch &S, const double *b, double *x,
                                 double tol, int maxit, int init, const fvc_opts &o,
                                 cudaStream_t stream, fvc_stats *st) {
   if (!A.mirror) return FVC_ERR_UNSUPPORTED;
-  return run_persistent(bicgstab_f64_t, A, S, b, x, tol, maxit, init, o, stream, st, 8, false);
+  if (A.n >= kStoreZRows)
+    return run_persistent(bicgstab_f64_tz, A, S, b, x, tol, maxit, init, o, stream, st, 10, false, 6);
+  return run_persistent(bicgstab_f64_t, A, S, b, x, tol, maxit, init, o, stream, st, 8, false, 3);
 }
 
 int32_t run_gmres(const DeviceMatrix &A, Scratch &S, const double *b, double *x, double tol,
@@ -1168,9 +1336,9 @@ int32_t enqueue_solve(const DeviceMatrix &A, Scratch &S, int code, const double 
     }
     if (A.n >= kStorePRows)
       return enqueue_persistent(pcg_f64<true>, A, S, b, x, tol, maxit, init, o, stream, 5, false,
-                                launch);
+                                launch, 3);
     return enqueue_persistent(pcg_f64<false>, A, S, b, x, tol, maxit, init, o, stream, 5, false,
-                              launch);
+                              launch, 3);
   }
   if (code == 2) {
     const int32_t rc = enqueue_bicgstab_cluster(A, S, b, x, tol, maxit, init, o, stream, launch);
@@ -1179,9 +1347,9 @@ int32_t enqueue_solve(const DeviceMatrix &A, Scratch &S, int code, const double 
   if (code == 2)
     return A.n >= kStoreZRows
                ? enqueue_persistent(bicgstab_f64_z, A, S, b, x, tol, maxit, init, o, stream, 10,
-                                    false, launch)
+                                    false, launch, 6)
                : enqueue_persistent(bicgstab_f64, A, S, b, x, tol, maxit, init, o, stream, 8,
-                                    false, launch);
+                                    false, launch, 3);
   if (code == 3)
     return enqueue_persistent(gmres_f64, A, S, b, x, tol, maxit, 1, o, stream, 0, true, launch);
   return FVC_ERR_UNSUPPORTED;
