@@ -279,6 +279,7 @@ struct MArgs {
   // one system of a batch: its slices [grp_s0, grp_s1) over grp_nb blocks
   // from block grp_base (grp_nb = 0: the whole matrix over the grid)
   int grp_s0 = 0, grp_s1 = 0, grp_nb = 0, grp_base = 0;
+  int cap = 0;  // rows per thread of the kept form
 };
 
 // the block that writes the system's results
@@ -1085,13 +1086,137 @@ __device__ __forceinline__ bool f32_refused(const MArgs &a) {
   return true;
 }
 
-template <bool kStaged, int kW, bool kX>
+// ---------------------------------------------------------------------
+// The kept form.  Everything of a row but its matrix row and 1/m lies in its
+// thread's shared memory for the whole solve -- q and z in one place (z from
+// phase B to p, q from A to B), the pairs r, p and e -- so that the two row
+// phases move nothing and q = A p_hi streams the operator and gathers p_hi.
+// p is then formed once per row and published by a barrier, instead of at
+// every read (plain) or once per block and halo row (staged).  The arithmetic
+// and its order are those of the other forms: the deferred e += alpha p of an
+// iteration runs before p changes, with the same factors.
+// What bounds it: 282 instructions per slice and iteration, 7.4 us of issue slots
+// at 1M rows, and the two sums and the barrier, some 9 us.  Per iteration against
+// the staged form (below 524k rows the plain one): 1M rows of quadrilaterals
+// 20.7 and 26.5 us, 980k of triangles 20.2 and 25.8, 490k 13.5 and 14.5, 194k 11.2
+// and 11.5.
+constexpr int kKeptVecs = 7;
+constexpr size_t kKeptBytes = 200 * 1024;  // the rest of the 227 KB: static, L1
+struct Kept {
+  float *base;
+  int cap;
+  __device__ __forceinline__ Kept(unsigned char *smem, const MArgs &a)
+      : base(reinterpret_cast<float *>(smem) + threadIdx.x), cap(a.cap) {}
+  __device__ __forceinline__ float &at(int v, int it) const {
+    return base[(v * cap + it) * blockDim.x];
+  }
+  __device__ __forceinline__ float &qz(int it) const { return at(0, it); }
+  __device__ __forceinline__ float &rs(int it) const { return at(1, it); }
+  __device__ __forceinline__ float &rsl(int it) const { return at(2, it); }
+  __device__ __forceinline__ float &ph(int it) const { return at(3, it); }
+  __device__ __forceinline__ float &pl(int it) const { return at(4, it); }
+  __device__ __forceinline__ float &eh(int it) const { return at(5, it); }
+  __device__ __forceinline__ float &el(int it) const { return at(6, it); }
+};
+
+#define KFOR_ROWS(P)                                                          \
+  _Pragma("unroll 1")                                                         \
+  for (int s_ = (P).sb + (P).warp, it_ = 0; s_ < (P).se; s_ += (P).nwarps, ++it_) \
+    for (int row = s_ * 32 + (P).lane, once_ = 1; once_ && row < (P).n; once_ = 0)
+
+// r and z from the last residual sweep, e = 0 (first: p = 0 too)
+__device__ __forceinline__ void kept_load(const MArgs &a, const MPart &P, const Kept &K,
+                                          bool first) {
+  KFOR_ROWS(P) {
+    K.rs(it_) = a.rs[row];
+    K.rsl(it_) = a.rsl[row];
+    K.qz(it_) = a.z[row];
+    K.eh(it_) = 0.0f;
+    K.el(it_) = 0.0f;
+    if (first) {
+      K.ph(it_) = 0.0f;
+      K.pl(it_) = 0.0f;
+    }
+  }
+}
+// what fold_correction reads
+__device__ __forceinline__ void kept_spill(const MArgs &a, const MPart &P, const Kept &K) {
+  KFOR_ROWS(P) {
+    a.rs[row] = K.rs(it_);
+    a.rsl[row] = K.rsl(it_);
+    a.e[row] = make_float2(K.eh(it_), K.el(it_));
+    a.pal[row] = K.pl(it_);
+  }
+}
+// e += a1 p (kUpdE: the deferred one), p = z + beta p
+template <bool kUpdE>
+__device__ __forceinline__ void kept_p(const MArgs &a, const MPart &P, const Kept &K, float a1,
+                                       float a1_lo, float bh, float bl) {
+  KFOR_ROWS(P) {
+    const float ph = K.ph(it_), pl = K.pl(it_);
+    if (kUpdE) {
+      const float2 e = df_axpy2(make_float2(K.eh(it_), K.el(it_)), a1, a1_lo, ph, pl);
+      K.eh(it_) = e.x;
+      K.el(it_) = e.y;
+    }
+    const float2 p = p_update(K.qz(it_), bh, bl, ph, pl);
+    K.ph(it_) = p.x;
+    K.pl(it_) = p.y;
+    a.pa[row] = p.x;
+  }
+}
+// q = A p_hi, returns p_hi.q
+__device__ __forceinline__ CSum kept_a(const MArgs &a, const MPart &P, const Kept &K) {
+  CSum cpq;
+  int it = 0;
+  const float *ph = a.pa;
+  mfor_rows2(P, [&](const int(&sl)[2], const int(&rw)[2], const bool(&ok)[2]) {
+    float t[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      t[u] = arow32(a, sl[u], P.lane, rw[u], [&](int k) { return ph[k]; });
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (ok[u]) {
+        K.qz(it + u) = t[u];
+        cpq.add(K.ph(it + u) * t[u]);
+      }
+    it += 2;
+  });
+  return cpq;
+}
+// e += alpha p (kUpdE), r -= alpha q, z = r/m; r.z and r.r
+template <bool kUpdE>
+__device__ __forceinline__ void kept_b(const MArgs &a, const MPart &P, const Kept &K, float alpha,
+                                       float alpha_lo, CSum &crz, CSum &crr) {
+  KFOR_ROWS(P) {
+    const float mv = a.minv[row];
+    if (kUpdE) {
+      const float2 e = df_axpy2(make_float2(K.eh(it_), K.el(it_)), alpha, alpha_lo, K.ph(it_),
+                                K.pl(it_));
+      K.eh(it_) = e.x;
+      K.el(it_) = e.y;
+    }
+    float2 none;
+    float ro, rlo, zo;
+    cg_row_b<true, false>(0.0f, 0.0f, alpha, alpha_lo, K.qz(it_), K.rs(it_), K.rsl(it_), mv,
+                          make_float2(0.0f, 0.0f), 0.0f, 0.0f, 0.0f, 0.0f, none, ro, rlo, zo, crz,
+                          crr);
+    K.rs(it_) = ro;
+    K.rsl(it_) = rlo;
+    K.qz(it_) = zo;
+  }
+}
+
+template <bool kStaged, int kW, bool kX, bool kKept = false>
 __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
   __shared__ double red[kMaxNV * 32];
   extern __shared__ __align__(128) unsigned char st_smem[];
   if (f32_refused(a)) return;
   const MPart P(a);
   StCount gch;  // staged copies issued so far, per ring
+  const Kept K(st_smem, a);
+  float ka = 0.0f, ka_lo = 0.0f;  // the last alpha (kept)
   if (kStaged) {
     if (threadIdx.x == 0) {
       StHdr *H = reinterpret_cast<StHdr *>(st_smem);
@@ -1127,6 +1252,7 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
   int it = 0;
   double res[4];
   if (!residual_sweep(a, ep, a.init != 0, res, red)) return;
+  if (kKept) kept_load(a, P, K, true);
   if (threadIdx.x == 0) {
     const double scale = (res[1] > 0.0) ? res[1] : 1.0;
     sh.bnorm2 = res[1];
@@ -1158,11 +1284,18 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
     Dir d;
     d.ph = flip ? a.pa : a.pb;
     d.pl = flip ? a.pal : a.pbl;
-    d.ch = flip ? a.pb : a.pa;
-    d.cl = flip ? a.pbl : a.pal;
+    d.ch = (flip && !kKept) ? a.pb : a.pa;
+    d.cl = (flip && !kKept) ? a.pbl : a.pal;
     // p = z + beta p_prev (an FP32 pair); q = A p_hi; p_hi.q
     CSum pq[1];
-    if (kStaged)
+    if (kKept) {
+      if (pending)
+        kept_p<true>(a, P, K, ka, ka_lo, bh, bl);
+      else
+        kept_p<false>(a, P, K, ka, ka_lo, bh, bl);
+      if (!grid_barrier(a.gs, ep)) return;
+      pq[0] = kept_a(a, P, K);
+    } else if (kStaged)
       pq[0] = (it == 1) ? cg_phase_a_st<true, kW>(a, P, bh, bl, d, st_smem, gch, a_pre)
                         : cg_phase_a_st<false, kW>(a, P, bh, bl, d, st_smem, gch, a_pre);
     else
@@ -1197,7 +1330,14 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
     // rs -= alpha q ; z = rs/m ; rs.z ; rs.rs ; every second iteration also
     // e += a_prev p_prev + alpha p (FP32 pair)
     CSum acc[2];
-    if (kStaged) {
+    if (kKept) {
+      ka = alpha;
+      ka_lo = alpha_lo;
+      if (pending)
+        kept_b<true>(a, P, K, alpha, alpha_lo, acc[0], acc[1]);
+      else
+        kept_b<false>(a, P, K, alpha, alpha_lo, acc[0], acc[1]);
+    } else if (kStaged) {
       if (pending)
         cg_phase_b_st<true, true>(a, P, a1, a1_lo, alpha, alpha_lo, d, acc[0], acc[1], st_smem,
                                   gch, true);
@@ -1215,7 +1355,7 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
       prefetch_a<kW>(a, P, st_smem, gch);
       a_pre = true;
     }
-    if (!grid_sum_ffx<2, true, kX>(a.gs, ep, xs, wrz, acc, red2, tot, none, none, [&](const double *t) {
+    if (!grid_sum_ffx<2, !kKept, kX>(a.gs, ep, xs, wrz, acc, red2, tot, none, none, [&](const double *t) {
           // the alpha*p of an iteration that did not update e is added later
           if (!was_pending) sh.pend_alpha = sh.alpha;
           const double rz_new = t[0];
@@ -1241,12 +1381,14 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
     if (action == kUpdate) {
       // reliable update: fold e (and a deferred alpha p) into x, recompute
       // the true residual in FP64
+      if (kKept) kept_spill(a, P, K);
       fold_correction(a, pending ? d.ch : nullptr, pending ? d.cl : nullptr, sh.pend_alpha);
       pending = false;
       if (!grid_barrier(a.gs, ep) || !residual_sweep(a, ep, false, res, red)) {
         if (a_pre) drain_prefetch_a(P, st_smem, gch);
         return;
       }
+      if (kKept) kept_load(a, P, K, false);
       if (threadIdx.x == 0) {
         const int u = ++sh.updates;
         const double relres = sqrt(res[0] / sh.scale);
@@ -1305,6 +1447,9 @@ __global__ void __launch_bounds__(1024, 1) mixed_cg(MArgs a) { mixed_cg_body<fal
 // the 16-bit column offsets (col16) present; _w3/_w4 when every slice has
 // width 3 / 4 in the padded uniform layout (ell_w; cells of triangle /
 // quadrilateral meshes).
+__global__ void __launch_bounds__(1024, 1) mixed_cg_kept(MArgs a) {
+  mixed_cg_body<false, 0, false, true>(a);
+}
 __global__ void __launch_bounds__(1024, 1) mixed_cg_staged(MArgs a) { mixed_cg_body<true, 0, false>(a); }
 __global__ void __launch_bounds__(1024, 1) mixed_cg_staged_w3(MArgs a) {
   mixed_cg_body<true, 3, false>(a);
@@ -1735,20 +1880,26 @@ int32_t enqueue_mixed(const DeviceMatrix &A0, Scratch &S, int code, const double
   if (rc != FVC_OK) return rc;
   if ((rc = ensure_f32_vectors(S, (size_t)A.n)) != FVC_OK) return rc;
   const int threads = block_threads_for(o.block_threads, A.nslices, sm_count_m());
-  // CG streams through shared-memory stages when its layout allows and
-  // each block owns enough 1024-row chunks to fill the pipeline beside its
-  // +-3-chunk window; below, plain loads are faster (per iteration on
-  // GB300, staged vs plain: 262k rows 16.5 vs 14.1 us, 1.05M 28.9 vs
-  // 28.6 us, 4.19M 87 vs 122 us)
+  // CG keeps its row vectors in shared memory while a block's rows fit (7 per
+  // thread, 1.09M rows on 152 SMs).  Above, it streams through shared-memory
+  // stages when its layout allows and each block owns enough 1024-row chunks
+  // to fill the pipeline beside its +-3-chunk window (per iteration on GB300,
+  // staged vs plain: 4.19M rows 87 vs 122 us; 262k 16.5 vs 14.1)
   const bool staged = code == 1 && threads == kStRows && A.col16_ok &&
                       (o.staging == 2 || (o.staging == 0 && A.n >= kStagedRows));
+  const int spb = (A.nslices + sm_count_m() - 1) / sm_count_m();
+  const int keep = (spb + threads / 32 - 1) / (threads / 32);
+  const bool kept = code == 1 && threads == kStRows && o.staging == 0 && o.max_blocks == 0 &&
+                    (size_t)keep * kKeptVecs * 4 * threads <= kKeptBytes;
   auto kern = (code != 1) ? mixed_bicgstab
+              : kept           ? mixed_cg_kept
               : !staged        ? mixed_cg
               : A.ell_w == 4   ? mixed_cg_staged_w4
               : A.ell_w == 3   ? mixed_cg_staged_w3
                                : mixed_cg_staged;
-  const size_t dsmem = staged ? kStSmem : 0;
-  if (staged) {
+  const size_t dsmem =
+      kept ? (size_t)keep * kKeptVecs * 4 * threads : staged ? kStSmem : 0;
+  if (kept || staged) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem) !=
         cudaSuccess)
       return FVC_ERR_CUDA;
@@ -1769,6 +1920,7 @@ int32_t enqueue_mixed(const DeviceMatrix &A0, Scratch &S, int code, const double
   reset_sync(S, stream, (size_t)blocks);
   MArgs a = mixed_args(A, S, b, x);
   a.rsl = (code == 1) ? S.f[9] : nullptr;
+  a.cap = keep;
   a.gs = make_sync(S, blocks);
   a.target = (o.refine_tol > 0) ? o.refine_tol : tol;
   a.inner_tol = (o.inner_tol > 0) ? o.inner_tol : kInnerTolDefault;
