@@ -1317,7 +1317,7 @@ __device__ __forceinline__ void mixed_cg_body(const MArgs &a) {
         a.history[it - 2] = (float)root(divide(sh.rr, sh.scale));
     };
     if (!grid_sum_ffx<1, false, kX>(a.gs, ep, xs, wpq, pq, red2, tot, before_pq, none, [&](const double *t) {
-          const double alpha_d = divide(sh.rz, t[0]);
+          const double alpha_d = quick_quotient(sh.rz, t[0]);
           sh.alpha = alpha_d;
           sh.alpha_f = (float)alpha_d;
           sh.alpha_lo = (float)(alpha_d - (double)sh.alpha_f);
@@ -1556,7 +1556,7 @@ __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
       // is and restart from an FP64 residual in the next sweep
       if (!grid_sum_ffx<2, false, true>(a.gs, ep, xs, w1, c01, red2, tot, none, none, [&](const double *q) {
             bs.rr0 = q[0];
-            bs.alpha = (float)divide(q[0], q[1]);
+            bs.alpha = (float)quick_quotient(q[0], q[1]);
             bs.go = (isfinite(bs.alpha) && bs.alpha != 0.0f) ? 1 : 0;
           }))
         return;
@@ -1603,7 +1603,7 @@ __device__ __forceinline__ void mixed_bicgstab_body(const MArgs &a) {
       });
       if (!grid_sum_ffx<2, false, true>(a.gs, ep, xs, w2, c23, red2, tot, [&] { bs.rv.set(bs.rr0); },
                                   none, [&](const double *q) {
-            bs.omega = (q[1] > 0.0) ? (float)divide(q[0], q[1]) : 0.0f;
+            bs.omega = (q[1] > 0.0) ? (float)quick_quotient(q[0], q[1]) : 0.0f;
             bs.go = isfinite(bs.omega) ? 1 : 0;
           }))
         return;
