@@ -1118,7 +1118,10 @@ bool mesh_geom_ok(const fvc_cell_mesh *m) {
          m->nelcon && m->num && m->e;
 }
 
-constexpr int kThreads = 128;
+// A warp per block: 20k cells spread over four times the SMs' schedulers (the
+// cell work of 20k cells 223 -> 189 us against blocks of 128; of 200k cells
+// equal).
+constexpr int kThreads = 32;
 inline int grid(int n) { return (n + kThreads - 1) / kThreads; }
 
 }  // namespace
