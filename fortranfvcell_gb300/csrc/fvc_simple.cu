@@ -220,8 +220,8 @@ __device__ void geom(Geom &G, const Stencil &S) {
 // without the cache computes them.  The kernels are bound by the FP64 pipe (one
 // warp instruction per 76 clocks and SM sub-partition): an operation read
 // instead of recomputed saves 0.4 us per 200k cells, its 8 bytes cost 0.24.
-// 200k cells of a mixed mesh, records against this: gradient 116 -> 22 us,
-// momentum 354 -> 298, p' 168 -> 104.
+// 200k cells of a mixed mesh, records against this: gradient 116 -> 21 us,
+// momentum 354 -> 278, p' 168 -> 98.
 enum FaceField : int {
   kN1, kN2,      // unit normal
   kMeta,         // face length
@@ -238,6 +238,7 @@ enum FaceField : int {
   kDxc1, kDxc2,  // own minus the neighbour's centroid
   kDxm1, kDxm2,  // face midpoint minus the neighbour's centroid
   kGn1, kGn2,    // Green-Gauss polygon: normal of side l
+  kRMksi, kRNk, kRNkMksi,  // reciprocals of kMksi, kNk, kNkMksi (quotient)
   kFaceFields
 };
 constexpr int kAreaField = kFaceFields * MS, kGgAreaField = kAreaField + 1;
@@ -275,7 +276,10 @@ __device__ double face_field(const Geom &G, const Stencil &S, int f, int i) {
     case kDxm1: return G.xm[0][i] - G.xc[0][i];
     case kDxm2: return G.xm[1][i] - G.xc[1][i];
     case kGn1: return G.xcg[1][s2] - G.xcg[1][i];
-    default: return -(G.xcg[0][s2] - G.xcg[0][i]);
+    case kGn2: return -(G.xcg[0][s2] - G.xcg[0][i]);
+    case kRMksi: return 1.0 / mk;
+    case kRNk: return 1.0 / (n1 * k1 + n2 * k2);
+    default: return 1.0 / ((n1 * k1 + n2 * k2) * mk);
   }
 }
 __device__ double gg_area(const Geom &G, int ns) {
@@ -283,6 +287,22 @@ __device__ double gg_area(const Geom &G, int ns) {
   for (int i = 0; i < 2; ++i)
     for (int l = 0; l < ns; ++l) eta[i][l] = G.xcg[i][(l + 1) % ns] - G.xcg[i][l];
   return areacell(eta, ns);
+}
+
+// t / d, correctly rounded as the division is, from y = 1 / d (rounded to
+// nearest): one residual step makes t y faithful, the second rounds it to
+// nearest (Markstein's theorem, IBM J. Res. Dev. 34, 1990).  Five FP64
+// instructions, a division has about eleven (200k cells: momentum 298 -> 278 us,
+// p' 104 -> 98).  Outside the middle of the
+// exponents, where a step could underflow, and for zeros: the division.
+__device__ __forceinline__ bool mid_exponent(double v) {
+  return (unsigned)(((__double2hiint(v) >> 20) & 0x7ff) - 623) <= 800u;
+}
+__device__ __forceinline__ double quotient(double t, double d, double y) {
+  if (!mid_exponent(t) || !mid_exponent(d)) return t / d;
+  double q = __dmul_rn(t, y);
+  q = __fma_rn(__fma_rn(-q, d, t), y, q);
+  return __fma_rn(__fma_rn(-q, d, t), y, q);
 }
 
 // A cell as the kernels see it: its sides, its neighbours (1-based; <= 0 a
@@ -314,6 +334,10 @@ struct Cell {
   }
   __device__ __forceinline__ double face(int f, int i) const {
     return kGeo ? __ldg(g + (size_t)(f * MS + i) * pitch) : face_field(G, S, f, i);
+  }
+  // t over face f's field, through its reciprocal field r when that is at hand
+  __device__ __forceinline__ double over(double t, int f, int r, int i) const {
+    return kGeo ? quotient(t, face(f, i), face(r, i)) : t / face(f, i);
   }
   __device__ __forceinline__ double area() const {
     return kGeo ? __ldg(g + kAreaField * pitch) : G.area;
@@ -354,7 +378,7 @@ __global__ void geometry_kernel(Mesh m, double *out) {
 #pragma unroll 1
     for (int f = 0; f < kFaceFields; ++f) {
       // a boundary face has no neighbour: only these are read there
-      const bool bnd = f <= kMeta || f == kDf1 || f == kDf2 || f == kCa || f >= kGn1;
+      const bool bnd = f <= kMeta || f == kDf1 || f == kDf2 || f == kCa || f == kGn1 || f == kGn2;
       o[(size_t)(f * MS + i) * pitch] = (inner || (face && bnd)) ? face_field(G, S, f, i) : 0.0;
     }
   }
@@ -515,6 +539,7 @@ __global__ void __launch_bounds__(128) momentum_kernel(Mesh m, MomArgs a) {
     return;
   }
   const double rhoP = idg ? ro3(ro, 3, nel) : rhoA;  // the cell's current density
+  const double rvisc = 1.0 / viscosity;
   double p = 0.0, pf = 0.0, sp = 0.0, cd = 0.0, cvc = 0.0;
   Four aa;
   const double w1P = v2(w, 1, nel), w2P = v2(w, 2, nel), pP = u0[nel - 1];
@@ -572,7 +597,9 @@ __global__ void __launch_bounds__(128) momentum_kernel(Mesh m, MomArgs a) {
       }
     } else {
       const double alpha = C.face(kAlpha, i - 1), beta = 1.0 - alpha;
-      double kf = alpha / viscosity + beta / prop(m, v, 1);
+      const double viscV = prop(m, v, 1);
+      double kf = quotient(alpha, viscosity, rvisc) +
+                  (viscV == viscosity ? quotient(beta, viscosity, rvisc) : beta / viscV);
       kf = 1.0 / kf;
       const double wf1 = beta * w1P + alpha * v2(w, 1, v);
       const double wf2 = beta * w2P + alpha * v2(w, 2, v);
@@ -580,16 +607,16 @@ __global__ void __launch_bounds__(128) momentum_kernel(Mesh m, MomArgs a) {
       const double gl1 = beta * go1P + alpha * go1V, gl2 = beta * go2P + alpha * go2V;
       double gf1 = gl1, gf2 = gl2;
       const double k1 = C.face(kKsi1, i - 1), k2 = C.face(kKsi2, i - 1);
-      const double mk = C.face(kMksi, i - 1), nk = C.face(kNk, i - 1);
+      const double mk = C.face(kMksi, i - 1);
       const double wfn = wf1 * n1 + wf2 * n2;
       double gfk = gf1 * k1 + gf2 * k2;
-      const double dgk = (uV - uP) / mk - gfk;
+      const double dgk = C.over(uV - uP, kMksi, kRMksi, i - 1) - gfk;
       gf1 = gf1 + dgk * k1;
       gf2 = gf2 + dgk * k2;
       const double gfn = gf1 * n1 + gf2 * n2;
       gfk = gf1 * k1 + gf2 * k2;
-      const double dfd = (kf * meta) / C.face(kNkMksi, i - 1);
-      cd = kf * meta * (gfn - gfk / nk);
+      const double dfd = C.over(kf * meta, kNkMksi, kRNkMksi, i - 1);
+      cd = kf * meta * (gfn - C.over(gfk, kNk, kRNk, i - 1));
       p = p + cd;
       const double rof = idg ? beta * rhoP + alpha * ro3(ro, 3, v) : rhoA;
       const double cv = rof * wfn * meta;
@@ -733,7 +760,7 @@ __global__ void __launch_bounds__(128) pc_kernel(Mesh m, PcArgs a) {
         const double dd1 = ddf[0] * n1, dd2 = ddf[1] * n2;
         ndd = dd1 * n1 + dd2 * n2;
       }
-      la.set(i - 1, (kf * C.face(kMeta, i - 1) * ndd) / C.face(kNkMksi, i - 1));
+      la.set(i - 1, C.over(kf * C.face(kMeta, i - 1) * ndd, kNkMksi, kRNkMksi, i - 1));
       const double wfn = cell_vel(a.intvel, w, a.gradp, ddf, C, a.p, nel, v, i, alpha);
       pp = pp - kf * wfn;
     }
@@ -836,7 +863,7 @@ __global__ void __launch_bounds__(128) pc_idg_kernel(Mesh m, PcIdgArgs a) {
         const double dd1 = ddf[0] * n1, dd2 = ddf[1] * n2;
         ndd = dd1 * n1 + dd2 * n2;
       }
-      la.set(i - 1, (kf * C.face(kMeta, i - 1) * ndd) / C.face(kNkMksi, i - 1));
+      la.set(i - 1, C.over(kf * C.face(kMeta, i - 1) * ndd, kNkMksi, kRNkMksi, i - 1));
       const double wfn = cell_vel(a.intvel, w, a.gradp, ddf, C, a.p, nel, v, i, alpha);
       pp = pp - kf * wfn;
     }
@@ -1036,16 +1063,16 @@ __global__ void __launch_bounds__(128) energy_kernel(Mesh m, EnArgs a) {
       double gf1 = (1.0 - alpha) * v2(grad, 1, nel) + alpha * v2(grad, 1, v);
       double gf2 = (1.0 - alpha) * v2(grad, 2, nel) + alpha * v2(grad, 2, v);
       const double k1 = C.face(kKsi1, i - 1), k2 = C.face(kKsi2, i - 1);
-      const double mk = C.face(kMksi, i - 1), nk = C.face(kNk, i - 1);
+      const double mk = C.face(kMksi, i - 1);
       const double wfn = wf1 * n1 + wf2 * n2;
       const double uv = u[v - 1];
       double gfk = gf1 * k1 + gf2 * k2;
-      gf1 = gf1 + ((uv - uP) / mk - gfk) * k1;
-      gf2 = gf2 + ((uv - uP) / mk - gfk) * k2;
+      gf1 = gf1 + (C.over(uv - uP, kMksi, kRMksi, i - 1) - gfk) * k1;
+      gf2 = gf2 + (C.over(uv - uP, kMksi, kRMksi, i - 1) - gfk) * k2;
       const double gfn = gf1 * n1 + gf2 * n2;
       gfk = gf1 * k1 + gf2 * k2;
-      const double dfd = (kf * meta) / C.face(kNkMksi, i - 1);
-      cd = kf * meta * (gfn - gfk / nk);
+      const double dfd = C.over(kf * meta, kNkMksi, kRNkMksi, i - 1);
+      cd = kf * meta * (gfn - C.over(gfk, kNk, kRNk, i - 1));
       p = p + cd;
       if (lib == 3) {
         rof = (1.0 - alpha) * ro3(ro, 3, nel) + alpha * ro3(ro, 3, v);

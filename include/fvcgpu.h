@@ -99,12 +99,14 @@ typedef struct {
   int32_t update_beta; /* MIXED CG: beta = (r.z)/(r_old.z_old) at a residual
                           replacement taken from 0: the replaced (true)
                           residual; 1: the recursive one                 */
-  int32_t staging;     /* MIXED CG: 0 streams the iteration's arrays through
-                          shared memory with bulk asynchronous copies when
-                          the layout allows (1024 threads, 16-bit column
-                          offsets) and the system has 524288 rows or more;
-                          1: plain loads; 2: staged whenever the layout
-                          allows                                           */
+  int32_t staging;     /* MIXED CG: 0 keeps the row vectors in shared memory
+                          while a block's fit (1024 threads, at most 7 rows
+                          per thread, no max_blocks), else streams the
+                          iteration's arrays through shared memory with bulk
+                          asynchronous copies when the layout allows (1024
+                          threads, 16-bit column offsets) and the system has
+                          524288 rows or more; 1: plain loads; 2: staged
+                          whenever the layout allows                       */
   int32_t max_blocks;  /* cap on the persistent grid (0 -> automatic)      */
   int32_t fp32_layout; /* MIXED: the FP32 operator's slice widths.  0: when
                           no row has more than 4 off-diagonals, every slice
@@ -453,7 +455,7 @@ typedef struct {
 
 /* The geometry of every cell of m (centroids, face normals, lengths and
  * midpoints, ghost centroids, the reference's cellGeom2D / vectorKm2d
- * quantities) computed once into a DEVICE buffer (*geometry, 756 bytes per
+ * quantities) computed once into a DEVICE buffer (*geometry, 852 bytes per
  * cell), for fvc_cell_mesh.geometry.  It depends only on coor, ix and
  * nelcon, which must hold their values when it is called (it runs on the
  * default stream and waits for the device).  Free it with
