@@ -18,8 +18,8 @@
 // Jacobi division r/m is a multiplication by 1/m computed once per matrix.
 // GB300 executes FP64 at ~1/64 of its FP32 rate, and these two changes
 // roughly halve the FP64 instructions per row; they move results only at
-// rounding level, like the dot products, which are tree sums in a fixed
-// (deterministic) order instead of the reference's sequential sums.
+// rounding level, like the dot products, which are exact integer sums
+// (exact_sum) instead of the reference's sequential sums.
 // BiCGSTAB adds one thing the reference lacks: where one of its
 // denominators is exactly zero (the reference goes on with Inf/NaN), the
 // recurrence restarts from the current residual, or the solve ends with
