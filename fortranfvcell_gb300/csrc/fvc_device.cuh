@@ -599,8 +599,8 @@ struct NoScalars {
 // and the blocks into one 64-bit word per limb with relaxed atomics.
 // Integer addition is associative, so the total does not depend on the
 // order: deterministic, and exact but for the bits below the window (less
-// than 2^-53.7 of the total, see sum_bad) and the limbs' addition in FP64.  The word's upper bits count the
-// blocks that have added, so that one poll of the words is the whole
+// than 2^-53.7 of the total, see sum_bad), rounded once.  The word's upper bits
+// count the blocks that have added, so that one poll of the words is the whole
 // exchange: no slots, no counter, no order between them.  The words only
 // grow; a total is the difference to their value one use earlier (snap).
 //
@@ -708,15 +708,24 @@ __device__ __forceinline__ void put_limbs(float s, float c, int top, int *acc) {
   warp_limbs(l, ovf, acc);
 }
 
-// L 2^(21 k) units of the window in FP64, rounded once, unless it leaves
-// FP64's exponents (then 0 or Inf).
-__device__ __forceinline__ double limb_value(long long L, int k, int top) {
-  const double v = (double)L;
-  const int hi = __double2hiint(v), sh = top - kWindowBits + kLimbBits * k;
-  const int e = ((hi >> 20) & 0x7ff) + sh;
-  if (L == 0 || e <= 0) return 0.0;
-  if (e >= 0x7ff) return __hiloint2double((hi & 0x80000000) | 0x7ff00000, 0);
-  return __hiloint2double(hi + (sh << 20), __double2loint(v));
+// T units of the window (its top) in FP64, rounded to nearest even; 0 or Inf
+// where it leaves FP64's exponents.  All in integers: a conversion and an FP64
+// addition are 60 clocks and more of the sum's critical path each.
+__device__ __forceinline__ double window_value(__int128 T, int top) {
+  const bool neg = T < 0;
+  const unsigned __int128 U = neg ? -(unsigned __int128)T : (unsigned __int128)T;
+  const unsigned long long h = (unsigned long long)(U >> 64), l = (unsigned long long)U;
+  const unsigned long long a = h ? h : l, b = h ? l : 0;
+  const int z = __clzll((long long)a);
+  const unsigned long long m = (a << z) | ((b >> 1) >> (63 - z)), rest = b << z;
+  const unsigned int rem = (unsigned int)m & 0x7ffu;
+  unsigned long long r = m >> 11;
+  r += (rem > 0x400u || (rem == 0x400u && (rest != 0 || (r & 1)))) ? 1 : 0;
+  const int e = top - kWindowBits + (h ? 127 : 63) - z + 1023;
+  unsigned long long v = ((unsigned long long)(e - 1) << 52) + r;
+  if (e >= 0x7ff) v = 0x7ff0000000000000ull;
+  if (a == 0 || e <= 0) v = 0;
+  return __longlong_as_double((long long)(v | ((unsigned long long)neg << 63)));
 }
 // Whether a total lies so low in its window that what the threads dropped
 // below it (up to 2^18.3 threads, less than one unit each) could matter:
@@ -734,9 +743,10 @@ __device__ __forceinline__ void exact_init(ExactState &xs) {  // a __syncthreads
   }
 }
 
-// The top of a window that holds partials of biased exponents up to m
+// The top of a window that holds partials of biased exponents up to m and the
+// sum of 2^19 of them
 __device__ __forceinline__ int top_of_partials(int m) {
-  return max(min(m, 0x7fe), 1) - 1022 + 1;
+  return max(min(m, 0x7fe), 1) - 1022 + 1 + 19;
 }
 
 // The window of a sum from its partials: its top above the largest exponent
@@ -798,11 +808,10 @@ __device__ __forceinline__ long long block_limbs(int *acc) {
   const bool o = __any_sync(0xffffffffu, (lane & 7) == kLimbs && w != 0);
   return ((lane & 7) < kLimbs ? w : 0) + ((long long)(o ? 1 : 0) << 42);
 }
-// Then, from the limbs of all blocks (L) and whether any overflowed (bad), the
-// totals t (in every lane) and the verdict: 0 a wait exceeded its bound, 1
-// good, 2 the window did not hold it (never where it follows from the
-// partials, sure).  Two limbs are added as integers (|L| < 2^41), the three
-// pairs in FP64.
+// Then, from the limbs of all blocks (L, |L| < 2^41) and whether any overflowed
+// (bad), the totals t (in every lane), each rounded once, and the verdict: 0 a
+// wait exceeded its bound, 1 good, 2 the window did not hold it (never where
+// it follows from the partials, sure: it has room for the sum of all threads).
 template <int NV>
 __device__ __forceinline__ int limb_totals(long long L, bool bad, bool ok, bool sure,
                                            const SumWindow<NV> &win, const ExactState &xs,
@@ -810,16 +819,19 @@ __device__ __forceinline__ int limb_totals(long long L, bool bad, bool ok, bool 
   const int lane = threadIdx.x & 31, lq = lane >> 3, lk = lane & 7;
   const bool mine = lq < NV && lk < kLimbs;
   const int top = win.top[lq < NV ? lq : 0];
-  if (!mine) L = 0;
   L += __shfl_down_sync(0xffffffffu, L, 1) << kLimbBits;
-  double tq = (lk & 1) ? 0.0 : limb_value(L, lk, top);
-#pragma unroll
-  for (int k = 2; k < 8; k <<= 1) tq = __dadd_rn(tq, __shfl_xor_sync(0xffffffffu, tq, k));
+  const int l0 = lane & 24;
+  const long long p0 = __shfl_sync(0xffffffffu, L, l0);
+  const long long p1 = __shfl_sync(0xffffffffu, L, l0 + 2);
+  const long long p2 = __shfl_sync(0xffffffffu, L, l0 + 4);
+  double tq = window_value(
+      (__int128)p0 + ((__int128)p1 << (2 * kLimbBits)) + ((__int128)p2 << (4 * kLimbBits)), top);
   if (sure) {
     bad = false;  // only NaN and Inf overflow such a window
     if (xs.nan) tq = __longlong_as_double(0x7ff8000000000000ll);
-  } else {
-    bad = mine && (bad || ((lk & 1) == 0 && sum_bad(tq, top)));
+  } else {  // (2^42 of the highest pair: the next doubling leaves 128 bits)
+    bad = mine && (bad || sum_bad(tq, top) ||
+                   (unsigned long long)(p2 + (1ll << 42)) >= (1ull << 43));
   }
   bad = __any_sync(0xffffffffu, bad);
   ok = __all_sync(0xffffffffu, ok);
