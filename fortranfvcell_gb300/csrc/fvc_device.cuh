@@ -390,10 +390,15 @@ __device__ __forceinline__ void cluster_sync_mid(M &&mid) {
 // carries that (release arrival and acquire wait of warp 2), beside the
 // partials and not before them: its wait for the block's stores hides in the
 // sum's two trips to L2.  tot: shared memory for cap partials of each quantity.
-template <int NV, bool kPublish, typename S, typename M, typename F>
+// overlap(): work of the warps that take no part, while the others wait.
+struct NoOverlap {
+  __device__ void operator()() const {}
+};
+template <int NV, bool kPublish, typename S, typename M, typename F, typename O = NoOverlap>
 __device__ __forceinline__ bool exchange_totals(const GridSync &gs, Episode &episode,
                                                 const double (&bsum)[NV], double *tot,
-                                                unsigned int cap, S &&side, M &&mid, F &&f) {
+                                                unsigned int cap, S &&side, M &&mid, F &&f,
+                                                O &&overlap = O()) {
   __shared__ int s_ok[2];
   __shared__ double s_t[NV];
   if (kPublish) ++episode.pub;
@@ -404,6 +409,8 @@ __device__ __forceinline__ bool exchange_totals(const GridSync &gs, Episode &epi
       f(bsum);
     } else if (threadIdx.x == 32) {
       side();
+    } else if (threadIdx.x >= 96) {
+      overlap();
     }
     __syncthreads();
     return true;
@@ -422,6 +429,8 @@ __device__ __forceinline__ bool exchange_totals(const GridSync &gs, Episode &epi
     if (threadIdx.x == 64) red_add_release(gs.count + 8, 1u);
     const bool ok = wait_count<true>(gs.count + 8, gs.err, episode.pub * nb);
     if (threadIdx.x == 64) s_ok[1] = ok ? 1 : 0;
+  } else if (threadIdx.x >= 96) {
+    overlap();
   }
   __syncthreads();
   if (!s_ok[0] || (kPublish && !s_ok[1])) return false;
@@ -459,22 +468,14 @@ __device__ __forceinline__ bool exchange_totals(const GridSync &gs, Episode &epi
   return true;
 }
 
-// Deterministic sum of NV FP64 values per thread over one cluster (or one
-// block) in a fixed order, which the cluster BiCGSTAB keeps (see
-// Scratch::ordered): four warps add blockDim / 128 values per lane (buf: NV x
-// blockDim doubles; blockDim.x a multiple of 128), warp 0 adds the four per
-// lane and finishes with a shuffle tree, the CTAs follow in rank order
-// (cluster_exchange).  Thread 0 then calls f(totals) -- the place for the
-// iteration's scalar FP64 work -- and one __syncthreads hands its results
-// (through shared memory) to the block.  Scalar work that needs nothing of
-// this sum (a division is 570 clocks) hides in the wait: thread 0 calls mid()
-// between its arrival and its wait, for values f uses; thread 32 calls side(),
-// for values of later phases.
-template <int NV, typename S, typename M, typename F>
-__device__ __forceinline__ void ordered_sum(const GridSync &gs, Episode &episode,
-                                            const double (&v)[NV], double *buf, S &&side, M &&mid,
-                                            F &&f) {
-  __shared__ double s_part[NV][128], s_slot[2][kMaxNV];
+// A block's sum of NV FP64 values per thread in a fixed order, in lane 0 of warp
+// 0: four warps add blockDim / 128 values per lane (buf: NV x blockDim doubles;
+// blockDim.x a multiple of 128), warp 0 adds the four per lane and finishes with
+// a shuffle tree.
+template <int NV>
+__device__ __forceinline__ void ordered_block_sum(const double (&v)[NV], double *buf,
+                                                  double (&t)[NV]) {
+  __shared__ double s_part[NV][128];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int bd = blockDim.x, per = bd >> 7;  // values per lane of the first level
 #pragma unroll
@@ -490,8 +491,6 @@ __device__ __forceinline__ void ordered_sum(const GridSync &gs, Episode &episode
     }
   }
   __syncthreads();
-  const unsigned int ep = ++episode.n;
-  double t[NV];
   if (warp == 0)
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
@@ -499,8 +498,29 @@ __device__ __forceinline__ void ordered_sum(const GridSync &gs, Episode &episode
 #pragma unroll
       for (int k = 1; k < 4; ++k) u = __dadd_rn(u, s_part[q][32 * k + lane]);
       t[q] = warp_sum(u);
-      if (lane == 0) s_slot[ep & 1u][q] = t[q];
     }
+}
+
+// Sums in that order: over one cluster or block, the CTAs following in rank
+// order (the cluster BiCGSTAB, see Scratch::ordered), or over a grid, the blocks
+// in block order (exchange_totals; the PCG of kOrderedRows rows and more).
+// Thread 0 then calls f(totals) -- the place for the iteration's scalar FP64
+// work -- and one __syncthreads hands its results (through shared memory) to
+// the block.  Scalar work that needs nothing of this sum (a division is 570
+// clocks) hides in the wait: thread 0 calls mid() between its arrival and its
+// wait, for values f uses; thread 32 calls side(), for values of later phases;
+// over a grid the warps from the fourth on run overlap().
+template <int NV, typename S, typename M, typename F>
+__device__ __forceinline__ void ordered_sum(const GridSync &gs, Episode &episode,
+                                            const double (&v)[NV], double *buf, S &&side, M &&mid,
+                                            F &&f) {
+  __shared__ double s_slot[2][kMaxNV];
+  double t[NV];
+  ordered_block_sum<NV>(v, buf, t);
+  const unsigned int ep = ++episode.n;
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) s_slot[ep & 1u][q] = t[q];
   if (threadIdx.x == 32) side();
   __syncwarp();
   if (gs.cluster) {
@@ -511,6 +531,14 @@ __device__ __forceinline__ void ordered_sum(const GridSync &gs, Episode &episode
   }
   if (threadIdx.x == 0) f(t);
   __syncthreads();
+}
+template <int NV, bool kPublish, typename S, typename M, typename F, typename O>
+__device__ __forceinline__ bool ordered_grid_sum(const GridSync &gs, Episode &episode,
+                                                 const double (&v)[NV], double *buf, S &&side,
+                                                 M &&mid, F &&f, O &&overlap) {
+  double t[NV];
+  ordered_block_sum<NV>(v, buf, t);
+  return exchange_totals<NV, kPublish>(gs, episode, t, buf, blockDim.x, side, mid, f, overlap);
 }
 
 // ---- scalar work of the recurrences ---------------------------------------
@@ -895,12 +923,14 @@ __device__ __forceinline__ void join_warps01() {
 // the limbs of the warp's values of quantity q (put_limbs), expo(q) gives the
 // value's biased FP64 exponent.  part: shared memory for NV * 32 ints.  win: the window of this kind of sum.  Thread 0 calls f(totals) as in
 // ordered_sum; thread 32 calls side() while warp 0 exchanges (kJoin: for values
-// f uses).  kPublish: as in exchange_totals.  Returns false when a wait
+// f uses); the warps from the fourth on run overlap() meanwhile.  kPublish: as
+// in exchange_totals.  Returns false when a wait
 // exceeded its bound (gs.err set).
-template <int NV, bool kPublish, bool kJoin, typename C, typename X, typename S, typename F>
+template <int NV, bool kPublish, bool kJoin, typename C, typename X, typename S, typename F,
+          typename O = NoScalars>
 __device__ __forceinline__ bool exact_sum(const GridSync &gs, Episode &episode, ExactState &xs,
                                           SumWindow<NV> &win, int *part, C &&put, X &&expo,
-                                          S &&side, F &&f) {
+                                          S &&side, F &&f, O &&overlap = O()) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (kPublish) ++episode.pub;
   bool first = true, have = true;
@@ -939,6 +969,8 @@ __device__ __forceinline__ bool exact_sum(const GridSync &gs, Episode &episode, 
         ok = wait_count<true>(gs.count + 8, gs.err, episode.pub * gs.nblocks);
       }
       if (lane == 0) xs.pub_ok = ok ? 1 : 0;
+    } else if (warp >= 3 && first) {
+      overlap();
     }
     __syncthreads();
     if (kPublish && !xs.pub_ok) return false;
@@ -950,14 +982,14 @@ __device__ __forceinline__ bool exact_sum(const GridSync &gs, Episode &episode, 
 }
 
 // exact_sum of FP64 partials; buf: NV x blockDim doubles of shared memory.
-template <int NV, bool kPublish, bool kJoin, typename S, typename F>
+template <int NV, bool kPublish, bool kJoin, typename S, typename F, typename O = NoScalars>
 __device__ __forceinline__ bool grid_sum_x(const GridSync &gs, Episode &episode, ExactState &xs,
                                            SumWindow<NV> &win, const double (&v)[NV], double *buf,
-                                           S &&side, F &&f) {
+                                           S &&side, F &&f, O &&overlap = O()) {
   return exact_sum<NV, kPublish, kJoin>(
       gs, episode, xs, win, reinterpret_cast<int *>(buf),
       [&](int q, int top, int *acc) { put_limbs(v[q], top, acc); },
-      [&](int q) { return (__double2hiint(v[q]) >> 20) & 0x7ff; }, side, f);
+      [&](int q) { return (__double2hiint(v[q]) >> 20) & 0x7ff; }, side, f, overlap);
 }
 
 // Streaming loads of read-only matrix data (never written by the kernel

@@ -102,6 +102,10 @@ struct Resident {
   __device__ __forceinline__ double &operator()(int vec, int it, double *g, int row) const {
     return it < cap ? resident_smem[(vec * cap + it) * blockDim.x + threadIdx.x] : g[row];
   }
+  // ... at the it-th row of thread tid
+  __device__ __forceinline__ double &of(int vec, int it, int tid, double *g, int row) const {
+    return it < cap ? resident_smem[(vec * cap + it) * blockDim.x + tid] : g[row];
+  }
   // entry k of the it-th row: its value (k = 4: the diagonal) and column
   __device__ __forceinline__ double &val(int k, int it) const {
     return resident_smem[(kVec * cap + k * capm + it) * blockDim.x + threadIdx.x];
@@ -178,20 +182,25 @@ __device__ __forceinline__ void finish(const KArgs &a, int iters, int status,
   finish_to(a.result, a.iresult, blockIdx.x == 0, iters, status, conv, crit, inner);
 }
 
-// The sums of the solver bodies: exact ones (kX), or ordered_sum's (the
-// cluster BiCGSTAB).
+// The sums of the solver bodies: exact ones (kSumExact), in a fixed order over
+// one cluster (kSumCluster: the cluster BiCGSTAB) or over the grid (kSumGrid: the
+// PCG of kOrderedRows rows and more).
 // side: scalars of later phases, mid: scalars f uses (thread 0 or 32).
-template <bool kX, int NV, bool kPublish, typename S, typename M, typename F>
+enum Sums { kSumCluster = 0, kSumExact = 1, kSumGrid = 2 };
+template <int kX, int NV, bool kPublish, typename S, typename M, typename F,
+          typename O = NoScalars>
 __device__ __forceinline__ bool sum_rows(const GridSync &gs, Episode &ep, ExactState &xs,
                                          SumWindow<NV> &win, const double (&v)[NV], double *buf,
-                                         S &&side, M &&mid, F &&f) {
+                                         S &&side, M &&mid, F &&f, O &&overlap = O()) {
   constexpr bool kMid = !std::is_same<std::decay_t<M>, NoScalars>::value;
-  if (!kX) {
+  if (kX == kSumCluster) {
     ordered_sum<NV>(gs, ep, v, buf, side, mid, f);
     return true;
   }
+  if (kX == kSumGrid)
+    return ordered_grid_sum<NV, kPublish>(gs, ep, v, buf, side, mid, f, overlap);
   if (kMid) return grid_sum_x<NV, kPublish, true>(gs, ep, xs, win, v, buf, mid, f);
-  return grid_sum_x<NV, kPublish, false>(gs, ep, xs, win, v, buf, side, f);
+  return grid_sum_x<NV, kPublish, false>(gs, ep, xs, win, v, buf, side, f, overlap);
 }
 
 // Energy norm x.Ax and the FP64 residual ||b-Ax||^2, ||b||^2 in one pass
@@ -234,10 +243,11 @@ __device__ __forceinline__ void epilogue_to(const KArgs &a, const Part &P, doubl
 // and z, which saves the barrier.  Both give the same bits.
 // kMaxT: the most threads per block the kernel is launched with (the
 // reductions' staging buffer holds that many values per reduced quantity).
-template <bool kStoreP, int kMaxT = 1024, bool kX = true>
+template <bool kStoreP, int kMaxT = 1024, int kX = kSumExact>
 __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const GridSync &gs,
                                         double *result, int *iresult, bool lead) {
-  __shared__ double buf[48];  // (window_by_partials: 3 x 32 ints)
+  // exact: window_by_partials' 3 x 32 ints; ordered: a value per thread and quantity
+  __shared__ double buf[kX == kSumExact ? 48 : 3 * kMaxT];
   // scalars of the recurrence, updated by lane 0 of warp 0 inside the
   // all-reduces and read by every thread after them
   __shared__ struct {
@@ -263,6 +273,10 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
   const NoScalars none;
   const double *minv = a.minv, *b = a.b;
   const bool rule0 = a.stop_rule == 0;
+  // x += alpha p under the r.z sum (below): not in a batch, whose small blocks
+  // have one warp for it, nor with more than ten rows per thread (3.2M rows: 103
+  // us per iteration without, 107 with)
+  const bool late_x = kMaxT >= 1024 && P.se - P.sb <= 10 * P.nwarps;
   Episode ep;
 
   FOR_ROWS(P) own.load<false>(a.A, s_, it_, P.lane, row);
@@ -335,11 +349,11 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
             [&](const double *t) { sh.alpha = quick_quotient(sh.d, t[0]); }))
       return;
     const double alpha = sh.alpha;
-    // x += alpha p ; r -= alpha q ; z = r/m ; r.z (and r.r for stop_rule 1)
+    // r -= alpha q ; z = r/m ; r.z (and r.r for stop_rule 1)
     double rz[1] = {0.0}, rr2[2] = {0.0, 0.0};
     FOR_ROWS(P) {
-      double &x = X_, &r = R_, &q = Q_;
-      x = fma(alpha, pcur[row], x);
+      if (!late_x) X_ = fma(alpha, pcur[row], X_);
+      double &r = R_, &q = Q_;
       const double ri = fma(-alpha, q, r);
       const double zi = ri * minv[row];
       r = ri;
@@ -366,8 +380,26 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
                 : sqrt_below(crit2, sh.conv, sh.bound)        ? 1
                                                               : 0;
     };
-    const bool ok = rule0 ? sum_rows<kX, 1, !kStoreP>(gs, ep, xs, wrz, rz, buf, none, none, step)
-                          : sum_rows<kX, 2, !kStoreP>(gs, ep, xs, wrr, rr2, buf, none, none, step);
+    // x += alpha p needs nothing of the sum: the warps that do not exchange run
+    // it meanwhile, each over its share of the block's rows (per iteration 66k
+    // rows 7.23 -> 7.06 us, 490k 19.3 -> 18.3, 1.05M 34.5 -> 33.7)
+    auto update_x = [&] {
+      if (!late_x) return;
+      int w = P.warp - 3, it = 0;
+      for (int sl = w; sl < P.se - P.sb; sl += P.nwarps - 3, w += P.nwarps - 3) {
+        while (w >= P.nwarps) {
+          w -= P.nwarps;
+          ++it;
+        }
+        const int row = (P.sb + sl) * 32 + P.lane;
+        if (row < P.n) {
+          double &x = own.of(2, it, 32 * w + P.lane, a.x, row);
+          x = fma(alpha, pcur[row], x);
+        }
+      }
+    };
+    const bool ok = rule0 ? sum_rows<kX, 1, !kStoreP>(gs, ep, xs, wrz, rz, buf, none, none, step, update_x)
+                          : sum_rows<kX, 2, !kStoreP>(gs, ep, xs, wrr, rr2, buf, none, none, step, update_x);
     if (!ok) return;
     if (sh.stop == 2) {
       status = FVC_ERR_NAN;
@@ -401,10 +433,19 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
 }
 
 constexpr int kStorePRows = 262144;
+// The CG's sums keep a fixed FP64 order from this many rows on.  The last bits
+// of its sums move the residual history of a solve of thousands of iterations
+// by parts in 1000, and with it the iteration that meets the tolerance: at 1.05M
+// rows and a tolerance of 1e-8 exact sums moved the solution by 3e-11 to 2e-9 (8
+// right-hand sides; its error is 1e-7), at 512k rows and 1e-9 by 3e-11, at 66k
+// rows by 1e-12.  In order, it stays the same bit for bit; per iteration at
+// 1.05M rows 36.9 us against 33.7 with exact sums, at 262k 15.2 against 12.2.
+constexpr int kOrderedRows = 524288;
 
-template <bool kStoreP>
+template <bool kStoreP, int kSums>
 __global__ void __launch_bounds__(1024, 1) pcg_f64(KArgs a) {
-  pcg_run<kStoreP>(a, Part(a.A.nslices, a.A.n), a.gs, a.result, a.iresult, blockIdx.x == 0);
+  pcg_run<kStoreP, 1024, kSums>(a, Part(a.A.nslices, a.A.n), a.gs, a.result, a.iresult,
+                                blockIdx.x == 0);
 }
 
 
@@ -432,10 +473,10 @@ __global__ void __launch_bounds__(1024, 1) pcg_f64(KArgs a) {
 // them -- five synchronisations per iteration instead of three, about half
 // the FP64 instructions (a gathered neighbour costs one FMA instead of
 // three or two), the same bits.
-template <int kMaxT = 1024, bool kT = false, bool kStoreZ = false, bool kX = true>
+template <int kMaxT = 1024, bool kT = false, bool kStoreZ = false, int kX = kSumExact>
 __device__ __forceinline__ void bicgstab_run(const KArgs &a, const Part &P, const GridSync &gs,
                                              double *result, int *iresult, bool lead) {
-  __shared__ double buf[kX ? 48 : 3 * kMaxT];
+  __shared__ double buf[kX == kSumExact ? 48 : 3 * kMaxT];
   __shared__ struct {
     double d, conv, rr0, alpha, w, aw, beta, crit2;
     Divisor dv, rv;   // d, and this iteration's s.r
@@ -685,7 +726,7 @@ __global__ void __launch_bounds__(1024, 1) bicgstab_f64(KArgs a) {
 // reductions and barriers through the cluster (GridSync.cluster), its
 // vectors in global memory (L2-resident at these sizes)
 __global__ void __launch_bounds__(256, 1) bicgstab_cl(KArgs a) {
-  bicgstab_run<256, false, false, false>(a, Part(a.A.nslices, a.A.n), a.gs, a.result, a.iresult, blockIdx.x == 0);
+  bicgstab_run<256, false, false, kSumCluster>(a, Part(a.A.nslices, a.A.n), a.gs, a.result, a.iresult, blockIdx.x == 0);
   cluster_close(a.gs);
 }
 
@@ -1011,15 +1052,16 @@ int32_t ensure_vectors(Scratch &S, size_t n, int nvec, size_t nblocks, bool gmre
   return ensure_sync(S, nblocks);
 }
 
-// Shared memory of a block for what Resident keeps, of the 227 KB; the rest is
-// left to L1 for the gathered vector.  Per iteration on GB300 with nothing
+// Shared memory of a block for what Resident keeps, of the 227 KB, beside up to
+// 31 KB of a kernel's own; the rest is left to L1 for the gathered vector.  Per
+// iteration on GB300 with nothing
 // kept, the vectors, and the matrix before the vectors: PCG 10k rows 5.9, 5.7,
 // 5.4 us, 66k rows 7.6, 7.5, 7.2, 176k rows 11.7, 11.8, 10.8, 490k rows 21.0,
 // 20.4, 19.4, 1.05M rows 36.3, 36.7, 34.5, 3.2M rows 109, 103, 107; BiCGSTAB
 // 10k rows 11.3, 11.2, 10.4, 176k rows 24.9, 24.2, 22.2, 490k rows 42.2, 40.3,
 // 36.7, 1.05M rows 71.5, 69.3, 65.5, 3.2M rows 236, 222, 229: the vectors first
 // where a thread has more than ten rows.
-constexpr size_t kResidentBytes = 216 * 1024;
+constexpr size_t kResidentBytes = 194 * 1024;
 constexpr size_t kMatrixFirst = 10;
 
 // Enqueues one persistent solve on `stream` and returns without waiting:
@@ -1195,6 +1237,15 @@ int32_t check_word_status(const Scratch &S, cudaStream_t stream) {
   return FVC_OK;
 }
 
+// The grid-wide PCG of n rows.  p stored from 262144 rows on: per iteration on
+// GB300, stored against formed at every read, 66k rows 7.8 vs 7.2 us, 176k 11.1
+// vs 10.8, 262k 12.7 vs 13.1, 490k 19.3 vs 21.5, 1.05M 34.5 vs 40.1
+static auto pcg_kernel(int n) {
+  return n >= kOrderedRows  ? pcg_f64<true, kSumGrid>
+         : n >= kStorePRows ? pcg_f64<true, kSumExact>
+                            : pcg_f64<false, kSumExact>;
+}
+
 int32_t run_pcg(const DeviceMatrix &A, Scratch &S, const double *b, double *x, double tol,
                 int maxit, int init, const fvc_opts &o, cudaStream_t stream, fvc_stats *st) {
   // a system that fits one thread-block cluster runs there (fvc_cluster.cu)
@@ -1203,12 +1254,7 @@ int32_t run_pcg(const DeviceMatrix &A, Scratch &S, const double *b, double *x, d
     const int32_t rc = run_pcg_cluster(A, S, b, x, tol, maxit, init, o, stream, st);
     if (rc != FVC_ERR_UNSUPPORTED) return rc;
   }
-  // p stored from 262144 rows on: per iteration on GB300, stored against
-  // formed at every read, 66k rows 7.8 vs 7.2 us, 176k 11.1 vs 10.8, 262k 12.7
-  // vs 13.1, 490k 19.3 vs 21.5, 1.05M 34.5 vs 40.1
-  if (A.n >= kStorePRows)
-    return run_persistent(pcg_f64<true>, A, S, b, x, tol, maxit, init, o, stream, st, 5, false, 3);
-  return run_persistent(pcg_f64<false>, A, S, b, x, tol, maxit, init, o, stream, st, 5, false, 3);
+  return run_persistent(pcg_kernel(A.n), A, S, b, x, tol, maxit, init, o, stream, st, 5, false, 3);
 }
 
 // FP64 BiCGSTAB with z stored once per row from this many rows on (below,
@@ -1334,10 +1380,7 @@ int32_t enqueue_solve(const DeviceMatrix &A, Scratch &S, int code, const double 
       const int32_t rc = enqueue_pcg_cluster(A, S, b, x, tol, maxit, init, o, stream, launch);
       if (rc != FVC_ERR_UNSUPPORTED) return rc;
     }
-    if (A.n >= kStorePRows)
-      return enqueue_persistent(pcg_f64<true>, A, S, b, x, tol, maxit, init, o, stream, 5, false,
-                                launch, 3);
-    return enqueue_persistent(pcg_f64<false>, A, S, b, x, tol, maxit, init, o, stream, 5, false,
+    return enqueue_persistent(pcg_kernel(A.n), A, S, b, x, tol, maxit, init, o, stream, 5, false,
                               launch, 3);
   }
   if (code == 2) {
