@@ -207,6 +207,18 @@ int32_t launch_mixed_batched(const DeviceMatrix &A, const Scratch &S, const Batc
                              const double *b, double *x, int maxit, const fvc_opts &o,
                              cudaStream_t stream);
 
+// A kernel's limit of dynamic shared memory belongs to the process, not to the
+// launch: another thread may set it between this thread's call and its launch.
+// So it is only ever set to one value per kernel, the most any launch of it
+// asks for; a launch names its own size.
+inline bool allow_dynamic_smem(const void *kernel, size_t most) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) ==
+      cudaSuccess)
+    return true;
+  cudaGetLastError();
+  return false;
+}
+
 // Threads per block of a persistent solver launch when the caller sets
 // none (or a multiple of 128 it asked for, clamped to 128..1024).  The
 // automatic choice is one block per SM with the fewest warps that still

@@ -1090,10 +1090,7 @@ int32_t enqueue_persistent(K kernel, const DeviceMatrix &A, Scratch &S, const do
     left -= capm * mat;
     if (need <= kMatrixFirst) cap = (int)std::min(need, left / vec);
     smem = cap * vec + capm * mat;
-    if (smem > 40 * 1024 &&
-        cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess) {
-      cudaGetLastError();
+    if (smem > 0 && !allow_dynamic_smem((const void *)kernel, kResidentBytes)) {
       cap = capm = 0;
       smem = 0;
     }

@@ -1900,8 +1900,7 @@ int32_t enqueue_mixed(const DeviceMatrix &A0, Scratch &S, int code, const double
   const size_t dsmem =
       kept ? (size_t)keep * kKeptVecs * 4 * threads : staged ? kStSmem : 0;
   if (kept || staged) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem) !=
-        cudaSuccess)
+    if (!allow_dynamic_smem((const void *)kern, kept ? kKeptBytes : (size_t)kStSmem))
       return FVC_ERR_CUDA;
   } else {
     // the plain-load kernels gather through L1: keep it at its largest
