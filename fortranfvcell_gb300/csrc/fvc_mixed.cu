@@ -330,25 +330,25 @@ __device__ __forceinline__ float arow32(const MArgs &a, int s, int lane, int row
   const float *vp = a.w32 + base + lane;
   const float yi = yf(row);
   float t = ld_stream(a.e32 + row) * yi;
-  if (w <= 4) {
+  auto four = [&](int k0) {  // its entries k0 .. k0+3, the loads before the gathers
     int c[4];
     float v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      c[k] = (k < w) ? ld_stream(cp + 32 * k) : row;
-      v[k] = (k < w) ? ld_stream(vp + 32 * k) : 0.0f;
+      const bool in = k0 + k < w;
+      c[k] = in ? ld_stream(cp + 32 * (k0 + k)) : row;
+      v[k] = in ? ld_stream(vp + 32 * (k0 + k)) : 0.0f;
       FVC_CHK((unsigned)c[k] < (unsigned)a.A.n, a.A.chk, kChkColumn, c[k] = row);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      if (k < w) t = fmaf(v[k], yi - yf(c[k]), t);
-    return t;
-  }
+      if (k0 + k < w) t = fmaf(v[k], yi - yf(c[k]), t);
+  };
+  if (w <= 4) {
+    four(0);
+  } else {
 #pragma unroll 1
-  for (int k = 0; k < w; ++k) {
-    int c = ld_stream(cp + 32 * k);
-    FVC_CHK((unsigned)c < (unsigned)a.A.n, a.A.chk, kChkColumn, c = row);
-    t = fmaf(ld_stream(vp + 32 * k), yi - yf(c), t);
+    for (int k0 = 0; k0 < w; k0 += 4) four(k0);
   }
   return t;
 }
