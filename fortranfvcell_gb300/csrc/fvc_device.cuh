@@ -1104,7 +1104,8 @@ __device__ __forceinline__ double sell_row_f64(const SellView<double> &A, int s,
 // gather of each wait for the last (1M rows of eight: PCG 67 -> 50 us per
 // iteration, BiCGSTAB 121 -> 92, transposed 183 -> 113, mixed BiCGSTAB 112 -> 75;
 // 262k rows 20.7 -> 16.3, 40.5 -> 31.9, 45.3 -> 31.7, 36.5 -> 28.7).
-template <typename XF>
+// kUnrolled: the wider rows' loop as the compiler unrolls it (spmv_f64).
+template <bool kUnrolled = false, typename XF>
 __device__ __forceinline__ double sell_row_fma(const SellView<double> &A, int s, int lane,
                                                int row, XF xf) {
   const int64_t base = A.sptr[s];
@@ -1132,6 +1133,12 @@ __device__ __forceinline__ double sell_row_fma(const SellView<double> &A, int s,
   };
   if (w <= 4) {
     four(0);
+  } else if (kUnrolled) {
+    for (int k = 0; k < w; ++k) {
+      int c = ld_stream(cp + 32 * k);
+      FVC_CHK((unsigned)c < (unsigned)A.n, A.chk, kChkColumn, c = row);
+      t = fma(ld_stream(vp + 32 * k), xf(c), t);
+    }
   } else {
 #pragma unroll 1
     for (int k0 = 0; k0 < w; k0 += 4) four(k0);

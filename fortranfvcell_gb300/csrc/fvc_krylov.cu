@@ -911,16 +911,18 @@ __global__ void __launch_bounds__(1024, 1) gmres_f64(KArgs a) {
 // ---------------------------------------------------------------------
 // Plain SpMV kernels (one warp per slice, grid-stride over slices)
 // ---------------------------------------------------------------------
-template <bool kFused>
-__global__ void __launch_bounds__(256) spmv_f64(SellView<double> A, const double *__restrict__ x,
-                                                double *__restrict__ y) {
+// kMany: few registers, so that the SMs hold all blocks of a large grid at once;
+// otherwise more, for more loads in flight per warp (kManySlices).
+template <bool kFused, bool kMany>
+__global__ void __launch_bounds__(256, kMany ? 8 : 6)
+    spmv_f64(SellView<double> A, const double *__restrict__ x, double *__restrict__ y) {
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < A.nslices; s += nw) {
     const int row = s * 32 + lane;
     if (row >= A.n) continue;
     auto xf = [&](int k) { return __ldg(x + k); };
-    y[row] = kFused ? sell_row_fma(A, s, lane, row, xf) : sell_row_f64(A, s, lane, row, xf);
+    y[row] = kFused ? sell_row_fma<!kMany>(A, s, lane, row, xf) : sell_row_f64(A, s, lane, row, xf);
   }
 }
 
@@ -1989,16 +1991,28 @@ int32_t run_krylov_batched(DeviceMatrix &A, Scratch &S, int nsys,
   return worst;
 }
 
+// The fused product in 32 registers (eight blocks an SM) from this many slices
+// on, two and a half rounds of the grid, while the rows have four entries or
+// fewer; in 40 below and on wider rows.  40 against 32 registers: quadrilaterals
+// 3.6k rows 2.72 and 2.85 us, 314k 5.8 and 5.9, 490k 8.2 and 8.3, 810k 13.5 and
+// 13.1, 2.0M 30.4 and 26.2; triangles 520k 8.5 and 8.9, 980k 16.5 and 16.1; mixed
+// 735k 12.2 and 12.4, 1.05M 16.8 and 16.0; rows of six and eight entries, 3.6k
+// rows 3.3 and 3.5, 3.2 and 3.5, 1M 24.5 and 25.6, 25.6 and 24.4.
+constexpr int kManySlices = 24576;
+
 int32_t launch_spmv(const DeviceMatrix &A, const double *x, double *y, cudaStream_t stream,
                     bool fused) {
   if (A.n <= 0) return FVC_ERR_ARG;
   const int threads = 256;
   int blocks = (A.nslices + 7) / 8;
   blocks = std::max(1, std::min(blocks, sm_count() * 8));
-  if (fused)
-    spmv_f64<true><<<blocks, threads, 0, stream>>>(view64(A), x, y);
+  const bool many = A.nslices >= kManySlices && A.slots <= (int64_t)128 * A.nslices;
+  if (fused && many)
+    spmv_f64<true, true><<<blocks, threads, 0, stream>>>(view64(A), x, y);
+  else if (fused)
+    spmv_f64<true, false><<<blocks, threads, 0, stream>>>(view64(A), x, y);
   else
-    spmv_f64<false><<<blocks, threads, 0, stream>>>(view64(A), x, y);
+    spmv_f64<false, true><<<blocks, threads, 0, stream>>>(view64(A), x, y);
   count_launch();
   return cudaPeekAtLastError() == cudaSuccess ? FVC_OK : FVC_ERR_CUDA;
 }

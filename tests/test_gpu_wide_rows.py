@@ -109,3 +109,24 @@ def test_solves(width, how):
         c.solve(1 if "pcg" in how else 2, bd, x, 1e-12, 1000, o)
     c.close()
     assert np.linalg.norm(x.cpu().numpy() - want) <= 1e-9 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("width", [4, 6])
+@pytest.mark.parametrize("slices", [24575, 24576, 24577])
+@pytest.mark.parametrize("ragged", [0, 31])
+def test_products_of_many_slices(width, slices, ragged):
+    """Both sides of the size from which narrow rows are summed in fewer
+    registers, the last slice full or of one row; bars as above."""
+    import torch
+    s = _csrd(32 * slices - ragged, width)
+    x = np.random.default_rng(3).uniform(-1, 1, s["n"])
+    want = _product(s, x)
+    c = _context(s)
+    xd = torch.from_numpy(x).cuda()
+    y = torch.empty_like(xd)
+    c.spmv(xd, y)
+    assert np.array_equal(y.cpu().numpy(), want)
+    c.spmv_fast(xd, y)
+    c.close()
+    scale = np.abs(s["ad"] * x) + np.bincount(s["rows"], np.abs(s["au"] * x[s["cols"]]), s["n"])
+    assert (np.abs(y.cpu().numpy() - want) <= 4 * (width + 1) * 2.0 ** -53 * scale).all()
