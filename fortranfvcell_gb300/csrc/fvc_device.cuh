@@ -781,16 +781,19 @@ __device__ __forceinline__ int top_of_partials(int m) {
 // (ex, biased) of all threads of all blocks, by a maximum exchanged through
 // the reduction slots and a barrier.  Cold: the first sum of a kind, and one
 // that its window did not hold.  False when a wait exceeded its bound.
-static __device__ __noinline__ bool window_by_partials(const GridSync &gs, Episode &episode,
-                                                       ExactState &xs, int *top, int nv,
-                                                       const int *ex, int *part) {
+// All by value: a reference to gs kept its owner (a batch kernel's whole MArgs, 416
+// bytes) in local memory for the length of the solve (batches 1-6 % slower).
+static __device__ __noinline__ bool window_by_partials(RedSlot *slots, unsigned int *count,
+                                                       int *err, unsigned int nb, unsigned int me,
+                                                       int cluster, unsigned int ep,
+                                                       ExactState &xs, int *top, int nv, int ex0,
+                                                       int ex1, int ex2, int *part) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const unsigned int ep = ++episode.n;
   __shared__ int s_ok;
-  RedSlot *slots = gs.slots + (size_t)(ep & 3u) * kMaxNV * gs.nblocks;
+  slots += (size_t)(ep & 3u) * kMaxNV * nb;
   __syncthreads();  // part is free
   for (int q = 0; q < nv; ++q) {
-    const int m = __reduce_max_sync(0xffffffffu, ex[q]);
+    const int m = __reduce_max_sync(0xffffffffu, q == 0 ? ex0 : q == 1 ? ex1 : ex2);
     if (lane == 0) part[q * 32 + warp] = m;
   }
   __syncthreads();
@@ -798,15 +801,15 @@ static __device__ __noinline__ bool window_by_partials(const GridSync &gs, Episo
     for (int q = 0; q < nv; ++q) {
       int m = 0;
       for (int w = 0; w < nw; ++w) m = max(m, part[q * 32 + w]);
-      st_slot(slots + (size_t)q * gs.nblocks + (blockIdx.x - gs.base), (double)m, ep);
+      st_slot(slots + (size_t)q * nb + me, (double)m, ep);
     }
     // (one block and a cluster count no arrivals, see grid_barrier)
-    if (gs.nblocks > 1 && !gs.cluster) red_add_release(gs.count, 1u);
+    if (nb > 1 && !cluster) red_add_release(count, 1u);
   }
-  if (gs.cluster) cooperative_groups::this_cluster().sync();
+  if (cluster) cooperative_groups::this_cluster().sync();
   if (warp == 0) {
     const bool ok =
-        gs.nblocks == 1 || gs.cluster || wait_count<true>(gs.count, gs.err, ep * gs.nblocks);
+        nb == 1 || cluster || wait_count<true>(count, err, ep * nb);
     if (lane == 0) s_ok = ok ? 1 : 0;
   }
   __syncthreads();
@@ -815,8 +818,8 @@ static __device__ __noinline__ bool window_by_partials(const GridSync &gs, Episo
     bool nan = false;
     for (int q = 0; q < nv; ++q) {
       int m = 0;
-      for (unsigned int b = lane; b < gs.nblocks; b += 32)
-        m = max(m, (int)__longlong_as_double((long long)ld_slot(slots + (size_t)q * gs.nblocks + b).v));
+      for (unsigned int b = lane; b < nb; b += 32)
+        m = max(m, (int)__longlong_as_double((long long)ld_slot(slots + (size_t)q * nb + b).v));
       m = __reduce_max_sync(0xffffffffu, m);
       nan = nan || m == 0x7ff;
       if (lane == 0) top[q] = top_of_partials(m);
@@ -939,10 +942,10 @@ __device__ __forceinline__ bool exact_sum(const GridSync &gs, Episode &episode, 
 #pragma unroll 1
   for (;;) {
     if (!have) {
-      int ex[NV];
-#pragma unroll
-      for (int q = 0; q < NV; ++q) ex[q] = expo(q);
-      if (!window_by_partials(gs, episode, xs, win.top, NV, ex, part)) return false;
+      if (!window_by_partials(gs.slots, gs.count, gs.err, gs.nblocks, blockIdx.x - gs.base,
+                              gs.cluster, ++episode.n, xs, win.top, NV, expo(0),
+                              NV > 1 ? expo(1 % NV) : 0, NV > 2 ? expo(2 % NV) : 0, part))
+        return false;
     }
     const unsigned int set = (episode.x++) & 1u;
 #pragma unroll
