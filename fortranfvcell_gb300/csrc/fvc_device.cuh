@@ -673,9 +673,10 @@ __device__ __forceinline__ void window_set(SumWindow<NV> &w, const double *t) {
   for (int q = 0; q < NV; ++q) w.top[q] = window_top(t[q]);
 }
 
-// A warp's values +-m 2^e (m < 2^53; up to two per lane) as limbs of the window
+// A warp's values +-m 2^e (m < 2^kMant; up to two per lane) as limbs of the window
 // with the given top, added over the warp and then to the block's acc[k] for
 // limb k.  True in the lanes whose value does not fit.
+template <int kMant>
 __device__ __forceinline__ bool add_limbs(int (&l)[kLimbs], unsigned long long m, int e, int neg,
                                           int top) {
   const int s = e - (top - kWindowBits);  // bit of the window m starts at
@@ -698,7 +699,9 @@ __device__ __forceinline__ bool add_limbs(int (&l)[kLimbs], unsigned long long m
                          (int)(hi >> 41) & M};
 #pragma unroll
   for (int k = 0; k < kLimbs; ++k) l[k] += (x[k] ^ -neg) + neg;
-  return s > kWindowBits - 53 - 1;
+  // (with the bound of FP64, FP32 parts lost 29 of the kWindowHead bits: up to every
+  // third sum of a BiCGSTAB whose products cancel was taken again)
+  return s > kWindowBits - kMant - 1;
 }
 __device__ __forceinline__ void warp_limbs(const int (&l)[kLimbs], bool ovf, int *acc) {
   const int lane = threadIdx.x & 31;
@@ -715,7 +718,7 @@ __device__ __forceinline__ void put_limbs(double v, int top, int *acc) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   const int ex = (int)(b >> 52) & 0x7ff;
   const unsigned long long m = (b & 0xfffffffffffffull) | ((unsigned long long)(ex != 0) << 52);
-  const bool ovf = add_limbs(l, m, (ex ? ex : 1) - 1075, (int)(b >> 63), top);
+  const bool ovf = add_limbs<53>(l, m, (ex ? ex : 1) - 1075, (int)(b >> 63), top);
   warp_limbs(l, ovf, acc);
 }
 // The value of an FP32 pair, its parts renormalised so that they do not overlap
@@ -731,7 +734,7 @@ __device__ __forceinline__ void put_limbs(float s, float c, int top, int *acc) {
     const unsigned int m = (b & 0x7fffffu) | ((unsigned int)(ex != 0) << 23);
     // NaN and Inf: an exponent no window holds
     const int e = ex == 0xff ? 4096 : (ex ? ex : 1) - 150;
-    ovf = add_limbs(l, (unsigned long long)m, e, (int)(b >> 31), top) || ovf;
+    ovf = add_limbs<24>(l, (unsigned long long)m, e, (int)(b >> 31), top) || ovf;
   }
   warp_limbs(l, ovf, acc);
 }
