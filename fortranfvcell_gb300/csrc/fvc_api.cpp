@@ -367,6 +367,7 @@ int32_t fvc_context_destroy(fvc_context *c) {
   cudaFree(c->S.g);
   cudaFree(c->S.sync);
   cudaFree(c->S.trace);
+  cudaFreeHost(c->S.est);
   cudaFree(c->S.history);
   cudaFree(c->d_b);
   cudaFree(c->d_x);

@@ -64,6 +64,8 @@ struct Scratch {
   double *result = nullptr;     // ... solver scalars written by block 0
   int *iresult = nullptr;
   double *trace = nullptr;      // per residual replacement: (iteration, ||r||/||b||)
+  int *est = nullptr;           // host: a batch's row starts and estimates, of nest systems
+  size_t nest = 0;
   float *history = nullptr;     // per iteration: recursive ||r||/||b|| (first kHistoryMax)
   // FP64 solves that fit one cluster add their sums in FP64 in a fixed order
   // instead of exactly.  Set for the systems of a SIMPLE loop with energy: the

@@ -286,8 +286,10 @@ int32_t fvc_solve_batched(fvc_context *ctx, int32_t nsys, const int32_t *row_sta
  * take (in a SIMPLE loop, its count in the previous outer iteration), which
  * sets its share of the launch's blocks: work = slices x iterations x SpMVs
  * per iteration.  Host arrays of nsys entries; NULL codes = all PCG, NULL
- * tols = tol for all, NULL its_hint (or an entry <= 0) = sqrt(rows).  The
- * hint moves only the speed, never the results beyond rounding.  Each
+ * tols = tol for all, NULL its_hint = estimated from the diagonal dominance of
+ * the rows where the batch has both solvers (one small kernel and a wait), else
+ * sqrt(rows), as is an entry <= 0.  The hint moves only the speed, never the
+ * results beyond rounding.  Each
  * system takes the warm-start rule of its solver (src/Solver.f) unless opts
  * sets init.  FVC_ERR_UNSUPPORTED for BiCGSTAB on matriz 2, as fvc_solve. */
 int32_t fvc_solve_batched_ex(fvc_context *ctx, int32_t nsys, const int32_t *row_start,
