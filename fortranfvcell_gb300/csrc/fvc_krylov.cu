@@ -1489,20 +1489,29 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
   // groups: 128-thread blocks by default, twice the co-resident blocks of
   // 256, so the one-block minimum of the small systems takes a smaller share
   // (the u, v, T and p' systems of 256 heated cavities, 1024 systems: 184 ms
-  // at 128 threads, 215 at 256, 386 at 512); clusters: 256.  Few systems
-  // (kSparse blocks or more each) leave half of the thread slots empty: eight
-  // blocks of 128 threads on an SM delay one another's sums by more than the
-  // rows they share save, 48 systems of 24^2 to 140^2 cells, mixed, 13.4 ms
-  // at eight a SM, 9.5 at four, 48 triangle meshes of 12^2 to 60^2 in FP64 5.9
-  // and 5.15 (but 150 systems 9.95 and 11.7); and with kSparse blocks of 256
-  // threads each those serve better, two to an SM: 20 systems of up to 100^2,
-  // mixed, 8.3 ms against 8.8 of four of 128, 12 of up to 140^2 16.7 and 18.3
+  // at 128 threads, 215 at 256, 386 at 512); clusters: 256.  With kSparse blocks
+  // of 256 threads or more for each system those serve better: their sums have half
+  // the blocks (48 systems of 100^2 to 280^2 cells, mixed, 26.3 ms at 256, 28.3 at
+  // 128; but 70 in FP64 73 and 63).
+  // Small batches (few: kHalfRows rows per thread slot of the device) leave half
+  // of the slots empty: a system has its rows' slices on a warp each either way,
+  // and eight blocks of 128 threads on an SM delay one another's sums by more than
+  // the rows they share save.  PCG and BiCGSTAB side by side, full and half: mixed,
+  // 136k rows 6.3 and 5.5 ms, 268k 6.7 and 5.7, 364k 14.0 and 11.8, 486k 17.4 and
+  // 17.0, 791k 16.6 and 17.8, 1.6M 25.5 and 36.3; FP64 117k 5.5 and 5.2, 175k 7.6 and
+  // 8.7, 268k 6.9 and 7.4, 1.6M 45 and 61; PCG alone, FP64, 64 of 128^2 20.3 and
+  // 28.4, 64 of 256^2 150 and 252.  In FP64 a batch whose every slice has a warp at
+  // half occupancy keeps the small blocks: 32 of 48^2 1.62 ms, 2.03 at 256 threads.
   constexpr int kSparse = 8;
-  const bool few = nsys * kSparse <= 4 * sm_count();
+  const double kHalfRows = mixed ? 2.4 : 1.0;
+  const bool few = nsys * kSparse <= 4 * sm_count() && A.n <= kHalfRows * 1024.0 * sm_count();
+  const bool wide = few ? nsys * kSparse <= 2 * sm_count() &&  // two an SM
+                              (mixed || A.n > 512 * sm_count())
+                        : nsys * (kSparse + 4) <= 4 * sm_count();  // four an SM
   auto threads_for = [&](int cs) {
-    return (o.block_threads > 0)                               ? block_threads_for(o.block_threads, 0, 1)
-           : cs > 0 || nsys * kSparse <= 2 * sm_count() ? 256
-                                                               : 128;
+    return (o.block_threads > 0) ? block_threads_for(o.block_threads, 0, 1)
+           : cs > 0 || wide      ? 256
+                                 : 128;
   };
   int threads = threads_for(csize);
   if (mixed) {
