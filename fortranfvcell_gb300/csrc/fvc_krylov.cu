@@ -1461,31 +1461,6 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
   // ceil(rows / (the largest system's rows / 16)) blocks, so that every block
   // has about as many rows and the per-iteration times line up
   bool adaptive = o.cluster_size <= 0;
-  if (o.cluster_size == 0) {
-    // automatic: clusters sized per system when their blocks fill the
-    // device, else groups, where a large system can spread over more than
-    // 16 blocks (the enthalpy systems of those SIMPLE cases in FP64: 256
-    // cases 184 ms on clusters against 233 ms in groups; 64 cases 83
-    // against 52 ms).  In FP64 twice over: 150 systems of 32^2 to 100^2 cells
-    // 11.4 ms on clusters, 10.0 in groups (mixed 10.0 and 11.1), 900 of 32^2
-    // to 64^2 17.6 and 19.7 (mixed 16.1 and 17.0)
-    int most_rows = 0;
-    for (int s = 0; s < nsys; ++s)
-      most_rows = std::max(most_rows, row_start[s + 1] - row_start[s]);
-    const long per = std::max(1024, (most_rows + 15) / 16);
-    long want = 0;
-    for (int s = 0; s < nsys; ++s)
-      want += std::min<long>(16, std::max<long>(1, (row_start[s + 1] - row_start[s] + per - 1) / per));
-    int occ256 = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &occ256, mixed ? mixed_batched_kernel(256) : krylov_batched_kernel(256), 256, 0);
-    const long fill = (long)std::max(occ256, 1) * sm_count();
-    if (want < (mixed ? fill : 2 * fill)) adaptive = false;
-  }
-  int csize = (o.cluster_size == 1)   ? 0
-              : (o.cluster_size >= 2) ? o.cluster_size
-              : adaptive              ? 16
-                                      : 0;
   // groups: 128-thread blocks by default, twice the co-resident blocks of
   // 256, so the one-block minimum of the small systems takes a smaller share
   // (the u, v, T and p' systems of 256 heated cavities, 1024 systems: 184 ms
@@ -1513,13 +1488,52 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
            : cs > 0 || wide      ? 256
                                  : 128;
   };
+  // co-resident blocks of one launch of groups
+  auto group_cap = [&](int t) {
+    int occ = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &occ, mixed ? mixed_batched_kernel(t) : krylov_batched_kernel(t), t, 0);
+    if (occ <= 0) occ = 1;
+    if (o.blocks_per_sm > 0)
+      occ = std::min(occ, o.blocks_per_sm);
+    else if (few && o.block_threads <= 0)
+      occ = std::min(occ, 512 / t);
+    const int blocks = occ * sm_count();
+    return (o.max_blocks > 0) ? std::min(blocks, o.max_blocks) : blocks;
+  };
+  if (o.cluster_size == 0) {
+    // automatic: clusters sized per system when their blocks fill the
+    // device, else groups, where a large system can spread over more than
+    // 16 blocks (the enthalpy systems of those SIMPLE cases in FP64: 256
+    // cases 184 ms on clusters against 233 ms in groups; 64 cases 83
+    // against 52 ms).  In FP64 twice over: 150 systems of 32^2 to 100^2 cells
+    // 11.4 ms on clusters, 10.0 in groups (mixed 10.0 and 11.1), 900 of 32^2
+    // to 64^2 17.6 and 19.7 (mixed 16.1 and 17.0), as long as the groups hold
+    // them (a caller's max_blocks, blocks_per_sm or block_threads)
+    int most_rows = 0;
+    for (int s = 0; s < nsys; ++s)
+      most_rows = std::max(most_rows, row_start[s + 1] - row_start[s]);
+    const long per = std::max(1024, (most_rows + 15) / 16);
+    long want = 0;
+    for (int s = 0; s < nsys; ++s)
+      want += std::min<long>(16, std::max<long>(1, (row_start[s + 1] - row_start[s] + per - 1) / per));
+    int occ256 = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &occ256, mixed ? mixed_batched_kernel(256) : krylov_batched_kernel(256), 256, 0);
+    const long fill = (long)std::max(occ256, 1) * sm_count();
+    if (want < fill || (!mixed && want < 2 * fill && nsys <= group_cap(threads_for(0))))
+      adaptive = false;
+  }
+  int csize = (o.cluster_size == 1)   ? 0
+              : (o.cluster_size >= 2) ? o.cluster_size
+              : adaptive              ? 16
+                                      : 0;
   int threads = threads_for(csize);
   if (mixed) {
     int32_t rc = build_f32_copy(A, stream, o.fp32_layout);
     if (rc == FVC_OK) rc = ensure_f32_vectors(S, (size_t)A.n);
     if (rc != FVC_OK) return rc;
   }
-  int occ = 0;
   // PCG stores p: most groups of a batch are one block, where publishing p
   // is a __syncthreads (the same 1024 systems: 159 ms vs 184 ms)
   const void *kern = mixed ? mixed_batched_kernel(threads) : krylov_batched_kernel(threads);
@@ -1552,12 +1566,7 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
     }
   }
   if (csize == 0) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, 0);
-    if (occ <= 0) occ = 1;
-    if (o.blocks_per_sm > 0 && o.blocks_per_sm < occ) occ = o.blocks_per_sm;
-    else if (few && o.blocks_per_sm <= 0 && o.block_threads <= 0) occ = std::min(occ, 512 / threads);
-    cap = occ * sm_count();
-    if (o.max_blocks > 0) cap = std::min(cap, o.max_blocks);
+    cap = group_cap(threads);
     if (nsys > cap) {
       fprintf(stderr, "fvcgpu: %d systems exceed the %d co-resident blocks of one launch\n", nsys,
               cap);
@@ -1578,7 +1587,7 @@ int32_t plan_batched(DeviceMatrix &A, Scratch &S, int nsys, const int32_t *row_s
   for (int s = 0; s < nsys; ++s) {
     const int rows = row_start[s + 1] - row_start[s];
     slices[s] = (rows + 31) / 32;
-    most[s] = (slices[s] + warps - 1) / warps;
+    most[s] = std::min((slices[s] + warps - 1) / warps, kXBlocks);
     const double its = (its_hint && its_hint[s] > 0.0) ? its_hint[s] : std::sqrt((double)rows);
     wt[s] = slices[s] * its * ((codes && codes[s] == 2) ? 2.0 : 1.0);
     wleft += wt[s];
