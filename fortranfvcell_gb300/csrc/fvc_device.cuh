@@ -739,8 +739,19 @@ __device__ __forceinline__ void put_limbs(float s, float c, int top, int *acc) {
   warp_limbs(l, ovf, acc);
 }
 
-// T units of the window (its top) in FP64, rounded to nearest even; 0 or Inf
-// where it leaves FP64's exponents.  All in integers: a conversion and an FP64
+// m 2^(e - 1086) (m's top bit set, rest: something below it), e < 1, as the bits of
+// a subnormal, rounded to nearest even.  Cold.
+static __device__ __noinline__ unsigned long long subnormal_bits(unsigned long long m, bool rest,
+                                                                 int e) {
+  const int sh = 12 - e;  // below the last bit
+  if (sh > 64) return 0;
+  unsigned long long r = sh < 64 ? m >> sh : 0;
+  const unsigned long long rem = m << (64 - sh), half = 1ull << 63;
+  r += (rem > half || (rem == half && (rest || (r & 1)))) ? 1 : 0;
+  return r;
+}
+// T units of the window (its top) in FP64, rounded to nearest even (Inf above its
+// exponents).  All in integers: a conversion and an FP64
 // addition are 60 clocks and more of the sum's critical path each.
 __device__ __forceinline__ double window_value(__int128 T, int top) {
   const bool neg = T < 0;
@@ -755,7 +766,10 @@ __device__ __forceinline__ double window_value(__int128 T, int top) {
   const int e = top - kWindowBits + (h ? 127 : 63) - z + 1023;
   unsigned long long v = ((unsigned long long)(e - 1) << 52) + r;
   if (e >= 0x7ff) v = 0x7ff0000000000000ull;
-  if (a == 0 || e <= 0) v = 0;
+  if (a == 0)
+    v = 0;
+  else if (e <= 0)
+    v = subnormal_bits(m, rest != 0, e);
   return __longlong_as_double((long long)(v | ((unsigned long long)neg << 63)));
 }
 // Whether a total lies so low in its window that what the threads dropped
