@@ -11,9 +11,8 @@ from _systems import pressure, unsymmetric
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("side", [40, 99])       # one cluster (PCG); the whole grid
-@pytest.mark.parametrize("code", [1, 2])
-def test_subnormal_sums(orc, side, code):
+def _residuals(orc, side, code, tol, scales):
+    """|b - A x| / |b| of the solves of the right-hand sides b * scale."""
     import scipy.sparse as sp
     import torch
     from fortranfvcell_gb300 import Context, mesh
@@ -28,13 +27,27 @@ def test_subnormal_sums(orc, side, code):
     b = np.random.default_rng(11).uniform(-1.0, 1.0, n)
     c = Context()
     c.set_matrix(1, True, n, s["nad"], s["ad"], s["au"], s["au"], s["ia"], s["ja"])
-
-    def residual(scale):
+    out = []
+    for scale in scales:
         x = torch.zeros(n, dtype=torch.float64, device="cuda")
-        c.solve(code, torch.from_numpy(b * scale).cuda(), x, 1e-3, 5000,
+        c.solve(code, torch.from_numpy(b * scale).cuda(), x, tol, 5000,
                 make_opts("fp64", init=1, stop_rule=1))
-        return np.linalg.norm(b - full @ (x.cpu().numpy() / scale)) / np.linalg.norm(b)
-    want = residual(1.0)
-    got = residual(1e-157)
+        out.append(np.linalg.norm(b - full @ (x.cpu().numpy() / scale)) / np.linalg.norm(b))
     c.close()
+    return out
+
+
+@pytest.mark.parametrize("side", [40, 99])       # one cluster (PCG); the whole grid
+@pytest.mark.parametrize("code", [1, 2])
+def test_subnormal_sums(orc, side, code):
+    want, got = _residuals(orc, side, code, 1e-3, [1.0, 1e-157])
     assert got <= 2.0 * want, (got, want)
+
+
+@pytest.mark.parametrize("side", [40, 99])
+@pytest.mark.parametrize("code", [1, 2])
+def test_sums_that_become_subnormal(orc, side, code):
+    """At 1e-150 the sums reach the subnormals as the solve converges: to the
+    tolerance, as at scale 1 (the recurrence's residual within a tenth)."""
+    got, = _residuals(orc, side, code, 1e-6, [1e-150])
+    assert got <= 1.1e-6, got
