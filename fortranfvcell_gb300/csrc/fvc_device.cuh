@@ -664,8 +664,9 @@ struct SumWindow {
 
 __device__ __forceinline__ int window_top(double total) {
   const int e = (__double2hiint(total) >> 20) & 0x7ff;
-  // zero, subnormal, NaN or Inf, or near the ends of the exponents: none
-  return (e < 200 || e > 1800) ? kNoWindow : e - 1022 + kWindowHead;
+  // zero, subnormal, NaN or Inf: none.  (Near the ends of the exponents a window is as
+  // good as elsewhere: below the smallest subnormal there is nothing to drop.)
+  return (e == 0 || e == 0x7ff) ? kNoWindow : e - 1022 + kWindowHead;
 }
 template <int NV>
 __device__ __forceinline__ void window_set(SumWindow<NV> &w, const double *t) {

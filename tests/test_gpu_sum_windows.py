@@ -40,3 +40,25 @@ def test_cancelling_products(nx, ny):
     hard, its_hard = _us_per_iteration(_system(nx, ny, 0.0))
     assert its_hard > 3 * its_easy
     assert hard <= 1.15 * easy, (hard, easy)
+
+
+@pytest.mark.parametrize("nx,ny", [(45, 46), (110, 109)])
+@pytest.mark.parametrize("code", [1, 2])
+@pytest.mark.parametrize("scale", [1e-130, 1e130])
+def test_sums_near_the_ends_of_the_exponents(nx, ny, code, scale):
+    """Totals of 1e-260 and 1e260 have windows like any other: an iteration takes
+    as long as with totals of 1e-200 (a tenth for the timing)."""
+    from fortranfvcell_gb300 import Context, make_opts
+    s = _system(nx, ny, 0.05)
+    ctx = Context()
+    ctx.set_matrix(1, True, s["n"], s["nad"], s["ad"], s["au"], s["au"], s["ia"], s["ja"])
+    b, us = np.random.default_rng(4).uniform(-1, 1, s["n"]), []
+    for sc in (1e-100, scale):
+        bd, x, best = torch_dev(b * sc), torch_dev(np.zeros(s["n"])), np.inf
+        for _ in range(6):
+            st = ctx.solve(code, bd, x, 0.0, 25, make_opts("fp64", init=1), raise_on_error=False)
+            assert st.iterations == 25
+            best = min(best, st.solve_ms)
+        us.append(best)
+    ctx.close()
+    assert us[1] <= 1.1 * us[0], us
