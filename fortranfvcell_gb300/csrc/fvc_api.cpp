@@ -367,7 +367,7 @@ int32_t fvc_context_destroy(fvc_context *c) {
   cudaFree(c->S.g);
   cudaFree(c->S.sync);
   cudaFree(c->S.trace);
-  cudaFreeHost(c->S.est);
+  if (c->S.est) cudaFreeHost(c->S.est);
   cudaFree(c->S.history);
   cudaFree(c->d_b);
   cudaFree(c->d_x);
@@ -685,7 +685,8 @@ int32_t fvc_autotune(fvc_context *c, int32_t code, int32_t precision, int32_t tr
   }
   // the launch shapes the kernels take: the automatic one (a cluster for
   // small PCG systems, else one block per SM with the fewest warps), block
-  // sizes, caps on the grid, and for mixed CG the staged or plain loads
+  // sizes (for mixed CG 1024 threads take the kept form while a block's rows fit),
+  // caps on the grid, and for mixed CG the staged or plain loads
   std::vector<fvc_opts> cand;
   fvc_opts base;
   fvc_opts_default(&base);

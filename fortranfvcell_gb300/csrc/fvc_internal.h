@@ -67,11 +67,13 @@ struct Scratch {
   int *est = nullptr;           // host: a batch's row starts and estimates, of nest systems
   size_t nest = 0;
   float *history = nullptr;     // per iteration: recursive ||r||/||b|| (first kHistoryMax)
-  // FP64 solves that fit one cluster add their sums in FP64 in a fixed order
-  // instead of exactly.  Set for the systems of a SIMPLE loop with energy: the
-  // last bits of a sum move its enthalpy by up to 1e-6 at a tolerance of 1e-10
-  // (BiCGSTAB stops an iteration earlier or later, both within the tolerance),
-  // so that a loop continued from a saved state would leave its old path.
+  // FP64 solves that fit one cluster add their sums in FP64 in the fixed order
+  // they had before the exact sums.  Set for the systems of a SIMPLE loop with
+  // energy: the last bits of a sum move its enthalpy by up to 1e-6 at a tolerance of
+  // 1e-10 (BiCGSTAB stops an iteration earlier or later, both within the
+  // tolerance).  Small loops, whose systems all fit a cluster, so stay on the path
+  // of states saved earlier; larger ones, and batches, take the exact sums, which
+  // are the more accurate, and may leave it by that much.
   bool ordered = false;
 };
 

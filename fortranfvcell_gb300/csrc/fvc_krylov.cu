@@ -19,7 +19,9 @@
 // GB300 executes FP64 at ~1/64 of its FP32 rate, and these two changes
 // roughly halve the FP64 instructions per row; they move results only at
 // rounding level, like the dot products, which are exact integer sums
-// (exact_sum) instead of the reference's sequential sums.
+// (exact_sum) or, in the PCG from kOrderedRows rows on, the cluster BiCGSTAB and
+// GMRES, FP64 sums in a fixed tree order, instead of the reference's
+// sequential sums.
 // BiCGSTAB adds one thing the reference lacks: where one of its
 // denominators is exactly zero (the reference goes on with Inf/NaN), the
 // recurrence restarts from the current residual, or the solve ends with
@@ -433,13 +435,15 @@ __device__ __forceinline__ void pcg_run(const KArgs &a, const Part &P, const Gri
 }
 
 constexpr int kStorePRows = 262144;
-// The CG's sums keep a fixed FP64 order from this many rows on.  The last bits
-// of its sums move the residual history of a solve of thousands of iterations
-// by parts in 1000, and with it the iteration that meets the tolerance: at 1.05M
-// rows and a tolerance of 1e-8 exact sums moved the solution by 3e-11 to 2e-9 (8
-// right-hand sides; its error is 1e-7), at 512k rows and 1e-9 by 3e-11, at 66k
-// rows by 1e-12.  In order, it stays the same bit for bit; per iteration at
-// 1.05M rows 36.9 us against 33.7 with exact sums, at 262k 15.2 against 12.2.
+// The CG's sums keep the fixed FP64 order they always had from this many rows on.
+// The exact ones are the more accurate, and no solution is better for the order:
+// what it keeps is agreement, bit for bit, with what the same solve gave before.
+// The last bits of the sums move the residual history of a solve of thousands of
+// iterations by parts in 1000, and with it the iteration that meets the
+// tolerance: at 1.05M rows and a tolerance of 1e-8 exact sums moved the solution by
+// 3e-11 to 2e-9 (8 right-hand sides; its error is 1e-7), at 512k rows and 1e-9 by
+// 3e-11, at 66k rows by 1e-12.  Per iteration at 1.05M rows 36.9 us against 33.7
+// with exact sums, at 262k 15.2 against 12.2.
 constexpr int kOrderedRows = 524288;
 
 template <bool kStoreP, int kSums>
@@ -1938,7 +1942,7 @@ static int32_t estimate_its(const DeviceMatrix &A, Scratch &S, int nsys, const i
   // pinned host memory, read and written by the kernel itself: with copies the
   // estimate of six systems took 70 us, so 25
   if (S.nest < (size_t)nsys) {
-    cudaFreeHost(S.est);
+    if (S.est) cudaFreeHost(S.est);
     S.est = nullptr;
     S.nest = 0;
     const size_t cap = std::max<size_t>(nsys, 64);

@@ -640,7 +640,7 @@ constexpr uint32_t kRegionB = kBStages * kB_Bytes;
 constexpr uint32_t kStHeader = 256;
 constexpr size_t kStSmem = kStHeader + (kRegionA > kRegionB ? kRegionA : kRegionB);
 static_assert(kA_Bytes % 128 == 0 && kB_Bytes % 128 == 0 && kA_Base % 128 == 0, "alignment");
-static_assert(kStSmem + 3072 <= 227 * 1024, "shared memory per block");
+static_assert(kStSmem + 5120 <= 227 * 1024, "shared memory per block, 5 KB of it static");
 static_assert(kLandAhead + 1 == kLandSlots, "landing ring");
 
 struct StHdr {

@@ -122,7 +122,7 @@ typedef struct {
                           launch, synchronised through global memory, the
                           share of blocks by expected work; k in 2..16: one
                           thread-block cluster of k blocks per system
-                          (cluster barrier and distributed shared memory;
+                          (cluster barrier;
                           an ordinary launch whose clusters start as SMs
                           free up, heaviest systems first; above 8 needs
                           the non-portable cluster sizes); -1: one cluster
@@ -131,8 +131,11 @@ typedef struct {
                           one launch per size, the launches side by side on
                           forked streams); 0: automatic -- -1 when the
                           systems' clusters would fill the device (their
-                          blocks at least its resident 256-thread
-                          blocks), else 1.  Single solves ignore it     */
+                          blocks at least its resident 256-thread blocks;
+                          FP64: twice as many, or more systems than one
+                          launch of groups holds), else 1.  The sums of the
+                          clusters' blocks too go through global memory.
+                          Single solves ignore it                       */
 } fvc_opts;
 
 typedef struct {
@@ -233,7 +236,8 @@ int32_t fvc_solve_async(fvc_context *ctx, int32_t code, const double *d_b,
  * over the shapes the kernels support -- the automatic choice (a thread-
  * block cluster for a PCG system of at most 8192 rows, else one block per
  * SM with the fewest warps that cover the rows), 128..1024 threads per
- * block, a cap of 16/38/76 blocks, for mixed CG plain loads or the
+ * block (mixed CG at 1024: row vectors kept in shared memory while they
+ * fit), a cap of 16/38/76 blocks, for mixed CG plain loads or the
  * staged copies at 1024 threads, and for mixed solves the FP32 operator's
  * slice widths (fvc_opts.fp32_layout: every slice padded to the widest row,
  * or each slice its own width) -- and writes the fastest per iteration to
